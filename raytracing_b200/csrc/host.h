@@ -417,6 +417,9 @@ private:
     // The wavefront form (RT_FORM_WAVEFRONT, or AUTO on a tree-searched scene)
     bool wavefront_ = false;
     std::unique_ptr<wave_runner> wave_;
+    bool pool_ = false;                 // AUTO's wavefront: the pool kernel
+    int pool_grid_ = 0;
+    device_array<float4> pool_samples_; // a pool launch's samples, kept for the next
     int32_t last_kernel_launches_ = 0; // the last launch's kernels
     wave_shape shape_{};                // how a step is launched (the autotuner's choice or the defaults)
     tune_candidate tuned_{};

@@ -21,12 +21,14 @@
 #include "ggx_energy_table.h"
 #include "kernels.cuh"
 #include "philox.cuh"
+#include "rounding.cuh"
 #include "rt_b200.h"
 
 namespace rtb
 {
 namespace
 {
+using rounds = rounds_compiler;
 #include "path.cuh"
 
 // ---- the persistent render kernel ------------------------------------------------------------------------------
@@ -1642,12 +1644,9 @@ cudaError_t launch_batch_reduce(const batch_params& p, int grid, cudaStream_t st
     return cudaGetLastError();
 }
 
-namespace
-{
-// A kernel's registers, local memory and resident blocks, and the device's multiprocessors (two attribute queries:
-// cudaGetDeviceProperties would fill every field of the device's description, a cost each session paid)
-template <class Kernel>
-cudaError_t attributes_of(Kernel kernel, kernel_attributes& out)
+// Two attribute queries for the device: cudaGetDeviceProperties would fill every field of its description, a cost each
+// session paid
+cudaError_t function_attributes(const void* kernel, kernel_attributes& out)
 {
     cudaFuncAttributes a{};
     cudaError_t e = cudaFuncGetAttributes(&a, kernel);
@@ -1682,6 +1681,14 @@ cudaError_t attributes_of(Kernel kernel, kernel_attributes& out)
     out.max_threads_per_sm = max_threads;
     out.multiprocessors = multiprocessors;
     return cudaSuccess;
+}
+
+namespace
+{
+template <class Kernel>
+cudaError_t attributes_of(Kernel kernel, kernel_attributes& out)
+{
+    return function_attributes(reinterpret_cast<const void*>(kernel), out);
 }
 } // namespace
 

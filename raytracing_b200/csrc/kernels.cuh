@@ -173,6 +173,9 @@ struct kernel_attributes
     int multiprocessors;
 };
 
+// A kernel's registers, local memory and resident blocks, and the device's multiprocessors
+cudaError_t function_attributes(const void* kernel, kernel_attributes& out);
+
 constexpr int render_block = 128;
 
 cudaError_t launch_render(const launch_params& p, bool quality, bool counting, int grid, cudaStream_t stream);
@@ -247,6 +250,27 @@ cudaError_t preload_wave_batch();
 // register cap)
 cudaError_t wave_attributes(const scene_view& scene, bool quality, kernel_attributes& shade, kernel_attributes& trace,
                             int trace_min_blocks = RTB_TRACE_MIN_BLOCKS_DEFAULT);
+
+// A launch of the pool kernel (the wavefront within a warp): each warp keeps its paths in shared memory and walks,
+// shades and starts them a warp's worth at a time. The samples' values go to `samples` as the wavefront's do.
+struct pool_run
+{
+    float4* samples;
+    int64_t sample_count;
+    int32_t claim; // samples a warp claims at a time, 1..32
+    int32_t pad0;
+};
+// Whether a session's AUTO renders a scene by the pool kernel: of those that suit the wavefront, the scenes searched
+// flat or through a tree four wide. Not those with triangles: a large mesh's walks live on the L1 cache that the paths
+// would take (the 1.3M-triangle mesh 2.7 G segments/s by the wavefront's steps, 1.75 here).
+inline bool pool_suits(const scene_view& v)
+{
+    return wavefront_suits(v) && (v.flat != 0 || v.wide_nodes != nullptr) && v.prim_count == v.triangle_base;
+}
+// Claims, renders and writes out every sample of the launch (`grid` blocks fill the GPU; a small launch takes fewer)
+cudaError_t launch_pool(const launch_params& p, bool quality, float4* samples, int64_t sample_count, int grid,
+                        cudaStream_t stream);
+cudaError_t pool_attributes(const scene_view& scene, bool quality, kernel_attributes& out);
 
 // The books' integrator in double (precision::float64; renderer.h:402-409, all_books_kernel<double>,
 // renderer.cu:445-451): a persistent launch over the same (pixel, chunk) work items as launch_params' and into the

@@ -1,6 +1,8 @@
 // What every kernel that shades and walks shares: the arithmetic, the random numbers, the primitive tests and the tree
 // walk, the materials, lights and camera, one vertex of a path under either integrator, and where a sample lies in a
 // launch. Included by each source that has kernels of its own, inside namespace rtb's anonymous namespace.
+//
+// The including source defines `struct rounds` first: how each dot product below is rounded (see `rounding`).
 #pragma once
 
 // ---- float3 arithmetic --------------------------------------------------------------------------------------
@@ -9,17 +11,51 @@ __device__ __forceinline__ float3 operator-(float3 a, float3 b) { return make_fl
 __device__ __forceinline__ float3 operator-(float3 a) { return make_float3(-a.x, -a.y, -a.z); }
 __device__ __forceinline__ float3 operator*(float t, float3 v) { return make_float3(t * v.x, t * v.y, t * v.z); }
 __device__ __forceinline__ float3 operator*(float3 a, float3 b) { return make_float3(a.x * b.x, a.y * b.y, a.z * b.z); }
-__device__ __forceinline__ float dot(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+// A dot product's rounding, written out or left to the compiler. Left to it, a * b + c * d becomes one multiply-add or
+// the other by what surrounds it in each kernel, a last bit apart, and a path through glass makes another path of a
+// last bit; written out, two kernels that render the same samples render the same image.
+template <rounding R = rounds::other>
+__device__ __forceinline__ float dot(float3 a, float3 b)
+{
+    if constexpr (R == rounding::x) // x fused onto y's product, z onto both
+    {
+        return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
+    }
+    else if constexpr (R == rounding::y) // y fused onto x's product, z onto both
+    {
+        return __fmaf_rn(a.z, b.z, __fmaf_rn(a.y, b.y, __fmul_rn(a.x, b.x)));
+    }
+    else if constexpr (R == rounding::yz) // y fused onto x's product, z's product rounded and added
+    {
+        return __fadd_rn(__fmul_rn(a.z, b.z), __fmaf_rn(a.y, b.y, __fmul_rn(a.x, b.x)));
+    }
+    else
+    {
+        return a.x * b.x + a.y * b.y + a.z * b.z;
+    }
+}
 __device__ __forceinline__ float3 cross(float3 u, float3 v)
 {
     return make_float3(u.y * v.z - u.z * v.y, u.z * v.x - u.x * v.z, u.x * v.y - u.y * v.x);
 }
-__device__ __forceinline__ float length_squared(float3 v) { return dot(v, v); }
-__device__ __forceinline__ float3 unit_vector(float3 v) { return rsqrtf(length_squared(v)) * v; }
-__device__ __forceinline__ float3 reflect(float3 v, float3 n) { return v - (2.0f * dot(v, n)) * n; }
+template <rounding R = rounds::other>
+__device__ __forceinline__ float length_squared(float3 v)
+{
+    return dot<R>(v, v);
+}
+template <rounding R = rounds::other>
+__device__ __forceinline__ float3 unit_vector(float3 v)
+{
+    return rsqrtf(length_squared<R>(v)) * v;
+}
+template <rounding R = rounds::other>
+__device__ __forceinline__ float3 reflect(float3 v, float3 n)
+{
+    return v - (2.0f * dot<R>(v, n)) * n;
+}
 __device__ __forceinline__ float3 refract(float3 uv, float3 n, float etai_over_etat) // vec3.cuh refract
 {
-    const float cos_theta = fminf(dot(-uv, n), 1.0f);
+    const float cos_theta = fminf(dot<rounds::dielectric_cosine>(-uv, n), 1.0f);
     const float3 perp = etai_over_etat * (uv + cos_theta * n);
     const float3 parallel = (-sqrtf(fabsf(1.0f - length_squared(perp)))) * n;
     return perp + parallel;
@@ -738,7 +774,7 @@ RTB_FEATURE_FUNCTION void media_event(const scene_view& S, float3 o, float3 d, f
     const float inverse_a = 1.0f / length_squared(d);
     const float3 inv = make_float3(safe_inverse(d.x), safe_inverse(d.y), safe_inverse(d.z));
     const float3 os = make_float3(o.x * inv.x, o.y * inv.y, o.z * inv.z);
-    const float length = sqrtf(length_squared(d));
+    const float length = sqrtf(length_squared<rounds::flight>(d));
     float4 u = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     for (int k = 0; k < S.medium_count; ++k)
     {
@@ -1008,7 +1044,7 @@ __device__ bool sample_lamp(const emitter20& e, float3 x, float a, float b, lamp
     if (e.kind == RT_LIGHT_QUAD)
     {
         const float3 to = (corner - x) + a * make_float3(e.ux, e.uy, e.uz) + b * make_float3(e.vx, e.vy, e.vz);
-        const float distance_squared = length_squared(to);
+        const float distance_squared = length_squared<rounds::lamp_distance>(to);
         const float inverse_distance = rsqrtf(distance_squared);
         out.wi = inverse_distance * to;
         out.distance = distance_squared * inverse_distance;
@@ -1080,7 +1116,7 @@ __device__ __forceinline__ void camera_ray(const camera_params& cam, int i, int 
 
 __device__ __forceinline__ float3 sky(const camera_params& cam, float3 direction)
 {
-    const float a = 0.5f * (unit_vector(direction).y + 1.0f);
+    const float a = 0.5f * (unit_vector<rounds::sky>(direction).y + 1.0f);
     return (1.0f - a) * f3v(cam.sky_bottom) + a * f3v(cam.sky_top);
 }
 
@@ -1306,11 +1342,11 @@ __device__ __forceinline__ step_result shade_books(const scene_view& S, const ca
     else // dielectric
     {
         const float ri = h.front ? 1.0f / m.ior : m.ior;
-        const float3 ud = unit_vector(ps.d);
-        const float cos_theta = fminf(dot(-ud, s.normal), 1.0f);
+        const float3 ud = unit_vector<rounds::dielectric_unit>(ps.d);
+        const float cos_theta = fminf(dot<rounds::dielectric_cosine>(-ud, s.normal), 1.0f);
         const float sin_theta = sqrtf(1.0f - cos_theta * cos_theta);
         const bool cannot_refract = ri * sin_theta > 1.0f;
-        direction = cannot_refract || reflectance(cos_theta, ri) > u.z ? reflect(ud, s.normal)
+        direction = cannot_refract || reflectance(cos_theta, ri) > u.z ? reflect<rounds::dielectric_cosine>(ud, s.normal)
                                                                        : refract(ud, s.normal, ri);
     }
     if (--ps.rays_left == 0)
@@ -1354,13 +1390,14 @@ __device__ __forceinline__ float3 schlick(float3 f0, float cosine)
 }
 
 // f * cos(theta_l) = F D cl / (2 (cl A_v + cv A_l)) and the visible-normal density D / (2 (cv + A_v))
+template <rounding LENGTH>
 __device__ float3 ggx_eval(float3 n, float3 v, float3 l, float alpha, float3 f0, float& pdf)
 {
     pdf = 0.0f;
-    const float cv = dot(n, v);
+    const float cv = dot<rounds::ggx_eval_view>(n, v);
     const float cl = dot(n, l);
     const float3 sum = v + l;
-    const float len2 = length_squared(sum);
+    const float len2 = length_squared<LENGTH>(sum);
     if (!(cv > 0.0f) || !(cl > 0.0f) || !(len2 > 0.0f))
     {
         return make_float3(0.0f, 0.0f, 0.0f);
@@ -1371,7 +1408,7 @@ __device__ float3 ggx_eval(float3 n, float3 v, float3 l, float alpha, float3 f0,
     const float av = smith_a(cv, alpha2);
     const float al = smith_a(cl, alpha2);
     pdf = d / (2.0f * (cv + av));
-    return (d * cl / (2.0f * (cl * av + cv * al))) * schlick(f0, dot(v, h));
+    return (d * cl / (2.0f * (cl * av + cv * al))) * schlick(f0, dot<rounds::ggx_eval_half>(v, h));
 }
 
 // A direction by the visible normals with spherical caps: u1 the azimuth, u2 the height in the cap; weight
@@ -1379,7 +1416,7 @@ __device__ float3 ggx_eval(float3 n, float3 v, float3 l, float alpha, float3 f0,
 __device__ bool ggx_sample(float3 n, float3 v, float alpha, float3 f0, float u1, float u2, float3& l, float3& weight,
                            float& pdf)
 {
-    const float cv = dot(n, v);
+    const float cv = dot<rounds::ggx_sample_view>(n, v);
     if (!(cv > 0.0f))
     {
         return false;
@@ -1400,7 +1437,7 @@ __device__ bool ggx_sample(float3 n, float3 v, float alpha, float3 f0, float u1,
         return false;
     }
     const float3 h = rsqrtf(m2) * m;
-    const float vh = dot(v, h);
+    const float vh = dot<rounds::ggx_sample_half>(v, h);
     l = (2.0f * vh) * h - v;
     const float cl = dot(n, l);
     if (!(cl > 0.0f) || !(vh > 0.0f))
@@ -1445,6 +1482,7 @@ __device__ __forceinline__ float gloss_crossing(float c)
 
 // The coat over a matte base of color rho: GGX with F0 0.04 plus the coupled diffuse term; pdf the half-and-half
 // mixture of the two lobes' densities
+template <rounding LENGTH>
 __device__ float3 gloss_eval(float3 n, float3 v, float3 l, float alpha, float3 rho, float& pdf)
 {
     pdf = 0.0f;
@@ -1455,7 +1493,7 @@ __device__ float3 gloss_eval(float3 n, float3 v, float3 l, float alpha, float3 r
         return make_float3(0.0f, 0.0f, 0.0f);
     }
     float coat_pdf;
-    const float3 coat = ggx_eval(n, v, l, alpha, make_float3(gloss_coat_f0, gloss_coat_f0, gloss_coat_f0), coat_pdf);
+    const float3 coat = ggx_eval<LENGTH>(n, v, l, alpha, make_float3(gloss_coat_f0, gloss_coat_f0, gloss_coat_f0), coat_pdf);
     pdf = 0.5f * (coat_pdf + cl * inverse_pi_f);
     const float base = gloss_diffuse_scale * (gloss_crossing(cl) * gloss_crossing(cv)) * cl;
     return coat + base * rho;
@@ -1587,12 +1625,12 @@ __device__ float3 eval_lobe(int lobe, const material12& m, float3 albedo, float3
     }
     if (lobe == lobe_conductor)
     {
-        const float3 single = ggx_eval(n, wo, wi, m.alpha, albedo, pdf);
-        return ggx_compensation(albedo, dot(n, wo), m.roughness) * single;
+        const float3 single = ggx_eval<rounds::ggx_light_length>(n, wo, wi, m.alpha, albedo, pdf);
+        return ggx_compensation(albedo, dot<rounds::energy>(n, wo), m.roughness) * single;
     }
     if (lobe == lobe_gloss)
     {
-        return gloss_eval(n, wo, wi, m.alpha, albedo, pdf);
+        return gloss_eval<rounds::ggx_light_length>(n, wo, wi, m.alpha, albedo, pdf);
     }
     pdf = 0.0f;
     return make_float3(0.0f, 0.0f, 0.0f);
@@ -1653,8 +1691,8 @@ __device__ __forceinline__ step_result shade_quality(const scene_view& S, const 
             float p_light = 0.0f;
             if (k >= 0)
             {
-                const float distance = h.t * sqrtf(length_squared(ps.d));
-                p_light = S.light_pmf * lamp_pdf(S.lamps[k], ps.o, unit_vector(ps.d), distance);
+                const float distance = h.t * sqrtf(length_squared<rounds::lamp_hit>(ps.d));
+                p_light = S.light_pmf * lamp_pdf(S.lamps[k], ps.o, unit_vector<rounds::lamp_hit>(ps.d), distance);
             }
             w = bsdf_weight(S.combination, ps.bsdf_pdf, p_light);
         }
@@ -1663,7 +1701,7 @@ __device__ __forceinline__ step_result shade_quality(const scene_view& S, const 
     }
     const int lobe = lobe_of(m);
     const bool delta = lobe >= lobe_smooth_conductor;
-    const float3 wo = -unit_vector(ps.d);
+    const float3 wo = -unit_vector<rounds::view>(ps.d);
     const int lights = S.lamp_count + (S.env.sampled ? 1 : 0);
     const bool nee = S.combination != RT_COMBINE_BSDF_ONLY && ps.rays_left > 1 && !delta && lights > 0 &&
                      largest_channel(ps.throughput) > 0.0f;
@@ -1741,7 +1779,7 @@ __device__ __forceinline__ step_result shade_quality(const scene_view& S, const 
         scattered = ggx_sample(s.normal, wo, m.alpha, albedo, u.x, u.y, wi, weight, pdf);
         if (scattered)
         {
-            weight = weight * ggx_compensation(albedo, dot(s.normal, wo), m.roughness);
+            weight = weight * ggx_compensation(albedo, dot<rounds::energy>(s.normal, wo), m.roughness);
         }
     }
     else if (lobe == lobe_gloss)
@@ -1761,7 +1799,7 @@ __device__ __forceinline__ step_result shade_quality(const scene_view& S, const 
         }
         if (scattered)
         {
-            const float3 f = gloss_eval(s.normal, wo, wi, m.alpha, albedo, pdf);
+            const float3 f = gloss_eval<rounds::ggx_gloss_length>(s.normal, wo, wi, m.alpha, albedo, pdf);
             scattered = pdf > 0.0f;
             weight = (1.0f / pdf) * f;
         }
@@ -1781,10 +1819,10 @@ __device__ __forceinline__ step_result shade_quality(const scene_view& S, const 
     else // dielectric
     {
         const float ri = h.front ? 1.0f / m.ior : m.ior;
-        const float3 ud = unit_vector(ps.d);
-        const float cos_theta = fminf(dot(-ud, s.normal), 1.0f);
+        const float3 ud = unit_vector<rounds::dielectric_unit>(ps.d);
+        const float cos_theta = fminf(dot<rounds::dielectric_cosine>(-ud, s.normal), 1.0f);
         const float sin_theta = sqrtf(1.0f - cos_theta * cos_theta);
-        wi = ri * sin_theta > 1.0f || reflectance(cos_theta, ri) > u.z ? reflect(ud, s.normal)
+        wi = ri * sin_theta > 1.0f || reflectance(cos_theta, ri) > u.z ? reflect<rounds::dielectric_cosine>(ud, s.normal)
                                                                        : refract(ud, s.normal, ri);
         weight = make_float3(1.0f, 1.0f, 1.0f);
     }

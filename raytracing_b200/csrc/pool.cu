@@ -1,0 +1,63 @@
+// A session's renders by the pool kernel (pool_kernel.cuh): the kernels' instantiations and their launch.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+
+#include "ggx_energy_table.h"
+#include "kernels.cuh"
+#include "philox.cuh"
+#include "rounding.cuh"
+#include "rt_b200.h"
+
+namespace rtb
+{
+namespace
+{
+using rounds = rounds_session;
+#include "path.cuh"
+#include "pool_kernel.cuh"
+
+// Before a launch of the pool kernel: no sample claimed
+__global__ void pool_prepare_kernel(unsigned long long* work_counter) { *work_counter = 0ull; }
+
+using pool_function = void (*)(launch_params, pool_run, wave_batch);
+
+template <bool QUALITY, bool FEATURES>
+pool_function pool_kernel_of(bool flat)
+{
+    return flat ? pool_kernel<QUALITY, FEATURES, true, false> : pool_kernel<QUALITY, FEATURES, false, false>;
+}
+
+pool_function pool_kernel_for(bool quality, bool features, bool flat)
+{
+    if (quality)
+    {
+        return features ? pool_kernel_of<true, true>(flat) : pool_kernel_of<true, false>(flat);
+    }
+    return features ? pool_kernel_of<false, true>(flat) : pool_kernel_of<false, false>(flat);
+}
+} // namespace
+
+cudaError_t launch_pool(const launch_params& p, bool quality, float4* samples, int64_t sample_count, int grid,
+                        cudaStream_t stream)
+{
+    // A launch of fewer samples than lanes spreads them over the warps, so that every multiprocessor takes part
+    constexpr int64_t block_warps = render_block / 32;
+    const int64_t warps = grid * block_warps;
+    const auto claim = static_cast<int32_t>(std::clamp<int64_t>((sample_count + warps - 1) / warps, 1, 32));
+    const int64_t blocks = std::min<int64_t>(grid, (sample_count + claim * block_warps - 1) / (claim * block_warps));
+    const pool_run run{samples, sample_count, claim, 0};
+    pool_prepare_kernel<<<1, 1, 0, stream>>>(p.work_counter);
+    pool_kernel_for(quality, has_features(p.scene), p.scene.flat != 0)<<<static_cast<unsigned>(std::max<int64_t>(blocks, 1)),
+                                                                         render_block, 0, stream>>>(p, run, wave_batch{});
+    return cudaGetLastError();
+}
+
+cudaError_t pool_attributes(const scene_view& scene, bool quality, kernel_attributes& out)
+{
+    return function_attributes(reinterpret_cast<const void*>(
+                                   pool_kernel_for(quality, has_features(scene), scene.flat != 0)),
+                               out);
+}
+} // namespace rtb

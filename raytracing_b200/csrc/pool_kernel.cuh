@@ -1,0 +1,712 @@
+// The pool kernel: the wavefront within a warp. Included after path.cuh by each source that compiles it.
+//
+// A persistent warp keeps 64 paths in shared memory and, in turn, walks rays (32 lanes, each with a path of its own),
+// shades answered paths and starts new samples, each phase with as full a warp as the lists hold; a path is never bound
+// to a lane between phases. What it replaces: the wavefront's steps keep up to 3 x 2^20 paths in HBM and run two kernels
+// a step over all of them, so every segment paid 160 to 224 bytes of HBM traffic and a round through a queue, and every
+// launch ended with a drain of a path's length of nearly empty steps (a 400x225, 32-pass cover render spent 4.4 ms in
+// 128 steps for 1.3 ms of work). Against the one-lane-one-path persistent kernel, shading and searches run with full
+// warps. Bound by instruction issue, with the lanes that materials and walks of uneven depth leave idle.
+// Measured on the B200, GPU time, against the steps (images equal bit for bit): glass 600x600 x 256 47.0 -> 28.1 ms,
+// cornell-mis x 64 30.0 -> 17.9, weekend 400x225 x 32 4.36 -> 1.27, one pass of weekend at 256x256 1.35 -> 0.25,
+// final 400x400 x 100 19.9 -> 17.0, smoke 300x300 x 64 5.8 -> 1.9, checker 400x225 x 64 4.9 -> 0.85.
+
+// The lanes still walking under which a warp stops its walks to give the others something to do
+#ifndef RTB_POOL_REFILL_LANES
+#define RTB_POOL_REFILL_LANES 20
+#endif
+
+// A warp's paths: twice its lanes, so that while up to 32 of them walk, enough others wait for a full warp's shading
+#ifndef RTB_POOL_PATHS
+#define RTB_POOL_PATHS 64
+#endif
+constexpr int pool_paths = RTB_POOL_PATHS;
+
+// A path's record in shared memory, as words of a structure of arrays ([word][path]): a warp's reads of a word touch
+// consecutive banks but for the paths' order
+template <bool QUALITY, bool FEATURES, bool BATCH>
+struct pool_record
+{
+    static constexpr int o = 0;          // origin
+    static constexpr int d = 3;          // direction
+    static constexpr int throughput = 6;
+    static constexpr int pixel = 9;      // the random numbers' counter and key: pixel, pass in its round, key's high word
+    static constexpr int pass = 10;
+    static constexpr int key = 11;
+    static constexpr int sample = 12;    // the sample's number in the launch (a batch: within its job)
+    static constexpr int meta = 13;      // depth << 6 and the flags below
+    static constexpr int from = 14;      // the primitive the ray leaves
+    static constexpr int hit_t = 15;     // the walk's answer
+    static constexpr int hit = 16;       // id << 1 | front, or -1
+    static constexpr int time = 17;
+    static constexpr int job = time + (FEATURES ? 1 : 0);
+    static constexpr int radiance = job + (BATCH ? 1 : 0);
+    static constexpr int pdf = radiance + 3;
+    static constexpr int shadow_d = pdf + 1;
+    static constexpr int shadow_t = shadow_d + 3;
+    static constexpr int light = shadow_t + 1; // what the shadow ray brings if nothing blocks it
+    static constexpr int skip = light + 3;
+    static constexpr int words = QUALITY ? skip + 1 : radiance;
+};
+constexpr uint32_t pool_inward = 1u;        // the ray starts inside the surface it leaves
+constexpr uint32_t pool_specular = 2u;
+constexpr uint32_t pool_ext = 4u;           // the path goes on: its next ray is to be walked
+constexpr uint32_t pool_shadow = 8u;        // a shadow ray is to be walked (before the next ray)
+constexpr uint32_t pool_shadow_inward = 16u;
+constexpr uint32_t pool_blocked = 32u;      // the shadow ray's answer, where the shading needs it (smoke)
+
+#ifndef RTB_POOL_BLOCKS_TREE
+#define RTB_POOL_BLOCKS_TREE 7
+#endif
+#ifndef RTB_POOL_BLOCKS_FLAT
+#define RTB_POOL_BLOCKS_FLAT 8
+#endif
+#ifndef RTB_POOL_BLOCKS_QUALITY
+#define RTB_POOL_BLOCKS_QUALITY 5
+#endif
+#ifndef RTB_POOL_BLOCKS_FEATURES
+#define RTB_POOL_BLOCKS_FEATURES 5
+#endif
+template <bool QUALITY, bool FEATURES, bool FLAT, bool BATCH>
+constexpr int pool_min_blocks()
+{
+    return FEATURES ? RTB_POOL_BLOCKS_FEATURES
+                    : (QUALITY || BATCH ? RTB_POOL_BLOCKS_QUALITY : (FLAT ? RTB_POOL_BLOCKS_FLAT : RTB_POOL_BLOCKS_TREE));
+}
+
+template <bool QUALITY, bool FEATURES, bool FLAT, bool BATCH>
+__global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURES, FLAT, BATCH>())
+    pool_kernel(const __grid_constant__ launch_params P, const __grid_constant__ pool_run R,
+                const __grid_constant__ wave_batch W)
+{
+    using record = pool_record<QUALITY, FEATURES, BATCH>;
+    constexpr int warps = render_block / 32;
+    __shared__ uint32_t records[warps][record::words][pool_paths];
+    __shared__ uint8_t lists[warps][3][pool_paths];
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned lanes_below = (1u << lane) - 1u;
+    const int warp = static_cast<int>(threadIdx.x >> 5);
+    uint32_t(*const rec)[pool_paths] = records[warp];
+    uint8_t* const walk_list = lists[warp][0];  // paths with a ray to walk
+    uint8_t* const shade_list = lists[warp][1]; // paths with an answer to shade
+    uint8_t* const free_list = lists[warp][2];  // records without a sample
+    const auto put3 = [&](int word, int p, float3 v) {
+        rec[word][p] = __float_as_uint(v.x);
+        rec[word + 1][p] = __float_as_uint(v.y);
+        rec[word + 2][p] = __float_as_uint(v.z);
+    };
+    const auto get3 = [&](int word, int p) {
+        return make_float3(__uint_as_float(rec[word][p]), __uint_as_float(rec[word + 1][p]),
+                           __uint_as_float(rec[word + 2][p]));
+    };
+    // The lanes for which `which` holds append their path to a list; its new length
+    const auto push = [&](uint8_t* list, int count, bool which, int p) -> int {
+        const unsigned lanes = __ballot_sync(full_warp, which);
+        if (which)
+        {
+            list[count + __popc(lanes & lanes_below)] = static_cast<uint8_t>(p);
+        }
+        return count + __popc(lanes);
+    };
+    for (int p = static_cast<int>(lane); p < pool_paths; p += 32)
+    {
+        free_list[p] = static_cast<uint8_t>(p);
+    }
+    int walk_count = 0;
+    int shade_count = 0;
+    int free_count = pool_paths;
+    const auto limit = static_cast<unsigned long long>(R.sample_count);
+    bool dry = limit == 0ull; // every sample of the launch is claimed
+    uint32_t rays = 0, shadow_rays = 0;
+    __syncwarp();
+
+    // The lane's walk (tree-searched scenes): the path it walks for (-1: none) and the walk's state
+    int slot = -1;
+    bool shadow = false;
+    int link = traversal_done;
+    int leaf = 0;
+    int sp = 0;
+    hit_info hit{-1, 0.0f, false};
+    int2 stack[FLAT ? 1 : wide_stack];
+
+    const auto job_of = [&](int p) -> const batch_job* { return BATCH ? W.jobs + rec[record::job][p] : nullptr; };
+
+    while (true)
+    {
+        enum class phase
+        {
+            walk,
+            start,
+            shade,
+            end
+        } next;
+        float3 o = make_float3(0.0f, 0.0f, 0.0f);
+        float3 d = o;
+        float time = 0.0f;
+        int from = -1, skip = -1;
+        bool inward = false;
+        if constexpr (!FLAT)
+        {
+            // The answered walks: a shadow ray's light is added (or lost), then its path's next ray is walked by the
+            // same lane; a next ray's hit goes to the shading
+            const bool answered = slot >= 0 && link == traversal_done && leaf == 0;
+            bool fresh = false;
+            bool to_shade = false, to_free = false;
+            const int was = slot;
+            if (answered)
+            {
+                if (QUALITY && shadow)
+                {
+                    uint32_t meta = rec[record::meta][slot];
+                    if constexpr (FEATURES)
+                    {
+                        meta |= hit.id >= 0 ? pool_blocked : 0u;
+                    }
+                    else
+                    {
+                        meta &= ~pool_shadow;
+                        if (hit.id < 0)
+                        {
+                            put3(record::radiance, slot, get3(record::radiance, slot) + get3(record::light, slot));
+                        }
+                    }
+                    rec[record::meta][slot] = meta;
+                    shadow = false;
+                    if (meta & pool_ext)
+                    {
+                        fresh = true;
+                    }
+                    else if (FEATURES)
+                    {
+                        to_shade = true;
+                        slot = -1;
+                    }
+                    else
+                    {
+                        const float3 sample = get3(record::radiance, slot);
+                        const batch_job* J = job_of(slot);
+                        stream_store(R.samples + (BATCH ? J->sample_begin : 0) + rec[record::sample][slot],
+                                     make_float4(sample.x, sample.y, sample.z, 0.0f));
+                        to_free = true;
+                        slot = -1;
+                    }
+                }
+                else
+                {
+                    rec[record::hit_t][slot] = __float_as_uint(hit.t);
+                    rec[record::hit][slot] = hit.id < 0 ? 0xffffffffu
+                                                        : (static_cast<uint32_t>(hit.id) << 1) | (hit.front ? 1u : 0u);
+                    to_shade = true;
+                    slot = -1;
+                }
+            }
+            shade_count = push(shade_list, shade_count, to_shade, was);
+            if (QUALITY && !FEATURES)
+            {
+                free_count = push(free_list, free_count, to_free, was);
+            }
+            // New rays for the idle lanes
+            const unsigned idle = __ballot_sync(full_warp, slot < 0);
+            const int taken = min(__popc(idle), walk_count);
+            const int rank = __popc(idle & lanes_below);
+            __syncwarp();
+            if (slot < 0 && rank < taken)
+            {
+                slot = walk_list[walk_count - 1 - rank];
+                fresh = true;
+                shadow = QUALITY && (rec[record::meta][slot] & pool_shadow) != 0u;
+            }
+            walk_count -= taken;
+            if (fresh)
+            {
+                hit = {-1, QUALITY && shadow ? __uint_as_float(rec[record::shadow_t][slot]) : infinity_f, false};
+                sp = 0;
+                leaf = 0;
+                const scene_view& S = BATCH ? job_of(slot)->scene : P.scene;
+                link = S.node_count == 0 ? traversal_done : 0;
+            }
+            const int walking = __popc(__ballot_sync(full_warp, slot >= 0));
+            const int startable = dry ? 0 : free_count;
+            // Few walks left and no ray to refill the lanes with: shade or start, whichever has the fuller warp
+            const bool few = walking < RTB_POOL_REFILL_LANES && walking * 8 < (walking + shade_count + startable) * 5;
+            if (walk_count == 0 && few)
+            {
+                next = startable > shade_count ? phase::start : phase::shade;
+            }
+            else
+            {
+                next = walking > 0 ? phase::walk : phase::end;
+            }
+        }
+        else
+        {
+            const int startable = dry ? 0 : free_count;
+            if (walk_count >= 32 || (walk_count >= startable && walk_count >= shade_count))
+            {
+                next = walk_count > 0 ? phase::walk : phase::end;
+            }
+            else
+            {
+                next = startable > shade_count ? phase::start : phase::shade;
+            }
+        }
+        if (next == phase::end)
+        {
+            break;
+        }
+        if (next == phase::walk)
+        {
+            if constexpr (FLAT)
+            {
+                const int taken = min(32, walk_count);
+                const bool mine = static_cast<int>(lane) < taken;
+                const int p = mine ? walk_list[walk_count - taken + static_cast<int>(lane)] : 0;
+                walk_count -= taken;
+                bool to_shade = false, to_free = false;
+                if (mine)
+                {
+                    const batch_job* J = job_of(p);
+                    const scene_view& S = BATCH ? J->scene : P.scene;
+                    uint32_t meta = rec[record::meta][p];
+                    o = get3(record::o, p);
+                    time = FEATURES ? __uint_as_float(rec[record::time][p]) : 0.0f;
+                    from = static_cast<int>(rec[record::from][p]);
+#pragma unroll 1
+                    for (int k = QUALITY ? 0 : 1; k < 2; ++k)
+                    {
+                        // the shadow ray first, then the next ray
+                        const bool any = QUALITY && k == 0;
+                        if ((meta & (any ? pool_shadow : pool_ext)) == 0u)
+                        {
+                            continue;
+                        }
+                        d = get3(QUALITY && any ? record::shadow_d : record::d, p);
+                        hit_info h{-1, QUALITY && any ? __uint_as_float(rec[record::shadow_t][p]) : infinity_f, false};
+                        flat_search<FEATURES>(S, o, d, time, from,
+                                              (meta & (any ? pool_shadow_inward : pool_inward)) != 0u,
+                                              QUALITY && any ? static_cast<int>(rec[record::skip][p]) : -1, any, h);
+                        if (!any)
+                        {
+                            rec[record::hit_t][p] = __float_as_uint(h.t);
+                            rec[record::hit][p] = h.id < 0 ? 0xffffffffu
+                                                           : (static_cast<uint32_t>(h.id) << 1) | (h.front ? 1u : 0u);
+                        }
+                        else if (FEATURES)
+                        {
+                            meta |= h.id >= 0 ? pool_blocked : 0u;
+                        }
+                        else
+                        {
+                            meta &= ~pool_shadow;
+                            if (h.id < 0)
+                            {
+                                put3(record::radiance, p, get3(record::radiance, p) + get3(record::light, p));
+                            }
+                        }
+                    }
+                    to_shade = true;
+                    if (QUALITY)
+                    {
+                        rec[record::meta][p] = meta;
+                        if (!FEATURES && (meta & pool_ext) == 0u)
+                        {
+                            const float3 sample = get3(record::radiance, p);
+                            stream_store(R.samples + (BATCH ? J->sample_begin : 0) + rec[record::sample][p],
+                                         make_float4(sample.x, sample.y, sample.z, 0.0f));
+                            to_shade = false;
+                            to_free = true;
+                        }
+                    }
+                }
+                shade_count = push(shade_list, shade_count, to_shade, p);
+                if (QUALITY && !FEATURES)
+                {
+                    free_count = push(free_list, free_count, to_free, p);
+                }
+            }
+            else
+            {
+                // The walks: the trace kernel's, until too few lanes walk or all are answered
+                const scene_view& S = BATCH && slot >= 0 ? job_of(slot)->scene : (BATCH ? W.jobs[W.job_first].scene : P.scene);
+                const bvh4_node* const tree = S.wide_nodes;
+                float inverse_a = 0.0f;
+                float3 inv = o, os = o;
+                if (slot >= 0)
+                {
+                    const uint32_t meta = rec[record::meta][slot];
+                    o = get3(record::o, slot);
+                    d = get3(QUALITY && shadow ? record::shadow_d : record::d, slot);
+                    time = FEATURES ? __uint_as_float(rec[record::time][slot]) : 0.0f;
+                    from = static_cast<int>(rec[record::from][slot]);
+                    skip = QUALITY && shadow ? static_cast<int>(rec[record::skip][slot]) : -1;
+                    inward = (meta & (QUALITY && shadow ? pool_shadow_inward : pool_inward)) != 0u;
+                    inverse_a = 1.0f / (FEATURES ? length_squared<rounds::walk_features>(d) : length_squared(d));
+                    inv = make_float3(safe_inverse(d.x), safe_inverse(d.y), safe_inverse(d.z));
+                    os = make_float3(o.x * inv.x, o.y * inv.y, o.z * inv.z);
+                }
+                const bool has_query = slot >= 0;
+                const auto pop = [&]() -> int {
+                    while (sp > 0)
+                    {
+                        const int2 e = stack[--sp];
+                        if ((QUALITY && shadow) || __int_as_float(e.y) < hit.t)
+                        {
+                            return e.x;
+                        }
+                    }
+                    return traversal_done;
+                };
+                const int total = __popc(__ballot_sync(full_warp, has_query)) + walk_count + shade_count +
+                                  (dry ? 0 : free_count);
+                const int enough = min(RTB_POOL_REFILL_LANES, (total * 5 + 7) / 8);
+                while (true)
+                {
+                    while (true)
+                    {
+                        const bool descending = has_query && link >= 0;
+                        if (!__any_sync(full_warp, descending))
+                        {
+                            break;
+                        }
+                        if (descending)
+                        {
+                            const float4* np = reinterpret_cast<const float4*>(tree + link);
+                            const float4 lx = __ldg(np), hx = __ldg(np + 1);
+                            const float4 ly = __ldg(np + 2), hy = __ldg(np + 3);
+                            const float4 lz = __ldg(np + 4), hz = __ldg(np + 5);
+                            const int4 nl = __ldg(reinterpret_cast<const int4*>(np + 6));
+                            const auto entry = [&](float lox, float hix, float loy, float hiy, float loz, float hiz,
+                                                   int child) -> float {
+                                const float a0 = fmaf(lox, inv.x, -os.x), a1 = fmaf(hix, inv.x, -os.x);
+                                const float b0 = fmaf(loy, inv.y, -os.y), b1 = fmaf(hiy, inv.y, -os.y);
+                                const float c0 = fmaf(loz, inv.z, -os.z), c1 = fmaf(hiz, inv.z, -os.z);
+                                const float enter =
+                                    fmaxf(fmaxf(fminf(a0, a1), fminf(b0, b1)), fmaxf(fminf(c0, c1), t_min));
+                                const float exit =
+                                    fminf(fminf(fmaxf(a0, a1), fmaxf(b0, b1)), fminf(fmaxf(c0, c1), hit.t));
+                                return enter <= exit && child != traversal_done ? enter : infinity_f;
+                            };
+                            float k0 = entry(lx.x, hx.x, ly.x, hy.x, lz.x, hz.x, nl.x);
+                            float k1 = entry(lx.y, hx.y, ly.y, hy.y, lz.y, hz.y, nl.y);
+                            float k2 = entry(lx.z, hx.z, ly.z, hy.z, lz.z, hz.z, nl.z);
+                            float k3 = entry(lx.w, hx.w, ly.w, hy.w, lz.w, hz.w, nl.w);
+                            int l0 = nl.x, l1 = nl.y, l2 = nl.z, l3 = nl.w;
+                            const auto order = [](float& ka, int& la, float& kb, int& lb) {
+                                if (kb < ka)
+                                {
+                                    const float k = ka;
+                                    ka = kb;
+                                    kb = k;
+                                    const int l = la;
+                                    la = lb;
+                                    lb = l;
+                                }
+                            };
+                            order(k0, l0, k1, l1);
+                            order(k2, l2, k3, l3);
+                            order(k0, l0, k2, l2);
+                            order(k1, l1, k3, l3);
+                            order(k1, l1, k2, l2);
+                            if (k0 == infinity_f)
+                            {
+                                link = pop();
+                            }
+                            else
+                            {
+                                if (k3 != infinity_f)
+                                {
+                                    stack[sp++] = make_int2(l3, __float_as_int(k3));
+                                }
+                                if (k2 != infinity_f)
+                                {
+                                    stack[sp++] = make_int2(l2, __float_as_int(k2));
+                                }
+                                if (k1 != infinity_f)
+                                {
+                                    stack[sp++] = make_int2(l1, __float_as_int(k1));
+                                }
+                                link = l0;
+                            }
+                            if (link < 0 && link != traversal_done && leaf == 0)
+                            {
+                                leaf = link;
+                                link = pop();
+                            }
+                        }
+                        if (!__any_sync(full_warp, has_query && link >= 0 && leaf == 0))
+                        {
+                            break;
+                        }
+                    }
+                    while (true)
+                    {
+                        const bool testing = has_query && leaf < 0;
+                        if (!__any_sync(full_warp, testing))
+                        {
+                            break;
+                        }
+                        if (testing)
+                        {
+                            if (test_leaf<false, false, FEATURES>(S, leaf, o, d, time, inverse_a, from, inward, skip, hit,
+                                                                  nullptr, QUALITY && shadow))
+                            {
+                                hit.id = 1; // a shadow ray's blocker: answered
+                                leaf = 0;
+                                link = traversal_done;
+                            }
+                            else
+                            {
+                                leaf = 0;
+                                if (link < 0 && link != traversal_done)
+                                {
+                                    leaf = link;
+                                    link = pop();
+                                }
+                            }
+                        }
+                    }
+                    const int walking =
+                        __popc(__ballot_sync(full_warp, has_query && !(link == traversal_done && leaf == 0)));
+                    if (walking < enough)
+                    {
+                        break;
+                    }
+                }
+            }
+            __syncwarp();
+            continue;
+        }
+        if (next == phase::start)
+        {
+            // New samples, a warp's worth of consecutive numbers at a time: a tile's pixels, their camera rays made
+            // side by side
+            const int wanted = min(min(32, free_count), R.claim);
+            unsigned long long base = 0;
+            if (lane == 0u)
+            {
+                base = atomicAdd(BATCH ? W.work_counter : P.work_counter, static_cast<unsigned long long>(wanted));
+            }
+            base = __shfl_sync(full_warp, base, 0);
+            dry = base + static_cast<unsigned long long>(wanted) >= limit;
+            const unsigned long long s = base + lane;
+            bool started = static_cast<int>(lane) < wanted && s < limit;
+            int job = 0;
+            const batch_job* J = nullptr;
+            if (BATCH && started)
+            {
+                job = find_job<job_samples>(W.jobs, W.job_first, W.job_end, static_cast<int64_t>(s));
+                J = W.jobs + job;
+            }
+            const camera_params& cam = BATCH && started ? J->cam : P.cam;
+            const int64_t index = static_cast<int64_t>(s) - (BATCH && started ? J->sample_begin : 0);
+            sample_place at{0, 0, 0};
+            if (started)
+            {
+                at = place_of(index, cam, BATCH ? J->pass_begin : P.pass_begin);
+                started = at.x < cam.width && at.y < cam.height; // a lane of a tile over the image's edge: no sample
+            }
+            const unsigned lanes = __ballot_sync(full_warp, started);
+            const int p = started ? free_list[free_count - 1 - __popc(lanes & lanes_below)] : 0;
+            __syncwarp();
+            free_count -= __popc(lanes);
+            if (started)
+            {
+                sampler rng;
+                rng.job = BATCH ? J->job : P.job;
+                const int round_pass = sample_rng(at, cam, BATCH ? J->seed : P.seed, rng);
+                int s_i, s_j;
+                stratum_of(cam, round_pass, s_i, s_j);
+                camera_ray(cam, at.x, at.y, s_i, s_j, rng.draw(0, 0), o, d);
+                put3(record::o, p, o);
+                put3(record::d, p, d);
+                put3(record::throughput, p, make_float3(1.0f, 1.0f, 1.0f));
+                rec[record::pixel][p] = rng.pixel;
+                rec[record::pass][p] = rng.pass;
+                rec[record::key][p] = rng.key.y;
+                rec[record::sample][p] = static_cast<uint32_t>(index);
+                rec[record::meta][p] = pool_specular | pool_ext;
+                rec[record::from][p] = 0xffffffffu;
+                if constexpr (FEATURES)
+                {
+                    const scene_view& S = BATCH ? J->scene : P.scene;
+                    rec[record::time][p] = __float_as_uint(S.has_motion ? rng.draw(0, block_time).x : 0.0f);
+                }
+                if constexpr (BATCH)
+                {
+                    rec[record::job][p] = static_cast<uint32_t>(job);
+                }
+                if constexpr (QUALITY)
+                {
+                    put3(record::radiance, p, make_float3(0.0f, 0.0f, 0.0f));
+                    rec[record::pdf][p] = 0u;
+                }
+            }
+            walk_count = push(walk_list, walk_count, started, p);
+            if constexpr (BATCH)
+            {
+                const unsigned peers = __match_any_sync(full_warp, started ? job : -1);
+                if (started && (peers & lanes_below) == 0u)
+                {
+                    atomicAdd(J->counters, static_cast<unsigned long long>(__popc(peers)));
+                }
+            }
+            else
+            {
+                rays += static_cast<uint32_t>(__popc(lanes));
+            }
+            __syncwarp();
+            continue;
+        }
+        // The shading of the answered paths, as the wavefront's shade kernel does it
+        const int taken = min(32, shade_count);
+        const bool mine = static_cast<int>(lane) < taken;
+        const int p = mine ? shade_list[shade_count - taken + static_cast<int>(lane)] : 0;
+        shade_count -= taken;
+        bool goes_on = false;
+        bool lit = false;
+        int job = 0;
+        const batch_job* J = nullptr;
+        if (mine)
+        {
+            job = BATCH ? static_cast<int>(rec[record::job][p]) : 0;
+            J = BATCH ? W.jobs + job : nullptr;
+            const scene_view& S = BATCH ? J->scene : P.scene;
+            const camera_params& cam = BATCH ? J->cam : P.cam;
+            const uint32_t meta = rec[record::meta][p];
+            path_state ps;
+            ps.o = get3(record::o, p);
+            ps.d = get3(record::d, p);
+            ps.throughput = get3(record::throughput, p);
+            ps.radiance = QUALITY ? get3(record::radiance, p) : make_float3(0.0f, 0.0f, 0.0f);
+            ps.bsdf_pdf = QUALITY ? __uint_as_float(rec[record::pdf][p]) : 0.0f;
+            ps.specular = (meta & pool_specular) != 0u;
+            ps.inward = (meta & pool_inward) != 0u;
+            ps.depth = static_cast<int>(meta >> 6);
+            ps.rays_left = cam.max_depth - ps.depth;
+            ps.from = static_cast<int>(rec[record::from][p]);
+            ps.time = FEATURES ? __uint_as_float(rec[record::time][p]) : 0.0f;
+            sampler rng;
+            rng.pixel = rec[record::pixel][p];
+            rng.pass = rec[record::pass][p];
+            rng.key = make_uint2(static_cast<uint32_t>(BATCH ? J->seed : P.seed), rec[record::key][p]);
+            rng.job = BATCH ? J->job : P.job;
+            float3 sample = make_float3(0.0f, 0.0f, 0.0f);
+            bool finished = false;
+            shadow_query sq;
+            sq.lit = false;
+            if constexpr (QUALITY && FEATURES)
+            {
+                if (meta & pool_shadow)
+                {
+                    if ((meta & pool_blocked) == 0u)
+                    {
+                        const float through = S.medium_count > 0
+                                                  ? transmittance(S, ps.o, get3(record::shadow_d, p), ps.time,
+                                                                  __uint_as_float(rec[record::shadow_t][p]))
+                                                  : 1.0f;
+                        ps.radiance = ps.radiance + through * get3(record::light, p);
+                    }
+                    if ((meta & pool_ext) == 0u)
+                    {
+                        sample = ps.radiance;
+                        finished = true;
+                    }
+                }
+            }
+            if (!finished)
+            {
+                const uint32_t answer = rec[record::hit][p];
+                hit_info h;
+                h.id = static_cast<int>(answer) < 0 ? -1 : static_cast<int>(answer >> 1);
+                h.t = __uint_as_float(rec[record::hit_t][p]);
+                h.front = (answer & 1u) != 0u;
+                ++ps.depth;
+                if (FEATURES && S.medium_count > 0)
+                {
+                    media_event(S, ps.o, ps.d, ps.time, rng, ps.depth, h);
+                }
+                step_result res;
+                if (QUALITY && (!BATCH || J->quality != 0))
+                {
+                    res = shade_quality<false, search_tree, FEATURES, true>(S, cam, rng, ps, h, sample, shadow_rays,
+                                                                            nullptr, &sq);
+                }
+                else
+                {
+                    res = shade_books<FEATURES>(S, cam, rng, ps, h, sample);
+                }
+                goes_on = res == step_result::go_on;
+                lit = QUALITY && sq.lit;
+                finished = !goes_on && !lit;
+                if (!finished)
+                {
+                    put3(record::o, p, QUALITY && !goes_on ? sq.o : ps.o);
+                    put3(record::d, p, ps.d);
+                    put3(record::throughput, p, ps.throughput);
+                    rec[record::from][p] = static_cast<uint32_t>(QUALITY && !goes_on ? sq.from : ps.from);
+                    rec[record::meta][p] = (static_cast<uint32_t>(ps.depth) << 6) | (ps.inward ? pool_inward : 0u) |
+                                           (ps.specular ? pool_specular : 0u) | (goes_on ? pool_ext : 0u) |
+                                           (lit ? pool_shadow : 0u) | (lit && sq.inward ? pool_shadow_inward : 0u);
+                    if constexpr (QUALITY)
+                    {
+                        put3(record::radiance, p, ps.radiance);
+                        rec[record::pdf][p] = __float_as_uint(ps.bsdf_pdf);
+                        if (lit)
+                        {
+                            put3(record::shadow_d, p, sq.d);
+                            rec[record::shadow_t][p] = __float_as_uint(sq.t_max);
+                            put3(record::light, p, sq.contribution);
+                            rec[record::skip][p] = static_cast<uint32_t>(sq.skip);
+                        }
+                    }
+                }
+            }
+            if (finished)
+            {
+                stream_store(R.samples + (BATCH ? J->sample_begin : 0) + rec[record::sample][p],
+                             make_float4(sample.x, sample.y, sample.z, 0.0f));
+            }
+        }
+        const bool queued = goes_on || lit;
+        walk_count = push(walk_list, walk_count, queued, p);
+        free_count = push(free_list, free_count, mine && !queued, p);
+        if constexpr (BATCH)
+        {
+            const unsigned on = __ballot_sync(full_warp, goes_on);
+            const unsigned lights = __ballot_sync(full_warp, lit);
+            const unsigned peers = __match_any_sync(full_warp, queued ? job : -1);
+            if (queued && (peers & lanes_below) == 0u)
+            {
+                const unsigned e = __popc(peers & on), sh = __popc(peers & lights);
+                if (e)
+                {
+                    atomicAdd(J->counters, static_cast<unsigned long long>(e));
+                }
+                if (sh)
+                {
+                    atomicAdd(J->counters + 1, static_cast<unsigned long long>(sh));
+                }
+            }
+        }
+        else
+        {
+            rays += static_cast<uint32_t>(__popc(__ballot_sync(full_warp, goes_on)));
+        }
+        __syncwarp();
+    }
+    if constexpr (!BATCH)
+    {
+        if (lane == 0u && rays != 0u)
+        {
+            atomicAdd(P.counters, static_cast<unsigned long long>(rays));
+        }
+        if constexpr (QUALITY)
+        {
+            const unsigned total = __reduce_add_sync(full_warp, shadow_rays);
+            if (lane == 0u && total != 0u)
+            {
+                atomicAdd(P.counters + 1, static_cast<unsigned long long>(total));
+            }
+        }
+    }
+}

@@ -74,6 +74,13 @@ session::session(std::shared_ptr<resident_scene> scene, const rt_session_options
     wavefront_ = !f64_ &&
                  (options_.form == RT_FORM_WAVEFRONT || (options_.form == RT_FORM_AUTO && wavefront_suits(view)));
     multiprocessors_ = a.multiprocessors;
+    pool_ = wavefront_ && options_.form == RT_FORM_AUTO && pool_suits(view);
+    if (pool_)
+    {
+        kernel_attributes pool{};
+        check(pool_attributes(view, scene_->quality(), pool), "querying the pool kernel");
+        pool_grid_ = pool.multiprocessors * std::max(1, pool.blocks_per_sm);
+    }
     if (wavefront_)
     {
         kernel_attributes shade{}, trace{};
@@ -143,6 +150,7 @@ void session::set_tuning(const rt_tuning& t)
     {
         fail(RT_ERR_INVALID, "shade_block must be 64 or 128");
     }
+    pool_ = false; // a shape asks for the steps that it shapes
     apply({t.slots, t.trace_blocks_per_sm, t.shade_block, t.trace_min_blocks});
     tuning_.from_cache = 0;
     tuning_.trials = 0;
@@ -187,8 +195,7 @@ rt_tuning session::autotune(int64_t trial_passes)
     counting_ = false;
     // Each candidate: the best of two measured launches, each after a one-chunk launch (the planner's probe) from a
     // fresh image
-    const auto measure = [&](const tune_candidate& c) {
-        apply(c);
+    const auto speed = [&] {
         double best = 0;
         for (int k = 0; k < 2; ++k)
         {
@@ -199,6 +206,13 @@ rt_tuning session::autotune(int64_t trial_passes)
         }
         return best;
     };
+    const auto measure = [&](const tune_candidate& c) {
+        apply(c);
+        return speed();
+    };
+    // An AUTO session that renders by the pool kernel stays with it unless the steps' best shape is faster
+    const double pool_speed = pool_ ? speed() : 0.0;
+    pool_ = false;
     const tune_outcome o = coordinate_descent(tuned_, space, measure);
     counting_ = counting;
     tuning_.from_cache = 0;
@@ -206,6 +220,7 @@ rt_tuning session::autotune(int64_t trial_passes)
     tuning_.samples_per_second = o.best_speed;
     tuning_.default_samples_per_second = o.default_speed;
     apply(o.best);
+    pool_ = pool_speed > o.best_speed;
     remember_tuning(tune_key(scene_->device(), view, scene_->quality()), o.best);
     set_camera(camera_);
     return tuning_;
@@ -231,6 +246,7 @@ session::~session()
     wave_.reset(); // its arrays are freed on the stream, before it goes
     rgba_.release();
     partials_.release();
+    pool_samples_.release();
     sums_.release();
     counters_.release();
     if (start_)
@@ -347,7 +363,16 @@ double session::launch(int64_t end)
 
     check(cudaMemsetAsync(counters_.data(), 0, sizeof(unsigned long long), stream_), "resetting the work counter");
     wave_buffers b{};
-    if (wave)
+    const bool pool = wave && pool_;
+    const int64_t samples = static_cast<int64_t>(padded_pixels_) * (end - passes_);
+    if (pool)
+    {
+        if (pool_samples_.size() < static_cast<size_t>(samples))
+        {
+            pool_samples_.allocate_async(std::max(static_cast<size_t>(samples), 2 * pool_samples_.size()), stream_);
+        }
+    }
+    else if (wave)
     {
         // allocated before the timing starts
         b = wave_->setup(static_cast<int64_t>(padded_pixels_) * (end - passes_), stream_);
@@ -355,7 +380,18 @@ double session::launch(int64_t end)
     check(cudaEventRecord(start_, stream_), "recording a CUDA event");
     int64_t steps = 0;
     cudaEvent_t* reduce_marks = timing_ ? marks(2) : nullptr;
-    if (wave)
+    if (pool)
+    {
+        b.samples = pool_samples_.data();
+        check(launch_pool(p, scene_->quality(), b.samples, samples, pool_grid_, stream_), "launching the pool kernel");
+        last_kernel_launches_ = 3;
+        if (timing_)
+        {
+            check(cudaEventRecord(reduce_marks[0], stream_), "recording a CUDA event");
+        }
+        check(launch_wave_reduce(r, b, p.pass_begin, p.pass_end, p.chunk, stream_), "launching the reduction");
+    }
+    else if (wave)
     {
         const bool quality = scene_->quality();
         steps = wave_->run(
@@ -426,7 +462,13 @@ double session::launch(int64_t end)
             check(cudaEventElapsedTime(&ms, a, b), "timing a kernel");
             return ms / 1000.0;
         };
-        if (wave)
+        if (pool)
+        {
+            times_.seconds[RT_KERNEL_RENDER] += elapsed(start_, marks_[0]);
+            ++times_.launches[RT_KERNEL_RENDER];
+            times_.seconds[RT_KERNEL_REDUCE] += elapsed(marks_[0], marks_[1]);
+        }
+        else if (wave)
         {
             for (int64_t k = 0; k < steps; ++k)
             {
@@ -450,8 +492,8 @@ double session::launch(int64_t end)
     float ms = 0;
     check(cudaEventElapsedTime(&ms, start_, stop_), "timing the GPU");
     const double seconds = std::max(1e-6, ms / 1000.0);
-    const double samples = static_cast<double>(camera_.image_width) * camera_.image_height * static_cast<double>(end - passes_);
-    samples_per_second_ = samples / seconds;
+    const double rendered = static_cast<double>(camera_.image_width) * camera_.image_height * static_cast<double>(end - passes_);
+    samples_per_second_ = rendered / seconds;
     passes_ = end;
     kernel_seconds_ += seconds;
     return seconds;
@@ -593,7 +635,11 @@ uint64_t session::shadow_rays() const
 rt_kernel_info session::kernel() const
 {
     kernel_attributes a{};
-    if (wavefront_ && !counting_)
+    if (pool_ && !counting_)
+    {
+        check(pool_attributes(scene_->view(), scene_->quality(), a), "querying the pool kernel");
+    }
+    else if (wavefront_ && !counting_)
     {
         kernel_attributes shade{};
         check(wave_attributes(scene_->view(), scene_->quality(), shade, a, shape_.trace_min_blocks),

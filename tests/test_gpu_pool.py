@@ -1,0 +1,52 @@
+"""The pool kernel (a session's AUTO form) against the wavefront's steps on a B200, through the C-ABI.
+
+Both render the same samples through the same arithmetic, rounding included, and add them in the same order, so the
+images and the counts are equal, with no tolerance. Sizes where the pool can go wrong: one sample; fewer samples than a
+warp; images whose tiles hang over both edges (claimed numbers without a pixel); more samples than every warp's paths;
+several launches; paths of one segment. Scenes: both searches, both integrators, with and without the second book's
+features.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SCENES = [("weekend", {}), ("weekend", dict(combination="mis")), ("glass", {}), ("glass", dict(sampling="lights")),
+          ("cornell-mis", {}), ("final", {}), ("bouncing", {}), ("smoke", {}), ("smoke", dict(combination="mis")),
+          ("perlin", {}), ("light", dict(combination="mis")), ("ggx-furnace", {})]
+SIZES = [(1, 1, 1, 0), (3, 5, 2, 0), (37, 21, 19, 0), (130, 67, 33, 0), (64, 64, 16, 1), (64, 64, 16, 2)]
+
+
+def _equal(rt, scene, seed, passes, **kw):
+    a = rt.Session(scene, seed=seed, **kw)
+    b = rt.Session(scene, seed=seed, form="wavefront", **kw)
+    assert a.render_to(passes)["kernel_launches"] < b.render_to(passes)["kernel_launches"]
+    assert np.array_equal(a.pixels(), b.pixels())
+    ca, cb = a.counters(), b.counters()
+    assert (ca["rays"], ca["shadow_rays"]) == (cb["rays"], cb["shadow_rays"])
+
+
+@pytest.mark.parametrize("name,kw", SCENES, ids=[f"{n}-{'-'.join(k.values())}" for n, k in SCENES])
+def test_pool_equals_the_wavefronts_steps(rt, name, kw):
+    for width, height, passes, depth in SIZES:
+        scene = rt.Scene(rt.builtin_scene(name, width=width, height=height, spp=passes, depth=depth, **kw))
+        _equal(rt, scene, 11, passes)
+
+
+@pytest.mark.parametrize("name", ["weekend", "glass"])
+def test_pool_many_samples_and_launches(rt, name):
+    # 8.9M samples in three launches: every warp's paths are renewed many times
+    scene = rt.Scene(rt.builtin_scene(name, width=521, height=357, spp=48))
+    _equal(rt, scene, 3, 48, launch_seconds=1e-4)
+
+
+def test_a_tuned_session_takes_the_steps(rt):
+    scene = rt.Scene(rt.builtin_scene("weekend", width=64, spp=16))
+    s = rt.Session(scene, seed=2)
+    s.render_to(16)
+    image, launches = s.pixels(), s.render_to(16)["launches"]
+    assert launches == 0
+    t = rt.Session(scene, seed=2)
+    t.set_tuning({**t.tuning(), "slots": 1 << 19})
+    assert t.render_to(16)["kernel_launches"] > 3
+    assert np.array_equal(t.pixels(), image)
