@@ -260,13 +260,18 @@ struct pool_run
     int32_t claim; // samples a warp claims at a time, 1..32
     int32_t pad0;
 };
-// Whether a session's AUTO renders a scene by the pool kernel: of those that suit the wavefront, the scenes searched
-// flat or through a tree four wide. Not those with triangles: a large mesh's walks live on the L1 cache that the paths
-// would take (the 1.3M-triangle mesh 2.7 G segments/s by the wavefront's steps, 1.75 here).
-inline bool pool_suits(const scene_view& v)
+// Whether a session's AUTO renders a scene by the pool kernel: one searched flat, or through a tree four wide. Not one
+// with triangles: a large mesh's walks live on the L1 cache that the paths would take (the 1.3M-triangle mesh 2.7 G
+// segments/s by the wavefront's steps, 1.75 here); nor a bare small scene under NEE/MIS, nor an empty one. The bare small
+// scenes too, which lost 40% in the steps: quads 397x401 x 100 2.02 ms in the persistent kernel, 0.96 here; materials
+// 800x450 x 64 6.77 and 2.82.
+inline bool pool_suits(const scene_view& v, bool quality)
 {
-    return wavefront_suits(v) && (v.flat != 0 || v.wide_nodes != nullptr) && v.prim_count == v.triangle_base;
+    const bool searched = v.node_count > 0 && (v.flat != 0 || v.wide_nodes != nullptr);
+    return searched && v.prim_count == v.triangle_base && (wavefront_suits(v) || !quality);
 }
+using pool_function = void (*)(launch_params, pool_run, wave_batch);
+pool_function bare_pool_kernel(); // a scene that does not suit the wavefront (pool_bare.cu)
 // Claims, renders and writes out every sample of the launch (`grid` blocks fill the GPU; a small launch takes fewer)
 cudaError_t launch_pool(const launch_params& p, bool quality, float4* samples, int64_t sample_count, int grid,
                         cudaStream_t stream);

@@ -1992,7 +1992,7 @@ template <bool FEATURES>
 __device__ __forceinline__ void flat_search(const scene_view& S, float3 o, float3 d, float time, int from, bool inward,
                                             int skip, bool any, hit_info& hit)
 {
-    const float inverse_a = 1.0f / length_squared(d);
+    const float inverse_a = 1.0f / length_squared<rounds::walk_flat>(d);
     for (int i = 0; i < S.quad_base; ++i)
     {
         const bool own = i == from;

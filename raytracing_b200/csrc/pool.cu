@@ -21,21 +21,24 @@ using rounds = rounds_session;
 // Before a launch of the pool kernel: no sample claimed
 __global__ void pool_prepare_kernel(unsigned long long* work_counter) { *work_counter = 0ull; }
 
-using pool_function = void (*)(launch_params, pool_run, wave_batch);
-
 template <bool QUALITY, bool FEATURES>
 pool_function pool_kernel_of(bool flat)
 {
     return flat ? pool_kernel<QUALITY, FEATURES, true, false> : pool_kernel<QUALITY, FEATURES, false, false>;
 }
 
-pool_function pool_kernel_for(bool quality, bool features, bool flat)
+pool_function pool_kernel_for(const scene_view& scene, bool quality)
 {
+    const bool flat = scene.flat != 0;
+    if (!wavefront_suits(scene))
+    {
+        return bare_pool_kernel();
+    }
     if (quality)
     {
-        return features ? pool_kernel_of<true, true>(flat) : pool_kernel_of<true, false>(flat);
+        return has_features(scene) ? pool_kernel_of<true, true>(flat) : pool_kernel_of<true, false>(flat);
     }
-    return features ? pool_kernel_of<false, true>(flat) : pool_kernel_of<false, false>(flat);
+    return has_features(scene) ? pool_kernel_of<false, true>(flat) : pool_kernel_of<false, false>(flat);
 }
 } // namespace
 
@@ -49,15 +52,13 @@ cudaError_t launch_pool(const launch_params& p, bool quality, float4* samples, i
     const int64_t blocks = std::min<int64_t>(grid, (sample_count + claim * block_warps - 1) / (claim * block_warps));
     const pool_run run{samples, sample_count, claim, 0};
     pool_prepare_kernel<<<1, 1, 0, stream>>>(p.work_counter);
-    pool_kernel_for(quality, has_features(p.scene), p.scene.flat != 0)<<<static_cast<unsigned>(std::max<int64_t>(blocks, 1)),
-                                                                         render_block, 0, stream>>>(p, run, wave_batch{});
+    pool_kernel_for(p.scene, quality)<<<static_cast<unsigned>(std::max<int64_t>(blocks, 1)), render_block, 0, stream>>>(
+        p, run, wave_batch{});
     return cudaGetLastError();
 }
 
 cudaError_t pool_attributes(const scene_view& scene, bool quality, kernel_attributes& out)
 {
-    return function_attributes(reinterpret_cast<const void*>(
-                                   pool_kernel_for(quality, has_features(scene), scene.flat != 0)),
-                               out);
+    return function_attributes(reinterpret_cast<const void*>(pool_kernel_for(scene, quality)), out);
 }
 } // namespace rtb

@@ -18,6 +18,7 @@ struct rounds_compiler
     static constexpr rounding other = rounding::compiler;
     static constexpr rounding sky = rounding::compiler;
     static constexpr rounding flight = rounding::compiler;
+    static constexpr rounding walk_flat = rounding::compiler;
     static constexpr rounding walk_features = rounding::compiler;
     static constexpr rounding dielectric_unit = rounding::compiler;
     static constexpr rounding dielectric_cosine = rounding::compiler;
@@ -41,6 +42,7 @@ struct rounds_session
     static constexpr rounding other = rounding::x;
     static constexpr rounding sky = rounding::y;
     static constexpr rounding flight = rounding::y;
+    static constexpr rounding walk_flat = rounding::x;
     static constexpr rounding walk_features = rounding::y;
     static constexpr rounding dielectric_unit = rounding::y;
     static constexpr rounding dielectric_cosine = rounding::yz;
@@ -54,5 +56,11 @@ struct rounds_session
     static constexpr rounding ggx_sample_view = rounding::y;
     static constexpr rounding ggx_sample_half = rounding::y;
     static constexpr rounding energy = rounding::y;
+};
+
+// The persistent kernel's flat search, which renders the bare small scenes: the same but for the ray's squared length
+struct rounds_bare : rounds_session
+{
+    static constexpr rounding walk_flat = rounding::y;
 };
 } // namespace rtb

