@@ -1346,7 +1346,7 @@ __device__ __forceinline__ step_result shade_books(const scene_view& S, const ca
         const float cos_theta = fminf(dot<rounds::dielectric_cosine>(-ud, s.normal), 1.0f);
         const float sin_theta = sqrtf(1.0f - cos_theta * cos_theta);
         const bool cannot_refract = ri * sin_theta > 1.0f;
-        direction = cannot_refract || reflectance(cos_theta, ri) > u.z ? reflect<rounds::dielectric_cosine>(ud, s.normal)
+        direction = cannot_refract || reflectance(cos_theta, ri) > u.z ? reflect<rounds::dielectric_reflect>(ud, s.normal)
                                                                        : refract(ud, s.normal, ri);
     }
     if (--ps.rays_left == 0)
@@ -1822,7 +1822,7 @@ __device__ __forceinline__ step_result shade_quality(const scene_view& S, const 
         const float3 ud = unit_vector<rounds::dielectric_unit>(ps.d);
         const float cos_theta = fminf(dot<rounds::dielectric_cosine>(-ud, s.normal), 1.0f);
         const float sin_theta = sqrtf(1.0f - cos_theta * cos_theta);
-        wi = ri * sin_theta > 1.0f || reflectance(cos_theta, ri) > u.z ? reflect<rounds::dielectric_cosine>(ud, s.normal)
+        wi = ri * sin_theta > 1.0f || reflectance(cos_theta, ri) > u.z ? reflect<rounds::dielectric_reflect>(ud, s.normal)
                                                                        : refract(ud, s.normal, ri);
         weight = make_float3(1.0f, 1.0f, 1.0f);
     }

@@ -55,8 +55,12 @@ constexpr uint32_t pool_shadow = 8u;        // a shadow ray is to be walked (bef
 constexpr uint32_t pool_shadow_inward = 16u;
 constexpr uint32_t pool_blocked = 32u;      // the shadow ray's answer, where the shading needs it (smoke)
 
+// The resident blocks per multiprocessor, which cap the registers: swept on the B200 from 4 to 10 (books tree 7 -> 8:
+// weekend 6.32 -> 6.18 ms; features 5 -> 6: final 11.25 -> 10.4; NEE/MIS flat 5 -> 6: cornell-mis 8.29 -> 7.95, where the
+// tree lost 8% and the features 11% of their time to spills). With the paths a warp keeps (48, 64, 80, 96: 64 within 1%
+// of the best on every scene, 96 -11% under NEE/MIS) they also set the shared memory, 17 to 31 KB a block.
 #ifndef RTB_POOL_BLOCKS_TREE
-#define RTB_POOL_BLOCKS_TREE 7
+#define RTB_POOL_BLOCKS_TREE 8
 #endif
 #ifndef RTB_POOL_BLOCKS_FLAT
 #define RTB_POOL_BLOCKS_FLAT 8
@@ -64,14 +68,20 @@ constexpr uint32_t pool_blocked = 32u;      // the shadow ray's answer, where th
 #ifndef RTB_POOL_BLOCKS_QUALITY
 #define RTB_POOL_BLOCKS_QUALITY 5
 #endif
+#ifndef RTB_POOL_BLOCKS_QUALITY_FLAT
+#define RTB_POOL_BLOCKS_QUALITY_FLAT 6
+#endif
 #ifndef RTB_POOL_BLOCKS_FEATURES
-#define RTB_POOL_BLOCKS_FEATURES 5
+#define RTB_POOL_BLOCKS_FEATURES 6
 #endif
 template <bool QUALITY, bool FEATURES, bool FLAT, bool BATCH>
 constexpr int pool_min_blocks()
 {
-    return FEATURES ? RTB_POOL_BLOCKS_FEATURES
-                    : (QUALITY || BATCH ? RTB_POOL_BLOCKS_QUALITY : (FLAT ? RTB_POOL_BLOCKS_FLAT : RTB_POOL_BLOCKS_TREE));
+    if (QUALITY || BATCH)
+    {
+        return FLAT && !FEATURES ? RTB_POOL_BLOCKS_QUALITY_FLAT : RTB_POOL_BLOCKS_QUALITY;
+    }
+    return FEATURES ? RTB_POOL_BLOCKS_FEATURES : (FLAT ? RTB_POOL_BLOCKS_FLAT : RTB_POOL_BLOCKS_TREE);
 }
 
 template <bool QUALITY, bool FEATURES, bool FLAT, bool BATCH>
@@ -331,6 +341,8 @@ __global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURE
                 const bvh4_node* const tree = S.wide_nodes;
                 float inverse_a = 0.0f;
                 float3 inv = o, os = o;
+                // where the near bounds of an axis lie in a node (lo_x, hi_x, lo_y, ...; the far ones 16 bytes off)
+                uint32_t near_x = 0, near_y = 32, near_z = 64;
                 if (slot >= 0)
                 {
                     const uint32_t meta = rec[record::meta][slot];
@@ -343,6 +355,9 @@ __global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURE
                     inverse_a = 1.0f / (FEATURES ? length_squared<rounds::walk_features>(d) : length_squared(d));
                     inv = make_float3(safe_inverse(d.x), safe_inverse(d.y), safe_inverse(d.z));
                     os = make_float3(o.x * inv.x, o.y * inv.y, o.z * inv.z);
+                    near_x = inv.x < 0.0f ? 16u : 0u;
+                    near_y = inv.y < 0.0f ? 48u : 32u;
+                    near_z = inv.z < 0.0f ? 80u : 64u;
                 }
                 const bool has_query = slot >= 0;
                 const auto pop = [&]() -> int {
@@ -370,20 +385,23 @@ __global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURE
                         }
                         if (descending)
                         {
-                            const float4* np = reinterpret_cast<const float4*>(tree + link);
-                            const float4 lx = __ldg(np), hx = __ldg(np + 1);
-                            const float4 ly = __ldg(np + 2), hy = __ldg(np + 3);
-                            const float4 lz = __ldg(np + 4), hz = __ldg(np + 5);
-                            const int4 nl = __ldg(reinterpret_cast<const int4*>(np + 6));
+                            // The near and far bound of each axis by the sign of the ray's direction there, instead
+                            // of a minimum and a maximum of both: the same numbers (a multiply-add is monotonic)
+                            const char* const node = reinterpret_cast<const char*>(tree + link);
+                            const auto row = [&](uint32_t at) {
+                                return __ldg(reinterpret_cast<const float4*>(node + at));
+                            };
+                            const float4 lx = row(near_x), hx = row(near_x ^ 16u);
+                            const float4 ly = row(near_y), hy = row(near_y ^ 16u);
+                            const float4 lz = row(near_z), hz = row(near_z ^ 16u);
+                            const int4 nl = __ldg(reinterpret_cast<const int4*>(tree[link].link));
                             const auto entry = [&](float lox, float hix, float loy, float hiy, float loz, float hiz,
                                                    int child) -> float {
                                 const float a0 = fmaf(lox, inv.x, -os.x), a1 = fmaf(hix, inv.x, -os.x);
                                 const float b0 = fmaf(loy, inv.y, -os.y), b1 = fmaf(hiy, inv.y, -os.y);
                                 const float c0 = fmaf(loz, inv.z, -os.z), c1 = fmaf(hiz, inv.z, -os.z);
-                                const float enter =
-                                    fmaxf(fmaxf(fminf(a0, a1), fminf(b0, b1)), fmaxf(fminf(c0, c1), t_min));
-                                const float exit =
-                                    fminf(fminf(fmaxf(a0, a1), fmaxf(b0, b1)), fminf(fmaxf(c0, c1), hit.t));
+                                const float enter = fmaxf(fmaxf(a0, b0), fmaxf(c0, t_min));
+                                const float exit = fminf(fminf(a1, b1), fminf(c1, hit.t));
                                 return enter <= exit && child != traversal_done ? enter : infinity_f;
                             };
                             float k0 = entry(lx.x, hx.x, ly.x, hy.x, lz.x, hz.x, nl.x);

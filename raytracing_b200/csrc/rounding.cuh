@@ -22,6 +22,7 @@ struct rounds_compiler
     static constexpr rounding walk_features = rounding::compiler;
     static constexpr rounding dielectric_unit = rounding::compiler;
     static constexpr rounding dielectric_cosine = rounding::compiler;
+    static constexpr rounding dielectric_reflect = rounding::compiler;
     static constexpr rounding view = rounding::compiler;
     static constexpr rounding lamp_distance = rounding::compiler;
     static constexpr rounding lamp_hit = rounding::compiler;
@@ -46,6 +47,7 @@ struct rounds_session
     static constexpr rounding walk_features = rounding::y;
     static constexpr rounding dielectric_unit = rounding::y;
     static constexpr rounding dielectric_cosine = rounding::yz;
+    static constexpr rounding dielectric_reflect = rounding::yz;
     static constexpr rounding view = rounding::y;
     static constexpr rounding lamp_distance = rounding::y;
     static constexpr rounding lamp_hit = rounding::y;
