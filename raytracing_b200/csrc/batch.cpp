@@ -44,6 +44,11 @@ batch_engine::batch_engine(size_t partial_budget_bytes, bool use_graph, bool hig
     kernel_attributes shade{}, trace{};
     check(wave_attributes(scene_view{}, false, shade, trace), "querying the wavefront kernels");
     trace_grid_ = trace.multiprocessors * std::max(1, trace.blocks_per_sm);
+    for (int k = 0; k < 2; ++k)
+    {
+        check(pool_batch_attributes(k != 0, a), "querying the pool kernel");
+        pool_grids_[k] = a.multiprocessors * std::max(1, a.blocks_per_sm);
+    }
     wave_ = std::make_unique<wave_runner>(wave_slots_mesh, wave_group); // the wavefront groups' slots, in turn
     work_counter_.allocate(batch_groups);
     header_.allocate(1);
@@ -234,13 +239,18 @@ double batch_engine::step(std::vector<assignment> work)
         return 0;
     }
     ensure_capacity(work.size(), static_cast<size_t>(entries) * 3);
+    // The books' jobs on trees four wide go to the pool kernel, in any step: its launches end without a drain.
     // A short step (a server's) keeps its wavefront runs to one: every run ends with a drain (its last paths finishing
     // while most slots idle, a path's length of steps), so the tree-searched jobs share one group (the kernels with
     // the second book's features render the scenes without them) and the flat-searched ones take the persistent
     // kernel, whose tail overlaps nothing either but is shorter. Measured on the 10 ms steps of the served stream: 2%
     // above the flat scenes in a wavefront group of their own, whose second drain costs more than its walks save.
+    const auto pooled = [](const job& j) {
+        return !j.scene->quality() && j.scene->view().flat == 0 && pool_suits(j.scene->view(), false);
+    };
     int64_t wave_samples = 0;
     bool tree_features = false;
+    bool pool_features = false;
     for (const assignment& a : work)
     {
         const job& j = *jobs_.at(a.handle);
@@ -248,13 +258,17 @@ double batch_engine::step(std::vector<assignment> work)
         if (wavefront_suits(v))
         {
             wave_samples += (a.pass_end - j.passes) * int64_t{j.padded};
-            tree_features = tree_features || (v.flat == 0 && has_features(v));
+            (pooled(j) ? pool_features : tree_features) |= v.flat == 0 && has_features(v);
         }
     }
     const bool short_step = wave_samples <= short_step_samples;
     // The jobs in their groups' order (each group's items form its own launch)
     const auto group_of = [&](const assignment& a) {
         const scene_view& v = jobs_.at(a.handle)->scene->view();
+        if (pooled(*jobs_.at(a.handle)))
+        {
+            return pool_batch_group(short_step ? pool_features : has_features(v));
+        }
         if (!wavefront_suits(v) || (short_step && v.flat != 0))
         {
             return batch_group(v.flat != 0, has_features(v));
@@ -327,7 +341,12 @@ double batch_engine::step(std::vector<assignment> work)
             group_depth[g] = std::max(group_depth[g], b.cam.max_depth);
         }
     }
-    wave_->setup(*std::max_element(group_samples, group_samples + batch_groups), stream_);
+    const int64_t wave_most = *std::max_element(group_samples, group_samples + pool_batch_group(false));
+    if (wave_most > 0)
+    {
+        wave_->setup(wave_most, stream_);
+    }
+    float4* const samples = wave_->samples(*std::max_element(group_samples, group_samples + batch_groups), stream_);
     check(cudaEventRecord(start_, stream_), "recording a CUDA event");
     if (use_graph_)
     {
@@ -360,6 +379,17 @@ double batch_engine::step(std::vector<assignment> work)
         // the group's samples claimed through its own work counter, zeroed with the others at the step's start
         const wave_batch w{table_.data(),          header.group_jobs[g],      header.group_jobs[g + 1],
                            header.group_items[g], header.group_items[g + 1], work_counter_.data() + g};
+        if (g >= pool_batch_group(false))
+        {
+            const bool features = g == pool_batch_group(true);
+            check(launch_pool_batch(w, features, samples, group_samples[g], pool_grids_[features ? 1 : 0], stream_),
+                  "launching the pool kernel");
+            wave_buffers b{};
+            b.samples = samples;
+            check(launch_wave_batch_partials(w, b, stream_), "launching the wavefront's partials");
+            launches_ += 3;
+            continue;
+        }
         const bool flat = g == wave_batch_group(true, false) || g == wave_batch_group(true, true);
         const bool features = g == wave_batch_group(flat, true);
         bool wide = true;

@@ -87,6 +87,7 @@ private:
     int grids_[persistent_groups] = {}; // each persistent group's launch (batch_group)
     std::unique_ptr<wave_runner> wave_;  // the wavefront's groups (wave_batch_group), one after another
     int trace_grid_ = 0;
+    int pool_grids_[2] = {}; // the pool kernel's launches without and with the second book's features
     device_array<double> arena_;
     device_array<batch_job> table_;
     device_array<batch_header> header_;

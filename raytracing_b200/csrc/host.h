@@ -258,6 +258,8 @@ public:
     // Buffers from the device's memory pool, stream-ordered on `stream` (which must outlive the runner): a one-shot
     // render that needs them takes them from what earlier renders left in the pool
     wave_buffers setup(int64_t samples, cudaStream_t stream);
+    // The samples' values alone, for a launch of the pool kernel
+    float4* samples(int64_t count, cudaStream_t stream);
     // step() enqueues one step on `stream`; returns the steps run
     // The steps of one launch until a step queues nothing. step(draining) launches one; draining is true once the
     // host has seen every sample of the launch claimed (work_counter, when given, at sample_count or beyond): the

@@ -18,7 +18,6 @@ using rounds = rounds_session;
 #include "path.cuh"
 #include "pool_kernel.cuh"
 
-// Before a launch of the pool kernel: no sample claimed
 __global__ void pool_prepare_kernel(unsigned long long* work_counter) { *work_counter = 0ull; }
 
 template <bool QUALITY, bool FEATURES>
@@ -42,18 +41,32 @@ pool_function pool_kernel_for(const scene_view& scene, bool quality)
 }
 } // namespace
 
+cudaError_t prepare_pool(unsigned long long* work_counter, cudaStream_t stream)
+{
+    pool_prepare_kernel<<<1, 1, 0, stream>>>(work_counter);
+    return cudaGetLastError();
+}
+
+// A launch of fewer samples than lanes spreads them over the warps, so that every multiprocessor takes part
+pool_launch pool_launch_of(int64_t sample_count, int grid)
+{
+    constexpr int64_t block_warps = render_block / 32;
+    const int64_t warps = grid * block_warps;
+    const int64_t claim = std::clamp<int64_t>((sample_count + warps - 1) / warps, 1, 32);
+    const int64_t blocks = std::min<int64_t>(grid, (sample_count + claim * block_warps - 1) / (claim * block_warps));
+    return {static_cast<int32_t>(claim), static_cast<unsigned>(std::max<int64_t>(blocks, 1))};
+}
+
 cudaError_t launch_pool(const launch_params& p, bool quality, float4* samples, int64_t sample_count, int grid,
                         cudaStream_t stream)
 {
-    // A launch of fewer samples than lanes spreads them over the warps, so that every multiprocessor takes part
-    constexpr int64_t block_warps = render_block / 32;
-    const int64_t warps = grid * block_warps;
-    const auto claim = static_cast<int32_t>(std::clamp<int64_t>((sample_count + warps - 1) / warps, 1, 32));
-    const int64_t blocks = std::min<int64_t>(grid, (sample_count + claim * block_warps - 1) / (claim * block_warps));
-    const pool_run run{samples, sample_count, claim, 0};
-    pool_prepare_kernel<<<1, 1, 0, stream>>>(p.work_counter);
-    pool_kernel_for(p.scene, quality)<<<static_cast<unsigned>(std::max<int64_t>(blocks, 1)), render_block, 0, stream>>>(
-        p, run, wave_batch{});
+    const pool_launch l = pool_launch_of(sample_count, grid);
+    const pool_run run{samples, sample_count, l.claim, 0};
+    if (const cudaError_t e = prepare_pool(p.work_counter, stream); e != cudaSuccess)
+    {
+        return e;
+    }
+    pool_kernel_for(p.scene, quality)<<<l.blocks, render_block, 0, stream>>>(p, run, wave_batch{});
     return cudaGetLastError();
 }
 

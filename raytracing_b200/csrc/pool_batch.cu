@@ -1,0 +1,45 @@
+// A batch's groups of books' jobs on tree-searched scenes by the pool kernel, each sample with its job's scene and
+// camera; the roundings are a session's, so a job's image is its session's.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+
+#include "ggx_energy_table.h"
+#include "kernels.cuh"
+#include "philox.cuh"
+#include "rounding.cuh"
+#include "rt_b200.h"
+
+namespace rtb
+{
+namespace
+{
+using rounds = rounds_session;
+#include "path.cuh"
+#include "pool_kernel.cuh"
+
+pool_function batch_kernel_of(bool features)
+{
+    return features ? pool_kernel<false, true, false, true> : pool_kernel<false, false, false, true>;
+}
+} // namespace
+
+cudaError_t launch_pool_batch(const wave_batch& w, bool features, float4* samples, int64_t sample_count, int grid,
+                              cudaStream_t stream)
+{
+    const pool_launch l = pool_launch_of(sample_count, grid);
+    const pool_run run{samples, sample_count, l.claim, 0};
+    if (const cudaError_t e = prepare_pool(w.work_counter, stream); e != cudaSuccess)
+    {
+        return e;
+    }
+    batch_kernel_of(features)<<<l.blocks, render_block, 0, stream>>>(launch_params{}, run, w);
+    return cudaGetLastError();
+}
+
+cudaError_t pool_batch_attributes(bool features, kernel_attributes& out)
+{
+    return function_attributes(reinterpret_cast<const void*>(batch_kernel_of(features)), out);
+}
+} // namespace rtb

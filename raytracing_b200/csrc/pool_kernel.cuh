@@ -57,7 +57,8 @@ constexpr uint32_t pool_blocked = 32u;      // the shadow ray's answer, where th
 
 // The resident blocks per multiprocessor, which cap the registers: swept on the B200 from 4 to 10 (books tree 7 -> 8:
 // weekend 6.32 -> 6.18 ms; features 5 -> 6: final 11.25 -> 10.4; NEE/MIS flat 5 -> 6: cornell-mis 8.29 -> 7.95, where the
-// tree lost 8% and the features 11% of their time to spills). With the paths a warp keeps (48, 64, 80, 96: 64 within 1%
+// tree lost 8% and the features 11% of their time to spills; a batch of 16 cover jobs 20.7, 19.8, 19.0 and 19.7 ms at 5, 6,
+// 7 and 8). With the paths a warp keeps (48, 64, 80, 96: 64 within 1%
 // of the best on every scene, 96 -11% under NEE/MIS) they also set the shared memory, 17 to 31 KB a block.
 #ifndef RTB_POOL_BLOCKS_TREE
 #define RTB_POOL_BLOCKS_TREE 8
@@ -71,15 +72,25 @@ constexpr uint32_t pool_blocked = 32u;      // the shadow ray's answer, where th
 #ifndef RTB_POOL_BLOCKS_QUALITY_FLAT
 #define RTB_POOL_BLOCKS_QUALITY_FLAT 6
 #endif
+#ifndef RTB_POOL_BLOCKS_BATCH
+#define RTB_POOL_BLOCKS_BATCH 7
+#endif
+#ifndef RTB_POOL_BLOCKS_BATCH_FEATURES
+#define RTB_POOL_BLOCKS_BATCH_FEATURES 5
+#endif
 #ifndef RTB_POOL_BLOCKS_FEATURES
 #define RTB_POOL_BLOCKS_FEATURES 6
 #endif
 template <bool QUALITY, bool FEATURES, bool FLAT, bool BATCH>
 constexpr int pool_min_blocks()
 {
-    if (QUALITY || BATCH)
+    if (QUALITY)
     {
         return FLAT && !FEATURES ? RTB_POOL_BLOCKS_QUALITY_FLAT : RTB_POOL_BLOCKS_QUALITY;
+    }
+    if (BATCH)
+    {
+        return FEATURES ? RTB_POOL_BLOCKS_BATCH_FEATURES : RTB_POOL_BLOCKS_BATCH;
     }
     return FEATURES ? RTB_POOL_BLOCKS_FEATURES : (FLAT ? RTB_POOL_BLOCKS_FLAT : RTB_POOL_BLOCKS_TREE);
 }

@@ -121,14 +121,10 @@ wave_buffers wave_runner::setup(int64_t samples, cudaStream_t stream)
         ext_result_.allocate_async(c, stream);
         shadow_result_.allocate_async(c, stream);
     }
-    if (samples_.size() < static_cast<size_t>(samples))
-    {
-        samples_.allocate_async(std::max(static_cast<size_t>(samples), 2 * samples_.size()), stream);
-    }
     wave_buffers b{};
     b.slots = slots_.data();
     b.slot_count = static_cast<int32_t>(n);
-    b.samples = samples_.data();
+    b.samples = this->samples(samples, stream);
     b.sample_count = samples;
     b.query_o = query_o_.data();
     b.query_d = query_d_.data();
@@ -137,6 +133,15 @@ wave_buffers wave_runner::setup(int64_t samples, cudaStream_t stream)
     b.shadow_result = shadow_result_.data();
     b.control = control_.data();
     return b;
+}
+
+float4* wave_runner::samples(int64_t count, cudaStream_t stream)
+{
+    if (samples_.size() < static_cast<size_t>(count))
+    {
+        samples_.allocate_async(std::max(static_cast<size_t>(count), 2 * samples_.size()), stream);
+    }
+    return samples_.data();
 }
 
 int64_t wave_runner::run(const wave_buffers& b, int max_depth, cudaStream_t stream,

@@ -61,3 +61,21 @@ def test_a_tuned_session_takes_the_steps(rt):
     t.set_tuning({**t.tuning(), "slots": 1 << 19})
     assert t.render_to(16)["kernel_launches"] > 3
     assert np.array_equal(t.pixels(), image)
+
+
+@pytest.mark.parametrize("passes", [1, 16, 33])
+@pytest.mark.parametrize("named", [[("weekend", {}), ("cover-60", {}), ("weekend", dict(combination="mis")),
+                                    ("glass", {}), ("cover-900", {})],
+                                   [("bouncing", {}), ("smoke", {}), ("final", {})]], ids=["plain", "features"])
+def test_batched_tree_jobs_equal_their_sessions(rt, named, passes):
+    # books' jobs on trees, of sizes whose tiles hang over the edges and whose samples start anywhere in a claim,
+    # between jobs of the other groups (NEE/MIS, flat-searched scenes)
+    jobs = [(rt.builtin_scene(n, width=21 + 8 * k, height=13 + 7 * k, spp=passes, **kw), 40 + k, passes)
+            for k, (n, kw) in enumerate(named)]
+    batch = rt.batch_render(jobs)
+    for (desc, seed, _), image, (name, kw) in zip(jobs, batch.images, named):
+        if name in ("glass", "smoke") or kw:
+            continue  # kernels of their own roundings
+        session = rt.Session(rt.Scene(desc), seed=seed, form="wavefront")
+        session.render_to(passes)
+        assert np.array_equal(image, session.pixels()), name
