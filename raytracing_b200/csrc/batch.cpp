@@ -44,10 +44,13 @@ batch_engine::batch_engine(size_t partial_budget_bytes, bool use_graph, bool hig
     kernel_attributes shade{}, trace{};
     check(wave_attributes(scene_view{}, false, shade, trace), "querying the wavefront kernels");
     trace_grid_ = trace.multiprocessors * std::max(1, trace.blocks_per_sm);
-    for (int k = 0; k < 2; ++k)
+    for (const bool flat : {false, true})
     {
-        check(pool_batch_attributes(k != 0, a), "querying the pool kernel");
-        pool_grids_[k] = a.multiprocessors * std::max(1, a.blocks_per_sm);
+        for (const bool features : {false, true})
+        {
+            check(pool_batch_attributes(flat, features, a), "querying the pool kernel");
+            pool_grids_[batch_group(flat, features)] = a.multiprocessors * std::max(1, a.blocks_per_sm);
+        }
     }
     wave_ = std::make_unique<wave_runner>(wave_slots_mesh, wave_group); // the wavefront groups' slots, in turn
     work_counter_.allocate(batch_groups);
@@ -192,7 +195,7 @@ void batch_engine::capture()
     check(cudaGraphInstantiate(&graph_exec_, graph_, 0), "instantiating the batch step's graph");
 }
 
-double batch_engine::step(std::vector<assignment> work)
+double batch_engine::step(std::vector<assignment> work, bool flat_pool)
 {
     // A path of no rays: every sample is 0, the job needs no launch (as a session's render_to)
     for (assignment& a : work)
@@ -245,8 +248,9 @@ double batch_engine::step(std::vector<assignment> work)
     // the second book's features render the scenes without them) and the flat-searched ones take the persistent
     // kernel, whose tail overlaps nothing either but is shorter. Measured on the 10 ms steps of the served stream: 2%
     // above the flat scenes in a wavefront group of their own, whose second drain costs more than its walks save.
-    const auto pooled = [](const job& j) {
-        return !j.scene->quality() && j.scene->view().flat == 0 && pool_suits(j.scene->view(), false);
+    const auto pooled = [&](const job& j) {
+        const scene_view& v = j.scene->view();
+        return !j.scene->quality() && (v.flat == 0 || flat_pool) && wavefront_suits(v) && pool_suits(v, false);
     };
     int64_t wave_samples = 0;
     bool tree_features = false;
@@ -267,7 +271,7 @@ double batch_engine::step(std::vector<assignment> work)
         const scene_view& v = jobs_.at(a.handle)->scene->view();
         if (pooled(*jobs_.at(a.handle)))
         {
-            return pool_batch_group(short_step ? pool_features : has_features(v));
+            return pool_batch_group(v.flat != 0, short_step && !flat_pool ? pool_features : has_features(v));
         }
         if (!wavefront_suits(v) || (short_step && v.flat != 0))
         {
@@ -341,7 +345,7 @@ double batch_engine::step(std::vector<assignment> work)
             group_depth[g] = std::max(group_depth[g], b.cam.max_depth);
         }
     }
-    const int64_t wave_most = *std::max_element(group_samples, group_samples + pool_batch_group(false));
+    const int64_t wave_most = *std::max_element(group_samples, group_samples + 2 * persistent_groups);
     if (wave_most > 0)
     {
         wave_->setup(wave_most, stream_);
@@ -379,10 +383,11 @@ double batch_engine::step(std::vector<assignment> work)
         // the group's samples claimed through its own work counter, zeroed with the others at the step's start
         const wave_batch w{table_.data(),          header.group_jobs[g],      header.group_jobs[g + 1],
                            header.group_items[g], header.group_items[g + 1], work_counter_.data() + g};
-        if (g >= pool_batch_group(false))
+        if (g >= 2 * persistent_groups)
         {
-            const bool features = g == pool_batch_group(true);
-            check(launch_pool_batch(w, features, samples, group_samples[g], pool_grids_[features ? 1 : 0], stream_),
+            const bool flat = g == pool_batch_group(true, false) || g == pool_batch_group(true, true);
+            check(launch_pool_batch(w, flat, g == pool_batch_group(flat, true), samples, group_samples[g],
+                                    pool_grids_[g - 2 * persistent_groups], stream_),
                   "launching the pool kernel");
             wave_buffers b{};
             b.samples = samples;
@@ -563,7 +568,13 @@ int64_t render_server::passes_of(const request& r) const
     {
         return r.state == RT_REQUEST_DONE ? r.target : 0;
     }
-    return stream_ ? stream_->passes(r.handle) : engine_->passes(r.handle);
+    return stream_ && !r.batched ? stream_->passes(r.handle) : engine_->passes(r.handle);
+}
+
+// An active request of the continuous server whose first frame is still to render
+bool render_server::waits_for_first(const request& r) const
+{
+    return r.batched ? r.state == RT_REQUEST_ACTIVE && engine_->passes(r.handle) == 0 : r.first_handle >= 0;
 }
 
 // A request's device memory back to the budget
@@ -576,7 +587,7 @@ void render_server::release(request& r)
     }
     if (r.handle >= 0)
     {
-        if (stream_)
+        if (stream_ && !r.batched)
         {
             stream_->remove(r.handle);
         }
@@ -588,6 +599,52 @@ void render_server::release(request& r)
         used_bytes_ -= r.bytes;
     }
     r.scene.reset();
+}
+
+// The continuous server's batched requests refined for about `seconds`, least remaining work first, each to the end of
+// a chunk or to its target (as the continuous run adds them), at most a values ring's worth of samples; the GPU seconds
+double render_server::refine_batched(double seconds)
+{
+    constexpr double most_samples = double(int64_t{1} << 26);
+    std::vector<std::pair<double, request*>> refine;
+    for (auto& [id, r] : requests_)
+    {
+        if (r.batched && r.state == RT_REQUEST_ACTIVE && engine_->passes(r.handle) < r.target)
+        {
+            refine.emplace_back(double(r.camera.image_width) * r.camera.image_height *
+                                    double(r.target - engine_->passes(r.handle)),
+                                &r);
+        }
+    }
+    std::stable_sort(refine.begin(), refine.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
+    std::vector<batch_engine::assignment> work;
+    std::vector<std::pair<const resident_scene*, double>> step_samples;
+    double planned = 0, samples = 0;
+    for (auto& [remaining, rp] : refine)
+    {
+        request& r = *rp;
+        if (!work.empty() && (planned >= seconds || samples >= most_samples))
+        {
+            break;
+        }
+        const int64_t done = engine_->passes(r.handle);
+        const double pixels = double(r.camera.image_width) * r.camera.image_height;
+        const double per_pass = pixels * cost_of(r.scene.get());
+        const double want = std::min((seconds - planned) / per_pass, (most_samples - samples) / pixels);
+        const int64_t boundary = (done / pass_chunk + 1) * pass_chunk;
+        const int64_t end = std::min(
+            r.target, std::max(boundary, (done + static_cast<int64_t>(std::max(want, 0.0))) / pass_chunk * pass_chunk));
+        work.push_back({r.handle, end});
+        step_samples.emplace_back(r.scene.get(), pixels * double(end - done));
+        planned += per_pass * double(end - done);
+        samples += pixels * double(end - done);
+    }
+    const double gpu = engine_->step(std::move(work), true);
+    if (gpu > 0)
+    {
+        learn_costs(step_samples, gpu);
+    }
+    return gpu;
 }
 
 // A step of the continuous wavefront: admission as in a batched step; the first frames of the admitted requests in
@@ -606,10 +663,15 @@ rt_server_step_report render_server::step_continuous()
         }
         // RNG job field 0, as in a batched step: the image equals a session's of the same view and seed
         const bool batched_first = options_.continuous == 1;
-        r.handle = stream_->add(r.scene, r.camera, r.seed, 0, r.target, batched_first);
+        const scene_view& v = r.scene->view();
+        // The books' requests that the pool kernel renders stay with the batch engine: it has no drain for the
+        // continuous run to save, and renders them three to five times as fast as the run's one kernel for every scene
+        r.batched = batched_first && !r.scene->quality() && wavefront_suits(v) && pool_suits(v, false);
+        r.handle = r.batched ? engine_->add(r.scene, r.camera, r.seed, 0)
+                             : stream_->add(r.scene, r.camera, r.seed, 0, r.target, batched_first);
         if (batched_first)
         {
-            r.first_handle = engine_->add(r.scene, r.camera, r.seed, 0);
+            r.first_handle = r.batched ? -1 : engine_->add(r.scene, r.camera, r.seed, 0);
             first_queue_.push_back(r.id);
         }
         r.state = RT_REQUEST_ACTIVE;
@@ -622,7 +684,7 @@ rt_server_step_report render_server::step_continuous()
     {
         if (r.state == RT_REQUEST_ACTIVE)
         {
-            before[id] = stream_->passes(r.handle);
+            before[id] = passes_of(r);
         }
     }
     // First frames: no group is launched meanwhile, and the groups in flight give way to the batch engine's stream
@@ -636,7 +698,7 @@ rt_server_step_report render_server::step_continuous()
     for (const int64_t id : first_queue_)
     {
         const auto it = requests_.find(id);
-        if (it != requests_.end() && it->second.first_handle >= 0)
+        if (it != requests_.end() && waits_for_first(it->second))
         {
             const request& r = it->second;
             waiting.emplace_back(double(r.camera.image_width) * r.camera.image_height * cost_of(r.scene.get()), id);
@@ -650,7 +712,7 @@ rt_server_step_report render_server::step_continuous()
         {
             break;
         }
-        work.push_back({r.first_handle, 1});
+        work.push_back({r.batched ? r.handle : r.first_handle, 1});
         step_samples.emplace_back(r.scene.get(), double(r.camera.image_width) * r.camera.image_height);
         planned += cost;
         firsts.push_back(id);
@@ -660,7 +722,7 @@ rt_server_step_report render_server::step_continuous()
     for (const int64_t id : first_queue_)
     {
         const auto it = requests_.find(id);
-        if (it != requests_.end() && it->second.first_handle >= 0 &&
+        if (it != requests_.end() && waits_for_first(it->second) &&
             std::find(firsts.begin(), firsts.end(), id) == firsts.end())
         {
             left.push_back(id);
@@ -678,6 +740,10 @@ rt_server_step_report render_server::step_continuous()
         for (const int64_t id : firsts)
         {
             request& r = requests_.at(id);
+            if (r.batched)
+            {
+                continue;
+            }
             engine_->copy_sums(r.first_handle, stream_->sums(r.handle));
             first_rays_ += engine_->rays(r.first_handle);
             first_shadow_rays_ += engine_->shadow_rays(r.first_handle);
@@ -690,7 +756,24 @@ rt_server_step_report render_server::step_continuous()
     // frame waits for no refinement; the pool's paths wait in their slots meanwhile, without draining)
     if (first_queue_.empty())
     {
-        report.gpu_seconds += stream_->advance(options_.step_seconds);
+        // the batched requests and the pool's halve the step when both have work
+        bool batched = false, streamed = false;
+        for (const auto& [id, r] : requests_)
+        {
+            if (r.state == RT_REQUEST_ACTIVE && passes_of(r) < r.target)
+            {
+                (r.batched ? batched : streamed) = true;
+            }
+        }
+        const double seconds = batched && streamed ? 0.5 * options_.step_seconds : options_.step_seconds;
+        if (batched)
+        {
+            report.gpu_seconds += refine_batched(seconds);
+        }
+        if (streamed)
+        {
+            report.gpu_seconds += stream_->advance(seconds);
+        }
     }
     stats_.gpu_seconds += report.gpu_seconds;
     ++stats_.steps;
@@ -701,7 +784,7 @@ rt_server_step_report render_server::step_continuous()
         {
             continue;
         }
-        const int64_t done = stream_->passes(r.handle);
+        const int64_t done = passes_of(r);
         const int64_t was = before[id];
         report.first_frames += was == 0 && done >= 1 ? 1 : 0;
         report.refined += was >= 1 && done > was ? 1 : 0;
@@ -713,8 +796,8 @@ rt_server_step_report render_server::step_continuous()
         {
             r.state = RT_REQUEST_DONE;
             r.done_seconds = std::chrono::duration<double>(now - r.submitted).count();
-            stats_.rays += stream_->rays(r.handle);
-            stats_.shadow_rays += stream_->shadow_rays(r.handle);
+            stats_.rays += r.batched ? engine_->rays(r.handle) : stream_->rays(r.handle);
+            stats_.shadow_rays += r.batched ? engine_->shadow_rays(r.handle) : stream_->shadow_rays(r.handle);
             ++stats_.completed;
             ++report.completed;
         }
@@ -950,7 +1033,7 @@ void render_server::fetch(int64_t id, double* pixels, int64_t count)
         fail(RT_ERR_LOGIC, "request " + std::to_string(id) + " has no image");
     }
     request& r = it->second;
-    if (stream_)
+    if (stream_ && !r.batched)
     {
         stream_->pixels(r.handle, pixels, count);
     }
@@ -971,7 +1054,7 @@ void render_server::display(int64_t id, const rt_display_options& options, uint8
     {
         fail(RT_ERR_LOGIC, "request " + std::to_string(id) + " has no image");
     }
-    if (stream_)
+    if (stream_ && !it->second.batched)
     {
         stream_->display(it->second.handle, options, rgba, count);
     }

@@ -38,7 +38,9 @@ public:
     };
     // One step; returns its GPU seconds. Jobs whose partials do not fit the arena this step are cut back to fewer
     // chunks (at least one each), so every assignment makes progress.
-    double step(std::vector<assignment> work);
+    // flat_pool: books' jobs on flat-searched scenes take the pool kernel (a continuous server's refinement, whose
+    // roundings are a session's), not the persistent kernel or the wavefront's steps.
+    double step(std::vector<assignment> work, bool flat_pool = false);
 
     // The wavefront's buffers for steps of up to `samples` samples and its kernels loaded now, not on first use
     void reserve_wavefront(int64_t samples);
@@ -87,7 +89,7 @@ private:
     int grids_[persistent_groups] = {}; // each persistent group's launch (batch_group)
     std::unique_ptr<wave_runner> wave_;  // the wavefront's groups (wave_batch_group), one after another
     int trace_grid_ = 0;
-    int pool_grids_[2] = {}; // the pool kernel's launches without and with the second book's features
+    int pool_grids_[persistent_groups] = {}; // the pool kernel's launches (batch_group)
     device_array<double> arena_;
     device_array<batch_job> table_;
     device_array<batch_header> header_;
@@ -251,7 +253,8 @@ private:
 // The server of a stream of render requests: requests are admitted under an HBM budget, every
 // step gives the newly admitted their first frame (one pass) before it refines the others, and a request is done when
 // it reaches its target passes. Driven by the caller: submit between steps, step, poll, fetch. Its steps are batches
-// of passes (batch_engine) or runs of the continuous wavefront (stream_engine).
+// of passes (batch_engine) or runs of the continuous wavefront (stream_engine); the continuous server's books'
+// requests, which the pool kernel renders, are refined in batched steps beside it.
 class render_server
 {
 public:
@@ -276,6 +279,7 @@ private:
         int64_t target;
         int handle = -1;
         int first_handle = -1; // the continuous server: its first frame's job in the batch engine, until handed over
+        bool batched = false; // the continuous server: refined in batched steps too (handle is the batch engine's)
         int32_t state = RT_REQUEST_QUEUED;
         clock::time_point submitted;
         double first_frame_seconds = -1;
@@ -299,6 +303,8 @@ private:
     rt_server_stats stats_{};
 
     int64_t passes_of(const request& r) const;
+    bool waits_for_first(const request& r) const;
+    double refine_batched(double seconds);
     rt_server_step_report step_continuous();
     void release(request& r);
     double cost_of(const resident_scene* scene) const;

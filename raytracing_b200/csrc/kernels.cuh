@@ -94,15 +94,18 @@ inline bool wavefront_suits(const scene_view& v)
     return v.node_count > 0 && (v.flat == 0 || heavy);
 }
 
-// The jobs come in ten groups: the scenes of each search (flat, tree) without and with the second book's features,
-// in each form, and the books' jobs on trees four wide, which the pool kernel renders (pool_batch_group). The first four are rendered each by its own launch of the persistent kernel compiled for it
+// The jobs come in twelve groups: the scenes of each search (flat, tree) without and with the second book's features,
+// in each form: the persistent kernel, the wavefront's steps, and the pool kernel (pool_batch_group: books' jobs). The first four are rendered each by its own launch of the persistent kernel compiled for it
 // (batch_group), the other four each by its own run of the wavefront's steps (wave_batch_group); a scene takes the
 // form wavefront_suits gives it, as a session's render of it does.
 constexpr int persistent_groups = 4;
-constexpr int batch_groups = 10;
+constexpr int batch_groups = 12;
 RTB_HD constexpr int batch_group(bool flat, bool features) { return (flat ? 0 : 2) + (features ? 1 : 0); }
 RTB_HD constexpr int wave_batch_group(bool flat, bool features) { return persistent_groups + batch_group(flat, features); }
-RTB_HD constexpr int pool_batch_group(bool features) { return 2 * persistent_groups + (features ? 1 : 0); }
+RTB_HD constexpr int pool_batch_group(bool flat, bool features)
+{
+    return 2 * persistent_groups + batch_group(flat, features);
+}
 
 struct batch_header
 {
@@ -277,10 +280,11 @@ pool_function bare_pool_kernel(); // a scene that does not suit the wavefront (p
 cudaError_t launch_pool(const launch_params& p, bool quality, float4* samples, int64_t sample_count, int grid,
                         cudaStream_t stream);
 cudaError_t pool_attributes(const scene_view& scene, bool quality, kernel_attributes& out);
-// The same for a batch's group of books' jobs on trees four wide (w's jobs, their samples numbered from 0)
-cudaError_t launch_pool_batch(const wave_batch& w, bool features, float4* samples, int64_t sample_count, int grid,
+// The same for a batch's group of books' jobs, searched flat or through trees four wide (w's jobs, their samples
+// numbered from 0)
+cudaError_t launch_pool_batch(const wave_batch& w, bool flat, bool features, float4* samples, int64_t sample_count, int grid,
                               cudaStream_t stream);
-cudaError_t pool_batch_attributes(bool features, kernel_attributes& out);
+cudaError_t pool_batch_attributes(bool flat, bool features, kernel_attributes& out);
 // The work counter cleared before a launch, and the launch's shape for its samples
 struct pool_launch
 {

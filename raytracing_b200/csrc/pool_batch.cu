@@ -1,4 +1,4 @@
-// A batch's groups of books' jobs on tree-searched scenes by the pool kernel, each sample with its job's scene and
+// A batch's groups of books' jobs by the pool kernel, each sample with its job's scene and
 // camera; the roundings are a session's, so a job's image is its session's.
 #include <cuda_runtime.h>
 
@@ -19,13 +19,17 @@ using rounds = rounds_session;
 #include "path.cuh"
 #include "pool_kernel.cuh"
 
-pool_function batch_kernel_of(bool features)
+pool_function batch_kernel_of(bool flat, bool features)
 {
+    if (flat)
+    {
+        return features ? pool_kernel<false, true, true, true> : pool_kernel<false, false, true, true>;
+    }
     return features ? pool_kernel<false, true, false, true> : pool_kernel<false, false, false, true>;
 }
 } // namespace
 
-cudaError_t launch_pool_batch(const wave_batch& w, bool features, float4* samples, int64_t sample_count, int grid,
+cudaError_t launch_pool_batch(const wave_batch& w, bool flat, bool features, float4* samples, int64_t sample_count, int grid,
                               cudaStream_t stream)
 {
     const pool_launch l = pool_launch_of(sample_count, grid);
@@ -34,12 +38,12 @@ cudaError_t launch_pool_batch(const wave_batch& w, bool features, float4* sample
     {
         return e;
     }
-    batch_kernel_of(features)<<<l.blocks, render_block, 0, stream>>>(launch_params{}, run, w);
+    batch_kernel_of(flat, features)<<<l.blocks, render_block, 0, stream>>>(launch_params{}, run, w);
     return cudaGetLastError();
 }
 
-cudaError_t pool_batch_attributes(bool features, kernel_attributes& out)
+cudaError_t pool_batch_attributes(bool flat, bool features, kernel_attributes& out)
 {
-    return function_attributes(reinterpret_cast<const void*>(batch_kernel_of(features)), out);
+    return function_attributes(reinterpret_cast<const void*>(batch_kernel_of(flat, features)), out);
 }
 } // namespace rtb

@@ -79,3 +79,25 @@ def test_batched_tree_jobs_equal_their_sessions(rt, named, passes):
         session = rt.Session(rt.Scene(desc), seed=seed, form="wavefront")
         session.render_to(passes)
         assert np.array_equal(image, session.pixels()), name
+
+
+@pytest.mark.parametrize("scenes", [[("weekend", {}), ("cover-60", {}), ("cover-700", {})],
+                                    [("final", {}), ("bouncing", {})]], ids=["plain", "features"])
+def test_continuous_servers_books_requests_equal_their_sessions(rt, scenes):
+    # refined in batched steps, each to the end of a chunk, after a first pass of its own
+    server = rt.Server(hbm_budget_bytes=1 << 30, step_seconds=0.001, continuous=1)
+    held = []
+    for k, (name, kw) in enumerate(scenes):
+        desc = rt.builtin_scene(name, width=33 + 10 * k, height=29, spp=35, **kw)
+        scene = rt.Scene(desc)
+        held.append((desc, scene, server.submit(scene, desc.camera, 60 + k, 35)))
+    while any(server.poll(i)["state"] != "done" for _, _, i in held):
+        assert all(server.poll(i)["passes"] in (0, 1, 35) or server.poll(i)["passes"] % 16 == 0 for _, _, i in held)
+        server.step()
+    for k, (desc, scene, i) in enumerate(held):
+        session = rt.Session(scene, seed=60 + k, form="wavefront")
+        session.render_to(1)
+        session.render_to(35)
+        assert np.array_equal(server.fetch(i), session.pixels()), scenes[k]
+    assert server.stats()["used_bytes"] == 0
+    server.close()
