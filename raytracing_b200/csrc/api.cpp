@@ -486,18 +486,7 @@ rt_status rt_scene_closest_hits(rt_scene* scene, const float* origins, const flo
         need(directions, "directions");
         need(ids, "ids");
         need(ts, "ts");
-        const size_t n = static_cast<size_t>(count);
-        rtb::device_array<float> o(3 * n);
-        rtb::device_array<float> d(3 * n);
-        rtb::device_array<int32_t> id(n);
-        rtb::device_array<float> t(n);
-        rtb::check(cudaMemcpy(o.data(), origins, o.bytes(), cudaMemcpyHostToDevice), "copying rays");
-        rtb::check(cudaMemcpy(d.data(), directions, d.bytes(), cudaMemcpyHostToDevice), "copying rays");
-        rtb::check(rtb::launch_closest_hits(scene->scene->view(), o.data(), d.data(), count, scene->scene->prim_source(),
-                                            id.data(), t.data(), nullptr),
-                   "launching the closest-hit queries");
-        rtb::check(cudaMemcpy(ids, id.data(), id.bytes(), cudaMemcpyDeviceToHost), "copying hits");
-        rtb::check(cudaMemcpy(ts, t.data(), t.bytes(), cudaMemcpyDeviceToHost), "copying hits");
+        rtb::trace_rays(scene->scene->view(), scene->scene->prim_source(), origins, directions, count, ids, ts);
     });
 }
 

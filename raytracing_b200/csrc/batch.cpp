@@ -465,14 +465,7 @@ void batch_engine::pixels(int handle, double* out, int64_t count)
     {
         fail(RT_ERR_LOGIC, "pixels: the image has no complete pass");
     }
-    check(cudaMemcpyAsync(out, j.sums.data(), static_cast<size_t>(n) * sizeof(double), cudaMemcpyDeviceToHost, stream_),
-          "copying the image");
-    check(cudaStreamSynchronize(stream_), "copying the image");
-    const double scale = 1.0 / static_cast<double>(j.passes);
-    for (int64_t i = 0; i < n; ++i)
-    {
-        out[i] *= scale;
-    }
+    fetch_image(j.sums.data(), n, 1.0 / static_cast<double>(j.passes), out, stream_);
 }
 
 void batch_engine::display(int handle, const rt_display_options& options, uint8_t* out, int64_t count)

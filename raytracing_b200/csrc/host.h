@@ -47,7 +47,7 @@ public:
     device_array(const device_array&) = delete;
     device_array& operator=(const device_array&) = delete;
     device_array(device_array&& o) noexcept
-        : data_(o.data_), count_(o.count_), stream_(o.stream_), device_(o.device_)
+        : data_(o.data_), count_(o.count_), stream_(o.stream_), device_(o.device_), owned_(o.owned_)
     {
         o.data_ = nullptr;
         o.count_ = 0;
@@ -61,6 +61,7 @@ public:
             count_ = o.count_;
             stream_ = o.stream_;
             device_ = o.device_;
+            owned_ = o.owned_;
             o.data_ = nullptr;
             o.count_ = 0;
         }
@@ -80,14 +81,6 @@ public:
         }
         count_ = count;
     }
-    void upload(const std::vector<T>& host)
-    {
-        allocate(host.size());
-        if (!host.empty())
-        {
-            check(cudaMemcpy(data_, host.data(), host.size() * sizeof(T), cudaMemcpyHostToDevice), "copying to the device");
-        }
-    }
     // Stream-ordered, from the device's memory pool (no device-wide synchronisation; the pool keeps freed memory for
     // the next request): for arrays that come and go while kernels run, as a server's requests do. `stream` must
     // outlive the array.
@@ -104,7 +97,7 @@ public:
     }
     void release()
     {
-        if (data_)
+        if (data_ && owned_)
         {
             if (stream_)
             {
@@ -130,6 +123,15 @@ public:
         data_ = nullptr;
         count_ = 0;
         stream_ = nullptr;
+        owned_ = true;
+    }
+    // A part of another array's memory, which outlives this view of it
+    void attach(T* data, size_t count)
+    {
+        release();
+        data_ = data;
+        count_ = count;
+        owned_ = false;
     }
     T* data() const { return data_; }
     size_t size() const { return count_; }
@@ -140,7 +142,44 @@ private:
     size_t count_ = 0;
     cudaStream_t stream_ = nullptr; // set when allocated stream-ordered on a caller's stream
     int device_ = 0;                // where allocate() took it
+    bool owned_ = true;
 };
+
+// A scene's tables onto the device in one allocation and one copy: add() each, then commit() into `memory`, whose parts
+// the tables' arrays become (a scene has about thirty; an allocation, a copy and a synchronisation each took most of a
+// millisecond a scene)
+class table_upload
+{
+public:
+    template <class T>
+    void add(device_array<T>& array, const std::vector<T>& host)
+    {
+        if (!host.empty())
+        {
+            items_.push_back({host.data(), host.size() * sizeof(T), 0, [&array, n = host.size()](void* p) {
+                                  array.attach(static_cast<T*>(p), n);
+                              }});
+        }
+    }
+    // (the vectors given to add must still be there)
+    void commit(device_array<unsigned char>& memory);
+
+private:
+    struct item
+    {
+        const void* data;
+        size_t bytes;
+        size_t offset;
+        std::function<void(void*)> attach;
+    };
+    std::vector<item> items_;
+};
+
+// An image: sums[i] * scale into the caller's memory, after what is queued on `stream`
+void fetch_image(const double* sums, int64_t count, double scale, double* out, cudaStream_t stream);
+// Closest hits of rays in the caller's memory (launch_closest_hits)
+void trace_rays(const scene_view& scene, const int32_t* prim_source, const float* origins, const float* directions,
+                int64_t count, int32_t* ids, float* ts);
 
 // The display transform (display.cu): the options' check (renderer.cu:1204-1220) and the kernel over an image's sums
 // times `scale`, queued on `stream`
@@ -187,6 +226,10 @@ private:
     scene_view view_{};
     bool has_f64_ = false;
     scene_view_f64 view_f64_{};
+    // what the tables below are parts of
+    device_array<unsigned char> tables_memory_;
+    device_array<unsigned char> tables_memory_f64_;
+    device_array<unsigned char> environment_memory_;
     device_array<sphere_d> spheres_d_;
     device_array<motion_d> sphere_motion_d_;
     device_array<frame_d> sphere_frames_d_;

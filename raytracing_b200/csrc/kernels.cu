@@ -17,6 +17,9 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <map>
+#include <mutex>
+#include <utility>
 
 #include "ggx_energy_table.h"
 #include "kernels.cuh"
@@ -1645,15 +1648,24 @@ cudaError_t launch_batch_reduce(const batch_params& p, int grid, cudaStream_t st
 }
 
 // Two attribute queries for the device: cudaGetDeviceProperties would fill every field of its description, a cost each
-// session paid
+// session paid. A kernel's attributes are asked for once a device: sessions and servers are made often, and the
+// queries take some 50 us a kernel.
 cudaError_t function_attributes(const void* kernel, kernel_attributes& out)
 {
+    static std::mutex mutex;
+    static auto* known = new std::map<std::pair<const void*, int>, kernel_attributes>();
     cudaFuncAttributes a{};
-    cudaError_t e = cudaFuncGetAttributes(&a, kernel);
     int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
     if (e == cudaSuccess)
     {
-        e = cudaGetDevice(&device);
+        const std::lock_guard<std::mutex> lock(mutex);
+        if (const auto it = known->find({kernel, device}); it != known->end())
+        {
+            out = it->second;
+            return cudaSuccess;
+        }
+        e = cudaFuncGetAttributes(&a, kernel);
     }
     int blocks = 0;
     if (e == cudaSuccess)
@@ -1680,6 +1692,8 @@ cudaError_t function_attributes(const void* kernel, kernel_attributes& out)
     out.threads_per_block = render_block;
     out.max_threads_per_sm = max_threads;
     out.multiprocessors = multiprocessors;
+    const std::lock_guard<std::mutex> lock(mutex);
+    (*known)[{kernel, device}] = out;
     return cudaSuccess;
 }
 

@@ -921,9 +921,11 @@ resident_scene::resident_scene(const rt_scene_desc& d)
     if (d.environment)
     {
         const environment_tables t = build_environment(*d.environment);
-        env_texels_.upload(t.texels);
-        env_bins_.upload(t.bins);
-        env_row_cos_.upload(t.row_cos);
+        table_upload tables;
+        tables.add(env_texels_, t.texels);
+        tables.add(env_bins_, t.bins);
+        tables.add(env_row_cos_, t.row_cos);
+        tables.commit(environment_memory_);
         env.texels = env_texels_.data();
         env.bins = env_bins_.data();
         env.row_cos = env_row_cos_.data();
@@ -996,33 +998,35 @@ resident_scene::resident_scene(const rt_scene_desc& d)
         sphere_motion.assign(spheres.size(), make_float4(0.0f, 0.0f, 0.0f, 0.0f)); // a moving boundary alone moves
     }
 
-    nodes_.upload(tree.nodes);
+    table_upload tables;
+    tables.add(nodes_, tree.nodes);
+    std::vector<bvh4_node> wide;
     // The tree four wide for the wavefront's walk, unless its depth would overflow that walk's stack
     if (!tree.nodes.empty())
     {
-        std::vector<bvh4_node> wide;
         if (collapse_bvh4(tree.nodes, wide) <= max_wide_depth)
         {
-            wide_nodes_.upload(wide);
+            tables.add(wide_nodes_, wide);
         }
     }
-    spheres_.upload(spheres);
-    sphere_motion_.upload(sphere_motion);
-    sphere_frames_.upload(sphere_frames);
-    textures_.upload(textures);
-    images_.upload(images);
-    texels_.upload(texels);
-    noises_.upload(noises);
-    media_.upload(media);
-    boundary_quads_.upload(boundary_quads);
-    quads_.upload(quads);
-    triangles_.upload(triangles);
-    prim_material_.upload(prim_material);
-    prim_source_.upload(prim_source);
-    materials_.upload(materials);
-    lights_.upload(lights);
-    lamps_.upload(lamps);
-    lamp_of_.upload(lamp_of);
+    tables.add(spheres_, spheres);
+    tables.add(sphere_motion_, sphere_motion);
+    tables.add(sphere_frames_, sphere_frames);
+    tables.add(textures_, textures);
+    tables.add(images_, images);
+    tables.add(texels_, texels);
+    tables.add(noises_, noises);
+    tables.add(media_, media);
+    tables.add(boundary_quads_, boundary_quads);
+    tables.add(quads_, quads);
+    tables.add(triangles_, triangles);
+    tables.add(prim_material_, prim_material);
+    tables.add(prim_source_, prim_source);
+    tables.add(materials_, materials);
+    tables.add(lights_, lights);
+    tables.add(lamps_, lamps);
+    tables.add(lamp_of_, lamp_of);
+    tables.commit(tables_memory_);
 
     view_.nodes = nodes_.data();
     view_.wide_nodes = wide_nodes_.data();
@@ -1228,16 +1232,17 @@ resident_scene::resident_scene(const rt_scene_desc& d)
         {
             motion_d_rows.assign(spheres.size(), d4{0.0, 0.0, 0.0, 0.0}); // a moving boundary alone moves
         }
-        spheres_d_.upload(spheres_d);
-        sphere_motion_d_.upload(motion_d_rows);
-        sphere_frames_d_.upload(frames_d);
-        quads_d_.upload(quads_d);
-        materials_d_.upload(materials_d);
-        lights_d_.upload(lights_d);
-        textures_d_.upload(textures_d);
-        noises_d_.upload(noises_d);
-        media_d_.upload(media_d);
-        boundary_quads_d_.upload(boundary_d);
+        tables.add(spheres_d_, spheres_d);
+        tables.add(sphere_motion_d_, motion_d_rows);
+        tables.add(sphere_frames_d_, frames_d);
+        tables.add(quads_d_, quads_d);
+        tables.add(materials_d_, materials_d);
+        tables.add(lights_d_, lights_d);
+        tables.add(textures_d_, textures_d);
+        tables.add(noises_d_, noises_d);
+        tables.add(media_d_, media_d);
+        tables.add(boundary_quads_d_, boundary_d);
+        tables.commit(tables_memory_f64_);
 
         view_f64_.nodes = nodes_.data();
         view_f64_.spheres = spheres_d_.data();

@@ -570,14 +570,7 @@ void session::pixels(double* out, int64_t count) const
     {
         fail(RT_ERR_LOGIC, "pixels: the image has no complete pass");
     }
-    check(cudaMemcpyAsync(out, sums_.data(), static_cast<size_t>(n) * sizeof(double), cudaMemcpyDeviceToHost, stream_),
-          "copying the image");
-    check(cudaStreamSynchronize(stream_), "copying the image");
-    const double scale = 1.0 / static_cast<double>(passes_);
-    for (int64_t i = 0; i < n; ++i)
-    {
-        out[i] *= scale;
-    }
+    fetch_image(sums_.data(), n, 1.0 / static_cast<double>(passes_), out, stream_);
 }
 
 void session::display(const rt_display_options& options, uint8_t* rgba, int64_t byte_count)

@@ -676,15 +676,7 @@ void stream_engine::pixels(int handle, double* out, int64_t count)
         fail(RT_ERR_LOGIC, "pixels: the image has no complete pass");
     }
     // the sums hold r.passes passes once the reductions enqueued so far have run (the accumulator holds the rest)
-    check(cudaMemcpyAsync(out, r.sums.data(), static_cast<size_t>(n) * sizeof(double), cudaMemcpyDeviceToHost,
-                          reduce_stream_),
-          "copying the image");
-    check(cudaStreamSynchronize(reduce_stream_), "copying the image");
-    const double scale = 1.0 / static_cast<double>(r.passes);
-    for (int64_t i = 0; i < n; ++i)
-    {
-        out[i] *= scale;
-    }
+    fetch_image(r.sums.data(), n, 1.0 / static_cast<double>(r.passes), out, reduce_stream_);
 }
 
 void stream_engine::display(int handle, const rt_display_options& options, uint8_t* out, int64_t count)
