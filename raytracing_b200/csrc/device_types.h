@@ -383,6 +383,7 @@ struct camera_d
 struct scene_view_f64
 {
     const bvh_node* nodes;      // the float tree (boxes rounded outward), shared with the float tables
+    const bvh4_node* wide_nodes; // the same four wide (null when it would be too deep)
     const sphere_d* spheres;    // leaf order, as scene_view's
     const quad_d* quads;
     const int32_t* prim_material;

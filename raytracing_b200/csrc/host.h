@@ -465,6 +465,7 @@ private:
     bool pool_ = false;                 // AUTO's wavefront: the pool kernel
     int pool_grid_ = 0;
     device_array<float4> pool_samples_; // a pool launch's samples, kept for the next
+    device_array<double> samples_f64_;  // the same of an FP64 session
     int32_t last_kernel_launches_ = 0; // the last launch's kernels
     wave_shape shape_{};                // how a step is launched (the autotuner's choice or the defaults)
     tune_candidate tuned_{};

@@ -1650,7 +1650,7 @@ cudaError_t launch_batch_reduce(const batch_params& p, int grid, cudaStream_t st
 // Two attribute queries for the device: cudaGetDeviceProperties would fill every field of its description, a cost each
 // session paid. A kernel's attributes are asked for once a device: sessions and servers are made often, and the
 // queries take some 50 us a kernel.
-cudaError_t function_attributes(const void* kernel, kernel_attributes& out)
+cudaError_t function_attributes(const void* kernel, kernel_attributes& out, int shared)
 {
     static std::mutex mutex;
     static auto* known = new std::map<std::pair<const void*, int>, kernel_attributes>();
@@ -1670,7 +1670,7 @@ cudaError_t function_attributes(const void* kernel, kernel_attributes& out)
     int blocks = 0;
     if (e == cudaSuccess)
     {
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, render_block, 0);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, render_block, static_cast<size_t>(shared));
     }
     int multiprocessors = 0;
     int max_threads = 0;

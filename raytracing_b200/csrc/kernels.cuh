@@ -177,8 +177,9 @@ struct kernel_attributes
     int multiprocessors;
 };
 
-// A kernel's registers, local memory and resident blocks, and the device's multiprocessors
-cudaError_t function_attributes(const void* kernel, kernel_attributes& out);
+// A kernel's registers, local memory and resident blocks (with `shared` bytes of dynamic shared memory a block), and the
+// device's multiprocessors
+cudaError_t function_attributes(const void* kernel, kernel_attributes& out, int shared = 0);
 
 constexpr int render_block = 128;
 
@@ -295,8 +296,9 @@ cudaError_t prepare_pool(unsigned long long* work_counter, cudaStream_t stream);
 pool_launch pool_launch_of(int64_t sample_count, int grid);
 
 // The books' integrator in double (precision::float64; renderer.h:402-409, all_books_kernel<double>,
-// renderer.cu:445-451): a persistent launch over the same (pixel, chunk) work items as launch_params' and into the
-// same chunk partials, so launch_reduce adds them into the sums. Its own random numbers: 53-bit uniforms.
+// renderer.cu:445-451): the samples of launch_params' passes and pixels by a pool kernel in double, their values added
+// into the sums by launch_reduce_f64 as launch_wave_reduce adds a float launch's. Its own random numbers: 53-bit
+// uniforms.
 struct launch_params_f64
 {
     scene_view_f64 scene;
@@ -304,19 +306,19 @@ struct launch_params_f64
     uint64_t seed;
     int64_t pass_begin;
     int64_t pass_end;
-    int64_t first_chunk;
+    int64_t sample_count;   // (pass_end - pass_begin) * padded_pixels
     int32_t chunk;
-    int32_t chunks;
     int32_t tiles_x;
     int32_t padded_pixels;
-    int64_t total_items;
     int32_t round_passes;
+    int32_t claim;          // set by the launch
     int32_t pad0;
     unsigned long long* work_counter;
-    double* partials;
+    double* samples;              // 3 a sample
     unsigned long long* counters; // [0] path segments
 };
 cudaError_t launch_render_f64(const launch_params_f64& p, int grid, cudaStream_t stream);
+cudaError_t launch_reduce_f64(const launch_params_f64& p, double* sums, cudaStream_t stream);
 cudaError_t render_f64_attributes(const scene_view_f64& scene, kernel_attributes& out);
 
 // Parity hooks: closest hits of given rays (source ids through prim_source), and the camera rays of one pass

@@ -18,6 +18,7 @@
 
 #include "kernels.cuh"
 #include "philox.cuh"
+#include "rounding.cuh"
 #include "rt_b200.h"
 
 namespace rtb
@@ -31,13 +32,47 @@ __device__ __forceinline__ v3 operator-(v3 a, v3 b) { return make_double3(a.x - 
 __device__ __forceinline__ v3 operator-(v3 a) { return make_double3(-a.x, -a.y, -a.z); }
 __device__ __forceinline__ v3 operator*(double t, v3 v) { return make_double3(t * v.x, t * v.y, t * v.z); }
 __device__ __forceinline__ v3 operator*(v3 a, v3 b) { return make_double3(a.x * b.x, a.y * b.y, a.z * b.z); }
-__device__ __forceinline__ double dot(v3 a, v3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__device__ __forceinline__ double length_squared(v3 v) { return dot(v, v); }
-__device__ __forceinline__ v3 unit_vector(v3 v) { return (1.0 / sqrt(length_squared(v))) * v; }
-__device__ __forceinline__ v3 reflect(v3 v, v3 n) { return v - (2.0 * dot(v, n)) * n; }
+// The dot products' roundings are written out (rounding.cuh), so that an image does not depend on what the compiler makes
+// of a product's surroundings: path after path of mirrors and glass would grow a last bit into another image. (A
+// mirror's is left to it: none of the written forms is the one its images have been rendered with.)
+template <rounding R = rounding::x>
+__device__ __forceinline__ double dot(v3 a, v3 b)
+{
+    if constexpr (R == rounding::x)
+    {
+        return __fma_rn(a.z, b.z, __fma_rn(a.x, b.x, __dmul_rn(a.y, b.y)));
+    }
+    else if constexpr (R == rounding::y)
+    {
+        return __fma_rn(a.z, b.z, __fma_rn(a.y, b.y, __dmul_rn(a.x, b.x)));
+    }
+    else if constexpr (R == rounding::yz)
+    {
+        return __dadd_rn(__dmul_rn(a.z, b.z), __fma_rn(a.y, b.y, __dmul_rn(a.x, b.x)));
+    }
+    else
+    {
+        return a.x * b.x + a.y * b.y + a.z * b.z;
+    }
+}
+template <rounding R = rounding::x>
+__device__ __forceinline__ double length_squared(v3 v)
+{
+    return dot<R>(v, v);
+}
+template <rounding R = rounding::x>
+__device__ __forceinline__ v3 unit_vector(v3 v)
+{
+    return (1.0 / sqrt(length_squared<R>(v))) * v;
+}
+template <rounding R = rounding::x>
+__device__ __forceinline__ v3 reflect(v3 v, v3 n)
+{
+    return v - (2.0 * dot<R>(v, n)) * n;
+}
 __device__ __forceinline__ v3 refract(v3 uv, v3 n, double etai_over_etat) // vec3.cuh refract
 {
-    const double cos_theta = fmin(dot(-uv, n), 1.0);
+    const double cos_theta = fmin(dot<rounding::yz>(-uv, n), 1.0);
     const v3 r_out_perp = etai_over_etat * (uv + cos_theta * n);
     const v3 r_out_parallel = -sqrt(fabs(1.0 - length_squared(r_out_perp))) * n;
     return r_out_perp + r_out_parallel;
@@ -297,7 +332,7 @@ __device__ hit_info closest_hit(const scene_view_f64& S, v3 o, v3 d, double time
     {
         return hit;
     }
-    const double inverse_a = 1.0 / length_squared(d);
+    const double inverse_a = 1.0 / length_squared<rounding::y>(d);
     if (S.flat)
     {
         for (int i = 0; i < S.quad_base; ++i)
@@ -443,7 +478,7 @@ __device__ void media_event(const scene_view_f64& S, v3 o, v3 d, double time, co
 {
     const double inverse_a = 1.0 / length_squared(d);
     const v3 inv = make_double3(safe_inverse(d.x), safe_inverse(d.y), safe_inverse(d.z));
-    const double length = sqrt(length_squared(d));
+    const double length = sqrt(length_squared<rounding::y>(d));
     uniforms u{};
     for (int k = 0; k < S.medium_count; ++k)
     {
@@ -654,7 +689,7 @@ __device__ __forceinline__ void camera_ray(const camera_d& cam, int i, int j, in
 
 __device__ __forceinline__ v3 sky(const camera_d& cam, v3 direction)
 {
-    const double a = 0.5 * (unit_vector(direction).y + 1.0);
+    const double a = 0.5 * (unit_vector<rounding::y>(direction).y + 1.0);
     return (1.0 - a) * vec(cam.sky_bottom) + a * vec(cam.sky_top);
 }
 
@@ -848,7 +883,7 @@ __device__ bool shade_books(const scene_view_f64& S, const camera_d& cam, const 
     }
     else if (m.kind == RT_METAL)
     {
-        direction = unit_vector(reflect(ps.d, s.normal)) + m.fuzz * random_unit_vector(u.x, u.y);
+        direction = unit_vector<rounding::compiler>(reflect(ps.d, s.normal)) + m.fuzz * random_unit_vector(u.x, u.y);
         if (dot(direction, s.normal) <= 0.0)
         {
             sample = black;
@@ -859,11 +894,11 @@ __device__ bool shade_books(const scene_view_f64& S, const camera_d& cam, const 
     else // dielectric
     {
         const double ri = h.front ? 1.0 / m.ior : m.ior;
-        const v3 ud = unit_vector(ps.d);
-        const double cos_theta = fmin(dot(-ud, s.normal), 1.0);
+        const v3 ud = unit_vector<rounding::y>(ps.d);
+        const double cos_theta = fmin(dot<rounding::yz>(-ud, s.normal), 1.0);
         const double sin_theta = sqrt(1.0 - cos_theta * cos_theta);
         const bool cannot_refract = ri * sin_theta > 1.0;
-        direction = cannot_refract || reflectance(cos_theta, ri) > u.z ? reflect(ud, s.normal)
+        direction = cannot_refract || reflectance(cos_theta, ri) > u.z ? reflect<rounding::yz>(ud, s.normal)
                                                                        : refract(ud, s.normal, ri);
     }
     if (--ps.rays_left == 0)
@@ -878,163 +913,441 @@ __device__ bool shade_books(const scene_view_f64& S, const camera_d& cam, const 
     return false;
 }
 
-// The persistent launch: lanes claim (pixel, chunk) items by a warp ballot and one atomic a warp, as render_kernel does
-// in float, trace one segment an iteration and start the next sample the moment one ends
-__global__ void __launch_bounds__(render_block) render_f64_kernel(const __grid_constant__ launch_params_f64 P)
-{
-    __shared__ unsigned long long block_rays;
-    if (threadIdx.x == 0)
-    {
-        block_rays = 0;
-    }
-    __syncthreads();
+// ---- the pool kernel in double ----------------------------------------------------------------------------------
+// The float pool kernel's form (pool_kernel.cuh): a persistent warp keeps 64 paths in shared memory and walks, shades
+// and starts them a warp's worth at a time; each finished sample's value goes to its place in a buffer that
+// reduce_f64_kernel adds up in pass order, chunk by chunk. Against a persistent kernel with a path bound to each lane
+// (162 registers, 12 warps a multiprocessor, walks and materials of a warp's lanes one after the other).
+constexpr unsigned full_warp = 0xffffffffu;
+constexpr int pool_paths = 64;
+constexpr int pool_refill = 20;
 
+struct pool_record
+{
+    double o[3][pool_paths], d[3][pool_paths], throughput[3][pool_paths];
+    double time[pool_paths], hit_t[pool_paths];
+    uint32_t pixel[pool_paths], pass[pool_paths], key[pool_paths], sample[pool_paths];
+    uint32_t meta[pool_paths]; // depth << 1 | the ray starts inside the surface it leaves
+    int32_t from[pool_paths];
+    int32_t hit[pool_paths]; // id << 1 | front, or -1
+    uint8_t walk[pool_paths], shade[pool_paths], free[pool_paths];
+};
+
+// A ray against the tree four wide in float: conservative, so that the walk meets every primitive the ray meets in
+// double. A plane at n is met at T = (n - o) / d; fmaf(n, inv, -c) is off it by at most 2^-24 (2 |T| + 4 |o / d|), the
+// direction's reciprocal, the origin and two products rounded; the near bound is set back and the far bound out by
+// 2^-20 |o / d| and the boxes' margin, and what is proportional to T by a factor of 1 + 2^-20 on the entry's side.
+struct float_ray
+{
+    float3 inv, near, far; // a near plane is met at fmaf(n, inv, -near), a far one at fmaf(n, inv, -far)
+    uint32_t x, y, z;      // where the near bounds of an axis lie in a node (the far ones 16 bytes off)
+};
+
+__device__ __forceinline__ float_ray float_ray_of(v3 o, v3 d, double margin)
+{
+    const v3 inv = make_double3(safe_inverse(d.x), safe_inverse(d.y), safe_inverse(d.z));
+    const auto axis = [&](double oa, double ia, float& f, float& near, float& far) {
+        f = static_cast<float>(ia);
+        const float os = static_cast<float>(oa) * f;
+        const float w = fmaf(fabsf(os), 0x1p-20f, __double2float_ru(margin) * fabsf(f) * 1.001f);
+        near = os + w;
+        far = os - w;
+    };
+    float_ray r;
+    axis(o.x, inv.x, r.inv.x, r.near.x, r.far.x);
+    axis(o.y, inv.y, r.inv.y, r.near.y, r.far.y);
+    axis(o.z, inv.z, r.inv.z, r.near.z, r.far.z);
+    r.x = inv.x < 0.0 ? 16u : 0u;
+    r.y = inv.y < 0.0 ? 48u : 32u;
+    r.z = inv.z < 0.0 ? 80u : 64u;
+    return r;
+}
+
+// STEPS: walks of the tree four wide, a lane's resumed from phase to phase; otherwise a whole search a phase
+// (closest_hit: a flat scene, or a tree too deep to be four wide)
+template <bool STEPS>
+__global__ void __launch_bounds__(render_block, 4) pool_f64_kernel(const __grid_constant__ launch_params_f64 P)
+{
+    extern __shared__ __align__(16) unsigned char shared[];
+    pool_record& R = reinterpret_cast<pool_record*>(shared)[threadIdx.x >> 5];
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lanes_below = (1u << lane) - 1u;
     const camera_d& cam = P.cam;
     const scene_view_f64& S = P.scene;
-
+    const auto put = [](double (*rows)[pool_paths], int p, v3 v) {
+        rows[0][p] = v.x;
+        rows[1][p] = v.y;
+        rows[2][p] = v.z;
+    };
+    const auto get = [](const double (*rows)[pool_paths], int p) {
+        return make_double3(rows[0][p], rows[1][p], rows[2][p]);
+    };
+    const auto push = [&](uint8_t* list, int count, bool which, int p) -> int {
+        const unsigned lanes = __ballot_sync(full_warp, which);
+        if (which)
+        {
+            list[count + __popc(lanes & lanes_below)] = static_cast<uint8_t>(p);
+        }
+        return count + __popc(lanes);
+    };
+    for (int p = static_cast<int>(lane); p < pool_paths; p += 32)
+    {
+        R.free[p] = static_cast<uint8_t>(p);
+    }
+    __syncwarp();
+    int walk_count = 0, shade_count = 0, free_count = pool_paths;
+    const auto limit = static_cast<unsigned long long>(P.sample_count);
+    bool dry = limit == 0ull;
     uint32_t rays = 0;
-    bool need = true;
-    bool start = false;
-    int px = 0, py = 0;
-    int64_t pass = 0, pass_end = 0;
-    int64_t slot = 0;
-    double acc_r = 0.0, acc_g = 0.0, acc_b = 0.0;
-    sampler rng{};
-    path_state ps{};
-
+    int slot = -1; // the path this lane walks for
+    int link = traversal_done_link;
+    int sp = 0;
+    hit_info hit{-1, infinity_d, false};
+    int2 stack[STEPS ? wide_stack : 1];
     while (true)
     {
-        const unsigned active = __activemask();
-        const unsigned needing = __ballot_sync(active, need);
-        if (needing != 0u)
+        enum class phase
         {
-            const int leader = __ffs(static_cast<int>(needing)) - 1;
-            unsigned long long base = 0;
-            if (static_cast<int>(lane) == leader)
+            walk,
+            start,
+            shade,
+            end
+        } next;
+        const int startable = dry ? 0 : free_count;
+        if constexpr (STEPS)
+        {
+            const bool answered = slot >= 0 && link == traversal_done_link;
+            if (answered)
             {
-                base = atomicAdd(P.work_counter, static_cast<unsigned long long>(__popc(needing)));
+                R.hit_t[slot] = hit.t;
+                R.hit[slot] = hit.id < 0 ? -1 : (hit.id << 1) | (hit.front ? 1 : 0);
             }
-            base = __shfl_sync(active, base, leader);
-            if (need)
+            shade_count = push(R.shade, shade_count, answered, slot);
+            slot = answered ? -1 : slot;
+            const unsigned idle = __ballot_sync(full_warp, slot < 0);
+            const int taken = min(__popc(idle), walk_count);
+            const int rank = __popc(idle & lanes_below);
+            __syncwarp();
+            if (slot < 0 && rank < taken)
             {
-                const unsigned long long item = base + static_cast<unsigned long long>(__popc(needing & lanes_below));
-                if (item >= static_cast<unsigned long long>(P.total_items))
+                slot = R.walk[walk_count - 1 - rank];
+                hit = {-1, infinity_d, false};
+                sp = 0;
+                link = 0;
+            }
+            walk_count -= taken;
+            const int walking = __popc(__ballot_sync(full_warp, slot >= 0));
+            const bool few = walking < pool_refill && walking * 8 < (walking + shade_count + startable) * 5;
+            next = walk_count == 0 && few ? (startable > shade_count ? phase::start : phase::shade)
+                   : walking > 0          ? phase::walk
+                                          : phase::end;
+        }
+        else if (walk_count >= 32 || (walk_count >= startable && walk_count >= shade_count))
+        {
+            next = walk_count > 0 ? phase::walk : phase::end;
+        }
+        else
+        {
+            next = startable > shade_count ? phase::start : phase::shade;
+        }
+        if (next == phase::end)
+        {
+            break;
+        }
+        if (next == phase::walk && !STEPS)
+        {
+            const int taken = min(32, walk_count);
+            const bool mine = static_cast<int>(lane) < taken;
+            const int p = mine ? R.walk[walk_count - taken + static_cast<int>(lane)] : 0;
+            walk_count -= taken;
+            if (mine)
+            {
+                const hit_info h = closest_hit(S, get(R.o, p), get(R.d, p), R.time[p], R.from[p], (R.meta[p] & 1u) != 0u);
+                R.hit_t[p] = h.t;
+                R.hit[p] = h.id < 0 ? -1 : (h.id << 1) | (h.front ? 1 : 0);
+            }
+            shade_count = push(R.shade, shade_count, mine, p);
+            __syncwarp();
+            continue;
+        }
+        if (next == phase::walk)
+        {
+            const bool walks = slot >= 0;
+            const int p = walks ? slot : 0;
+            const float_ray r = float_ray_of(get(R.o, p), get(R.d, p), S.box_margin);
+            float bound = __double2float_ru(hit.t); // the closest hit so far, rounded up
+            const auto pop = [&]() -> int {
+                while (sp > 0)
+                {
+                    const int2 e = stack[--sp];
+                    if (__int_as_float(e.y) < bound)
+                    {
+                        return e.x;
+                    }
+                }
+                return traversal_done_link;
+            };
+            const int total =
+                __popc(__ballot_sync(full_warp, walks)) + walk_count + shade_count + (dry ? 0 : free_count);
+            const int enough = min(pool_refill, (total * 5 + 7) / 8);
+            while (true)
+            {
+                while (__any_sync(full_warp, walks && link >= 0))
+                {
+                    if (walks && link >= 0)
+                    {
+                        const char* const node = reinterpret_cast<const char*>(S.wide_nodes + link);
+                        const auto row = [&](uint32_t at) { return __ldg(reinterpret_cast<const float4*>(node + at)); };
+                        const float4 nx = row(r.x), fx = row(r.x ^ 16u);
+                        const float4 ny = row(r.y), fy = row(r.y ^ 16u);
+                        const float4 nz = row(r.z), fz = row(r.z ^ 16u);
+                        const int4 nl = __ldg(reinterpret_cast<const int4*>(S.wide_nodes[link].link));
+                        const auto entry = [&](float ax, float bx, float ay, float by, float az, float bz,
+                                               int child) -> float {
+                            const float enter =
+                                0x1.ffffep-1f * fmaxf(fmaxf(fmaf(ax, r.inv.x, -r.near.x), fmaf(ay, r.inv.y, -r.near.y)),
+                                                      fmaxf(fmaf(az, r.inv.z, -r.near.z), 0.00099f));
+                            const float exit = fminf(fminf(fmaf(bx, r.inv.x, -r.far.x), fmaf(by, r.inv.y, -r.far.y)),
+                                                     fminf(fmaf(bz, r.inv.z, -r.far.z), bound));
+                            return enter <= exit * 0x1.00001p+0f && child != traversal_done_link
+                                       ? enter
+                                       : __int_as_float(0x7f800000);
+                        };
+                        float k0 = entry(nx.x, fx.x, ny.x, fy.x, nz.x, fz.x, nl.x);
+                        float k1 = entry(nx.y, fx.y, ny.y, fy.y, nz.y, fz.y, nl.y);
+                        float k2 = entry(nx.z, fx.z, ny.z, fy.z, nz.z, fz.z, nl.z);
+                        float k3 = entry(nx.w, fx.w, ny.w, fy.w, nz.w, fz.w, nl.w);
+                        int l0 = nl.x, l1 = nl.y, l2 = nl.z, l3 = nl.w;
+                        const auto order = [](float& ka, int& la, float& kb, int& lb) {
+                            if (kb < ka)
+                            {
+                                const float k = ka;
+                                ka = kb;
+                                kb = k;
+                                const int l = la;
+                                la = lb;
+                                lb = l;
+                            }
+                        };
+                        order(k0, l0, k1, l1);
+                        order(k2, l2, k3, l3);
+                        order(k0, l0, k2, l2);
+                        order(k1, l1, k3, l3);
+                        order(k1, l1, k2, l2);
+                        const auto met = [](float k) { return k < __int_as_float(0x7f800000); };
+                        if (met(k3))
+                        {
+                            stack[sp++] = make_int2(l3, __float_as_int(k3));
+                        }
+                        if (met(k2))
+                        {
+                            stack[sp++] = make_int2(l2, __float_as_int(k2));
+                        }
+                        if (met(k1))
+                        {
+                            stack[sp++] = make_int2(l1, __float_as_int(k1));
+                        }
+                        link = met(k0) ? l0 : pop();
+                    }
+                }
+                // every walking lane holds a leaf, or is done
+                if (walks && link != traversal_done_link)
+                {
+                    const v3 d = get(R.d, p);
+                    test_leaf(S, link, get(R.o, p), d, R.time[p], 1.0 / length_squared<rounding::y>(d), R.from[p],
+                              (R.meta[p] & 1u) != 0u, hit);
+                    bound = __double2float_ru(hit.t);
+                    link = pop();
+                }
+                if (__popc(__ballot_sync(full_warp, walks && link != traversal_done_link)) < enough)
                 {
                     break;
                 }
-                const int64_t k = static_cast<int64_t>(item / static_cast<unsigned long long>(P.padded_pixels));
-                const int q = static_cast<int>(item % static_cast<unsigned long long>(P.padded_pixels));
-                const int tile = q >> 5;
-                const int l = q & 31;
-                px = (tile % P.tiles_x) * 8 + (l & 7);
-                py = (tile / P.tiles_x) * 4 + (l >> 3);
-                if (px >= cam.width || py >= cam.height)
-                {
-                    continue; // a lane of a tile over the image's edge
-                }
-                const int64_t chunk_first = (P.first_chunk + k) * P.chunk;
-                pass = chunk_first > P.pass_begin ? chunk_first : P.pass_begin;
-                const int64_t chunk_end = chunk_first + P.chunk;
-                pass_end = chunk_end < P.pass_end ? chunk_end : P.pass_end;
-                slot = k * P.padded_pixels + q;
-                acc_r = acc_g = acc_b = 0.0;
-                rng.pixel = static_cast<uint32_t>(py) * static_cast<uint32_t>(cam.width) + static_cast<uint32_t>(px);
-                need = false;
-                start = true;
             }
+            __syncwarp();
+            continue;
         }
-        if (start)
+        if (next == phase::start)
         {
-            // Pass n is pass n % k^2 of round n / k^2, whose numbers come from seed + round * 2^32
-            const int64_t round = pass / P.round_passes;
-            const int in_round = static_cast<int>(pass - round * P.round_passes);
-            const uint64_t key = P.seed + (static_cast<uint64_t>(round) << 32);
-            rng.key = make_uint2(static_cast<uint32_t>(key), static_cast<uint32_t>(key >> 32));
-            rng.pass = static_cast<uint32_t>(in_round);
-            camera_ray(cam, px, py, in_round % cam.sqrt_spp, in_round / cam.sqrt_spp, rng.draw(0, block_material),
-                       ps.o, ps.d);
-            ps.time = S.has_motion ? rng.draw(0, block_time).x : 0.0;
-            ps.throughput = make_double3(1.0, 1.0, 1.0);
-            ps.rays_left = cam.max_depth;
-            ps.depth = 0;
-            ps.from = -1;
-            ps.inward = false;
-            start = false;
-        }
-
-        hit_info h = closest_hit(S, ps.o, ps.d, ps.time, ps.from, ps.inward);
-        ++rays;
-        ++ps.depth;
-        if (S.medium_count > 0)
-        {
-            media_event(S, ps.o, ps.d, ps.time, rng, ps.depth, h);
-        }
-        v3 sample;
-        if (shade_books(S, cam, rng, ps, h, sample))
-        {
-            acc_r += without_nan(sample.x);
-            acc_g += without_nan(sample.y);
-            acc_b += without_nan(sample.z);
-            if (++pass == pass_end)
+            const int wanted = min(min(32, free_count), P.claim);
+            unsigned long long base = 0;
+            if (lane == 0u)
             {
-                double* out = P.partials + 3 * slot;
-                out[0] = acc_r;
-                out[1] = acc_g;
-                out[2] = acc_b;
-                need = true;
+                base = atomicAdd(P.work_counter, static_cast<unsigned long long>(wanted));
+            }
+            base = __shfl_sync(full_warp, base, 0);
+            dry = base + static_cast<unsigned long long>(wanted) >= limit;
+            const unsigned long long s = base + lane;
+            bool started = static_cast<int>(lane) < wanted && s < limit;
+            int px = 0, py = 0;
+            int64_t pass = 0;
+            if (started)
+            {
+                // sample s: pass-major, then the pixels in 8 x 4 tiles; off the image for a tile over its edge
+                const auto padded = static_cast<unsigned long long>(P.padded_pixels);
+                const int q = static_cast<int>(s % padded);
+                pass = P.pass_begin + static_cast<int64_t>(s / padded);
+                const int tile = q >> 5;
+                px = (tile % P.tiles_x) * 8 + (q & 7);
+                py = (tile / P.tiles_x) * 4 + ((q & 31) >> 3);
+                started = px < cam.width && py < cam.height;
+            }
+            const unsigned lanes = __ballot_sync(full_warp, started);
+            const int p = started ? R.free[free_count - 1 - __popc(lanes & lanes_below)] : 0;
+            __syncwarp();
+            free_count -= __popc(lanes);
+            if (started)
+            {
+                // Pass n is pass n % k^2 of round n / k^2, whose numbers come from seed + round * 2^32
+                const int64_t round = pass / P.round_passes;
+                const int in_round = static_cast<int>(pass - round * P.round_passes);
+                const uint64_t key = P.seed + (static_cast<uint64_t>(round) << 32);
+                sampler rng;
+                rng.key = make_uint2(static_cast<uint32_t>(key), static_cast<uint32_t>(key >> 32));
+                rng.pass = static_cast<uint32_t>(in_round);
+                rng.pixel = static_cast<uint32_t>(py) * static_cast<uint32_t>(cam.width) + static_cast<uint32_t>(px);
+                v3 o, d;
+                camera_ray(cam, px, py, in_round % cam.sqrt_spp, in_round / cam.sqrt_spp, rng.draw(0, block_material), o,
+                           d);
+                put(R.o, p, o);
+                put(R.d, p, d);
+                put(R.throughput, p, make_double3(1.0, 1.0, 1.0));
+                R.time[p] = S.has_motion ? rng.draw(0, block_time).x : 0.0;
+                R.pixel[p] = rng.pixel;
+                R.pass[p] = rng.pass;
+                R.key[p] = rng.key.y;
+                R.sample[p] = static_cast<uint32_t>(s);
+                R.meta[p] = 0u;
+                R.from[p] = -1;
+            }
+            walk_count = push(R.walk, walk_count, started, p);
+            rays += static_cast<uint32_t>(__popc(lanes));
+            __syncwarp();
+            continue;
+        }
+        const int taken = min(32, shade_count);
+        const bool mine = static_cast<int>(lane) < taken;
+        const int p = mine ? R.shade[shade_count - taken + static_cast<int>(lane)] : 0;
+        shade_count -= taken;
+        bool goes_on = false;
+        if (mine)
+        {
+            path_state ps;
+            ps.o = get(R.o, p);
+            ps.d = get(R.d, p);
+            ps.throughput = get(R.throughput, p);
+            ps.time = R.time[p];
+            ps.depth = static_cast<int>(R.meta[p] >> 1);
+            ps.inward = (R.meta[p] & 1u) != 0u;
+            ps.rays_left = cam.max_depth - ps.depth;
+            ps.from = R.from[p];
+            sampler rng;
+            rng.pixel = R.pixel[p];
+            rng.pass = R.pass[p];
+            rng.key = make_uint2(static_cast<uint32_t>(P.seed), R.key[p]);
+            const int answer = R.hit[p];
+            hit_info h{answer < 0 ? -1 : answer >> 1, R.hit_t[p], (answer & 1) != 0};
+            ++ps.depth;
+            if (S.medium_count > 0)
+            {
+                media_event(S, ps.o, ps.d, ps.time, rng, ps.depth, h);
+            }
+            v3 sample;
+            goes_on = !shade_books(S, cam, rng, ps, h, sample);
+            if (goes_on)
+            {
+                put(R.o, p, ps.o);
+                put(R.d, p, ps.d);
+                put(R.throughput, p, ps.throughput);
+                R.meta[p] = (static_cast<uint32_t>(ps.depth) << 1) | (ps.inward ? 1u : 0u);
+                R.from[p] = ps.from;
             }
             else
             {
-                start = true;
+                double* const out = P.samples + 3 * static_cast<int64_t>(R.sample[p]);
+                out[0] = without_nan(sample.x);
+                out[1] = without_nan(sample.y);
+                out[2] = without_nan(sample.z);
             }
         }
+        walk_count = push(R.walk, walk_count, goes_on, p);
+        free_count = push(R.free, free_count, mine && !goes_on, p);
+        rays += static_cast<uint32_t>(__popc(__ballot_sync(full_warp, goes_on)));
+        __syncwarp();
     }
-    atomicAdd(&block_rays, static_cast<unsigned long long>(rays));
-    __syncthreads();
-    if (threadIdx.x == 0)
+    if (lane == 0u && rays != 0u)
     {
-        atomicAdd(P.counters, block_rays);
+        atomicAdd(P.counters, static_cast<unsigned long long>(rays));
     }
 }
+
+// The launch's samples into the image's sums: each chunk's in pass order into its partial, the partials in chunk order
+__global__ void reduce_f64_kernel(const __grid_constant__ launch_params_f64 P, double* sums)
+{
+    const int x = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
+    const int y = static_cast<int>(blockIdx.y);
+    if (x >= P.cam.width || y >= P.cam.height)
+    {
+        return;
+    }
+    const int q = ((y >> 2) * P.tiles_x + (x >> 3)) * 32 + ((y & 3) << 3) + (x & 7);
+    double* const sum = sums + 3 * (static_cast<int64_t>(y) * P.cam.width + x);
+    double r = sum[0], g = sum[1], b = sum[2];
+    for (int64_t pass = P.pass_begin; pass < P.pass_end;)
+    {
+        const int64_t chunk_end = (pass / P.chunk + 1) * P.chunk;
+        const int64_t end = chunk_end < P.pass_end ? chunk_end : P.pass_end;
+        double pr = 0.0, pg = 0.0, pb = 0.0;
+        for (; pass < end; ++pass)
+        {
+            const double* const s = P.samples + 3 * ((pass - P.pass_begin) * P.padded_pixels + q);
+            pr += s[0];
+            pg += s[1];
+            pb += s[2];
+        }
+        r += pr;
+        g += pg;
+        b += pb;
+    }
+    sum[0] = r;
+    sum[1] = g;
+    sum[2] = b;
+}
+
+using pool_f64_function = void (*)(launch_params_f64);
+
+pool_f64_function pool_f64_of(const scene_view_f64& scene)
+{
+    return scene.flat == 0 && scene.wide_nodes != nullptr && scene.node_count > 0 ? pool_f64_kernel<true>
+                                                                                   : pool_f64_kernel<false>;
+}
+
+constexpr int pool_f64_shared = render_block / 32 * static_cast<int>(sizeof(pool_record));
 } // namespace
 
 cudaError_t launch_render_f64(const launch_params_f64& p, int grid, cudaStream_t stream)
 {
-    render_f64_kernel<<<grid, render_block, 0, stream>>>(p);
+    launch_params_f64 q = p;
+    const pool_launch l = pool_launch_of(p.sample_count, grid);
+    q.claim = l.claim;
+    if (const cudaError_t e = prepare_pool(p.work_counter, stream); e != cudaSuccess)
+    {
+        return e;
+    }
+    pool_f64_of(p.scene)<<<l.blocks, render_block, pool_f64_shared, stream>>>(q);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_reduce_f64(const launch_params_f64& p, double* sums, cudaStream_t stream)
+{
+    const dim3 block(128, 1);
+    const dim3 grid(static_cast<unsigned>((p.cam.width + 127) / 128), static_cast<unsigned>(p.cam.height));
+    reduce_f64_kernel<<<grid, block, 0, stream>>>(p, sums);
     return cudaGetLastError();
 }
 
 cudaError_t render_f64_attributes(const scene_view_f64& scene, kernel_attributes& out)
 {
-    (void)scene;
-    cudaFuncAttributes a{};
-    cudaError_t e = cudaFuncGetAttributes(&a, render_f64_kernel);
-    if (e != cudaSuccess)
-    {
-        return e;
-    }
-    int device = 0;
-    e = cudaGetDevice(&device);
-    if (e != cudaSuccess)
-    {
-        return e;
-    }
-    e = cudaDeviceGetAttribute(&out.multiprocessors, cudaDevAttrMultiProcessorCount, device);
-    if (e != cudaSuccess)
-    {
-        return e;
-    }
-    e = cudaDeviceGetAttribute(&out.max_threads_per_sm, cudaDevAttrMaxThreadsPerMultiProcessor, device);
-    if (e != cudaSuccess)
-    {
-        return e;
-    }
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&out.blocks_per_sm, render_f64_kernel, render_block, 0);
-    out.registers = a.numRegs;
-    out.local_bytes = static_cast<int>(a.localSizeBytes);
-    out.threads_per_block = render_block;
-    return e;
+    return function_attributes(reinterpret_cast<const void*>(pool_f64_of(scene)), out, pool_f64_shared);
 }
 } // namespace rtb

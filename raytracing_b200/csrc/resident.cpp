@@ -1245,6 +1245,7 @@ resident_scene::resident_scene(const rt_scene_desc& d)
         tables.commit(tables_memory_f64_);
 
         view_f64_.nodes = nodes_.data();
+        view_f64_.wide_nodes = wide_nodes_.data();
         view_f64_.spheres = spheres_d_.data();
         view_f64_.quads = quads_d_.data();
         view_f64_.prim_material = prim_material_.data();

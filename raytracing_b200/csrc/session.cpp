@@ -247,6 +247,7 @@ session::~session()
     rgba_.release();
     partials_.release();
     pool_samples_.release();
+    samples_f64_.release();
     sums_.release();
     counters_.release();
     if (start_)
@@ -315,9 +316,10 @@ int64_t session::plan(int64_t target, double budget_seconds) const
         end = std::max(next_chunk, end / pass_chunk * pass_chunk);
     }
     // At most what the partials buffer holds (the wavefront: its samples buffer)
+    const size_t sample_bytes = f64_ ? 3 * sizeof(double) : sizeof(float4);
     const int64_t max_chunks =
-        (wavefront_ || pool_) && !counting_
-            ? std::max<int64_t>(1, static_cast<int64_t>(wave_sample_budget_bytes / sizeof(float4)) /
+        (wavefront_ || pool_ || f64_) && !counting_
+            ? std::max<int64_t>(1, static_cast<int64_t>(wave_sample_budget_bytes / sample_bytes) /
                                        (static_cast<int64_t>(padded_pixels_) * pass_chunk))
             : std::max<int64_t>(1, max_partial_entries_ / padded_pixels_);
     end = std::min(end, (passes_ / pass_chunk + max_chunks) * pass_chunk);
@@ -329,8 +331,16 @@ double session::launch(int64_t end)
     const int64_t first_chunk = passes_ / pass_chunk;
     const int64_t chunks = (end + pass_chunk - 1) / pass_chunk - first_chunk;
     const bool wave = (wavefront_ || pool_) && !counting_;
+    const int64_t samples = static_cast<int64_t>(padded_pixels_) * (end - passes_);
     const size_t needed = static_cast<size_t>(chunks) * static_cast<size_t>(padded_pixels_) * 3;
-    if (!wave && partials_.size() < needed)
+    if (f64_)
+    {
+        if (samples_f64_.size() < 3 * static_cast<size_t>(samples))
+        {
+            samples_f64_.allocate_async(3 * static_cast<size_t>(samples), stream_);
+        }
+    }
+    else if (!wave && partials_.size() < needed)
     {
         partials_.allocate_async(needed, stream_);
     }
@@ -364,7 +374,6 @@ double session::launch(int64_t end)
     check(cudaMemsetAsync(counters_.data(), 0, sizeof(unsigned long long), stream_), "resetting the work counter");
     wave_buffers b{};
     const bool pool = wave && pool_;
-    const int64_t samples = static_cast<int64_t>(padded_pixels_) * (end - passes_);
     if (pool)
     {
         if (pool_samples_.size() < static_cast<size_t>(samples))
@@ -417,23 +426,21 @@ double session::launch(int64_t end)
     else
     {
         cudaEvent_t* m = timing_ ? marks(3) : nullptr;
+        launch_params_f64 p64{};
         if (f64_)
         {
-            launch_params_f64 p64{};
             p64.scene = *scene_->view_f64();
             p64.cam = cam_d_;
             p64.seed = p.seed;
             p64.pass_begin = p.pass_begin;
             p64.pass_end = p.pass_end;
-            p64.first_chunk = p.first_chunk;
+            p64.sample_count = samples;
             p64.chunk = p.chunk;
-            p64.chunks = p.chunks;
             p64.tiles_x = p.tiles_x;
             p64.padded_pixels = p.padded_pixels;
-            p64.total_items = p.total_items;
             p64.round_passes = p.round_passes;
             p64.work_counter = p.work_counter;
-            p64.partials = p.partials;
+            p64.samples = samples_f64_.data();
             p64.counters = p.counters;
             check(launch_render_f64(p64, grid_, stream_), "launching the FP64 render kernel");
         }
@@ -446,8 +453,9 @@ double session::launch(int64_t end)
             check(cudaEventRecord(m[2], stream_), "recording a CUDA event");
             reduce_marks = m + 2;
         }
-        check(launch_reduce(r, stream_), "launching the reduction");
-        last_kernel_launches_ = 2;
+        check(f64_ ? launch_reduce_f64(p64, sums_.data(), stream_) : launch_reduce(r, stream_),
+              "launching the reduction");
+        last_kernel_launches_ = f64_ ? 3 : 2;
     }
     if (timing_)
     {
