@@ -21,6 +21,10 @@ constexpr double max_launch_seconds = 0.5;              // renderer.h:413
 constexpr size_t partial_budget_bytes = size_t{1} << 30; // a launch's chunk partials: at most 1 GiB
 constexpr size_t wave_sample_budget_bytes = size_t{2} << 30; // a wavefront launch's samples (16 bytes each): 2 GiB
 constexpr double trial_samples = 32e6; // the autotuner's measured launch, by default
+// What a pool launch of an unknown view is taken to render a second, well under any scene's speed (0.5 to 7 G samples/s
+// measured): a first launch of that many samples fits launch_seconds, and a short render is one launch, not a chunk to
+// measure the speed and the rest (each launch ends with its last paths: 400x225 x 32 in 1.27 ms as two launches)
+constexpr double least_samples_per_second = 1e8;
 } // namespace
 
 session::session(std::shared_ptr<resident_scene> scene, const rt_session_options& options)
@@ -302,7 +306,10 @@ int64_t session::plan(int64_t target, double budget_seconds) const
 {
     const int64_t next_chunk = (passes_ / pass_chunk + 1) * pass_chunk;
     int64_t end;
-    if (samples_per_second_ <= 0)
+    const double speed = samples_per_second_ > 0         ? samples_per_second_
+                         : (pool_ || f64_) && !counting_ ? least_samples_per_second
+                                                         : 0.0;
+    if (speed <= 0)
     {
         end = next_chunk; // the probe: one chunk
     }
@@ -311,7 +318,7 @@ int64_t session::plan(int64_t target, double budget_seconds) const
         // As many whole chunks as fit the budget, at least one: a launch ends on a chunk boundary (or at the target),
         // so every chunk's partial is summed from the same samples in the same order however the launches fall
         const double pixels = static_cast<double>(camera_.image_width) * camera_.image_height;
-        const double passes = std::floor(budget_seconds * samples_per_second_ / pixels);
+        const double passes = std::floor(budget_seconds * speed / pixels);
         end = passes_ + static_cast<int64_t>(std::min(passes, 1e12));
         end = std::max(next_chunk, end / pass_chunk * pass_chunk);
     }
