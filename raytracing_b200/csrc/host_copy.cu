@@ -201,7 +201,7 @@ void pipeline(int64_t blocks, cudaStream_t stream, bool own_stream, const Launch
             take(block, stage[k].block);
         }
     };
-    the_helpers().run(static_cast<int>(std::min<int64_t>((blocks + 1) / 2, most_helpers + 1)), work);
+    the_helpers().run(static_cast<int>(std::min<int64_t>(blocks, most_helpers + 1)), work);
 }
 
 // out[i] = sums[i] * scale, into page-locked memory: as many 16-byte stores in flight as PCIe takes

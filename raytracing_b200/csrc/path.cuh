@@ -701,6 +701,122 @@ __device__ __forceinline__ bool traverse(const scene_view& S, float3 o, float3 d
     return hit.id >= 0;
 }
 
+// ---- the walk of the tree four wide ----------------------------------------------------------------------------
+// A ray as the wide nodes are tested: the direction's reciprocals, the origin times them, and where the near bounds of
+// an axis lie in a node (lo_x, hi_x, lo_y, ...: the low or the high row by the direction's sign; the far ones 16 bytes
+// off), instead of a minimum and a maximum of both: the same numbers, since a multiply-add is monotonic
+struct wide_ray
+{
+    float3 inv, os;
+    uint32_t x, y, z;
+};
+
+__device__ __forceinline__ wide_ray wide_ray_of(float3 o, float3 d)
+{
+    wide_ray r;
+    r.inv = make_float3(safe_inverse(d.x), safe_inverse(d.y), safe_inverse(d.z));
+    r.os = make_float3(o.x * r.inv.x, o.y * r.inv.y, o.z * r.inv.z);
+    r.x = r.inv.x < 0.0f ? 16u : 0u;
+    r.y = r.inv.y < 0.0f ? 48u : 32u;
+    r.z = r.inv.z < 0.0f ? 80u : 64u;
+    return r;
+}
+
+// One inner node: its children that the ray enters before `limit`, the nearest returned, the others pushed on the
+// stack, farthest deepest (pop() where it enters none)
+template <class Pop>
+__device__ __forceinline__ int wide_step(const bvh4_node* tree, int link, const wide_ray& r, float limit, int2* stack,
+                                         int& sp, const Pop& pop)
+{
+    const char* const node = reinterpret_cast<const char*>(tree + link);
+    const auto row = [&](uint32_t at) { return __ldg(reinterpret_cast<const float4*>(node + at)); };
+    const float4 nx = row(r.x), fx = row(r.x ^ 16u);
+    const float4 ny = row(r.y), fy = row(r.y ^ 16u);
+    const float4 nz = row(r.z), fz = row(r.z ^ 16u);
+    const int4 nl = __ldg(reinterpret_cast<const int4*>(tree[link].link));
+    // each child's entry distance, or infinity where the ray misses it (or the slot is unused)
+    const auto entry = [&](float ax, float bx, float ay, float by, float az, float bz, int child) -> float {
+        const float enter = fmaxf(fmaxf(fmaf(ax, r.inv.x, -r.os.x), fmaf(ay, r.inv.y, -r.os.y)),
+                                  fmaxf(fmaf(az, r.inv.z, -r.os.z), t_min));
+        const float exit = fminf(fminf(fmaf(bx, r.inv.x, -r.os.x), fmaf(by, r.inv.y, -r.os.y)),
+                                 fminf(fmaf(bz, r.inv.z, -r.os.z), limit));
+        return enter <= exit && child != traversal_done ? enter : infinity_f;
+    };
+    float k0 = entry(nx.x, fx.x, ny.x, fy.x, nz.x, fz.x, nl.x);
+    float k1 = entry(nx.y, fx.y, ny.y, fy.y, nz.y, fz.y, nl.y);
+    float k2 = entry(nx.z, fx.z, ny.z, fy.z, nz.z, fz.z, nl.z);
+    float k3 = entry(nx.w, fx.w, ny.w, fy.w, nz.w, fz.w, nl.w);
+    int l0 = nl.x, l1 = nl.y, l2 = nl.z, l3 = nl.w;
+    const auto order = [](float& ka, int& la, float& kb, int& lb) {
+        if (kb < ka)
+        {
+            const float k = ka;
+            ka = kb;
+            kb = k;
+            const int l = la;
+            la = lb;
+            lb = l;
+        }
+    };
+    order(k0, l0, k1, l1);
+    order(k2, l2, k3, l3);
+    order(k0, l0, k2, l2);
+    order(k1, l1, k3, l3);
+    order(k1, l1, k2, l2);
+    if (k0 == infinity_f)
+    {
+        return pop();
+    }
+    if (k3 != infinity_f)
+    {
+        stack[sp++] = make_int2(l3, __float_as_int(k3));
+    }
+    if (k2 != infinity_f)
+    {
+        stack[sp++] = make_int2(l2, __float_as_int(k2));
+    }
+    if (k1 != infinity_f)
+    {
+        stack[sp++] = make_int2(l1, __float_as_int(k1));
+    }
+    return l0;
+}
+
+// The closest hit of one ray per lane (a query of rays that do not follow from one another): the walk's inner nodes and
+// leaves by turns, each lane through the whole of its walk
+__device__ __forceinline__ void closest_hit_wide(const scene_view& S, float3 o, float3 d, hit_info& hit)
+{
+    hit = {-1, infinity_f, false};
+    const float inverse_a = 1.0f / length_squared(d);
+    const wide_ray ray = wide_ray_of(o, d);
+    int2 stack[wide_stack];
+    int sp = 0;
+    int link = 0;
+    const auto pop = [&]() -> int {
+        while (sp > 0)
+        {
+            const int2 e = stack[--sp];
+            if (__int_as_float(e.y) < hit.t)
+            {
+                return e.x;
+            }
+        }
+        return traversal_done;
+    };
+    while (link != traversal_done)
+    {
+        while (link >= 0)
+        {
+            link = wide_step(S.wide_nodes, link, ray, hit.t, stack, sp, pop);
+        }
+        if (link != traversal_done)
+        {
+            test_leaf<false, false, true>(S, link, o, d, 0.0f, inverse_a, -1, false, -1, hit, nullptr);
+            link = pop();
+        }
+    }
+}
+
 // ---- volumes of smoke (constant_medium.cuh:29-120, camera.cuh:259-284, shadow.cuh:129-165) -------------------------
 constexpr int block_media = 4; // max_media volumes: one number each from blocks 4-15 of a vertex
 

@@ -351,9 +351,7 @@ __global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURE
                 const scene_view& S = BATCH && slot >= 0 ? job_of(slot)->scene : (BATCH ? W.jobs[W.job_first].scene : P.scene);
                 const bvh4_node* const tree = S.wide_nodes;
                 float inverse_a = 0.0f;
-                float3 inv = o, os = o;
-                // where the near bounds of an axis lie in a node (lo_x, hi_x, lo_y, ...; the far ones 16 bytes off)
-                uint32_t near_x = 0, near_y = 32, near_z = 64;
+                wide_ray ray{};
                 if (slot >= 0)
                 {
                     const uint32_t meta = rec[record::meta][slot];
@@ -364,11 +362,7 @@ __global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURE
                     skip = QUALITY && shadow ? static_cast<int>(rec[record::skip][slot]) : -1;
                     inward = (meta & (QUALITY && shadow ? pool_shadow_inward : pool_inward)) != 0u;
                     inverse_a = 1.0f / (FEATURES ? length_squared<rounds::walk_features>(d) : length_squared(d));
-                    inv = make_float3(safe_inverse(d.x), safe_inverse(d.y), safe_inverse(d.z));
-                    os = make_float3(o.x * inv.x, o.y * inv.y, o.z * inv.z);
-                    near_x = inv.x < 0.0f ? 16u : 0u;
-                    near_y = inv.y < 0.0f ? 48u : 32u;
-                    near_z = inv.z < 0.0f ? 80u : 64u;
+                    ray = wide_ray_of(o, d);
                 }
                 const bool has_query = slot >= 0;
                 const auto pop = [&]() -> int {
@@ -396,66 +390,7 @@ __global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURE
                         }
                         if (descending)
                         {
-                            // The near and far bound of each axis by the sign of the ray's direction there, instead
-                            // of a minimum and a maximum of both: the same numbers (a multiply-add is monotonic)
-                            const char* const node = reinterpret_cast<const char*>(tree + link);
-                            const auto row = [&](uint32_t at) {
-                                return __ldg(reinterpret_cast<const float4*>(node + at));
-                            };
-                            const float4 lx = row(near_x), hx = row(near_x ^ 16u);
-                            const float4 ly = row(near_y), hy = row(near_y ^ 16u);
-                            const float4 lz = row(near_z), hz = row(near_z ^ 16u);
-                            const int4 nl = __ldg(reinterpret_cast<const int4*>(tree[link].link));
-                            const auto entry = [&](float lox, float hix, float loy, float hiy, float loz, float hiz,
-                                                   int child) -> float {
-                                const float a0 = fmaf(lox, inv.x, -os.x), a1 = fmaf(hix, inv.x, -os.x);
-                                const float b0 = fmaf(loy, inv.y, -os.y), b1 = fmaf(hiy, inv.y, -os.y);
-                                const float c0 = fmaf(loz, inv.z, -os.z), c1 = fmaf(hiz, inv.z, -os.z);
-                                const float enter = fmaxf(fmaxf(a0, b0), fmaxf(c0, t_min));
-                                const float exit = fminf(fminf(a1, b1), fminf(c1, hit.t));
-                                return enter <= exit && child != traversal_done ? enter : infinity_f;
-                            };
-                            float k0 = entry(lx.x, hx.x, ly.x, hy.x, lz.x, hz.x, nl.x);
-                            float k1 = entry(lx.y, hx.y, ly.y, hy.y, lz.y, hz.y, nl.y);
-                            float k2 = entry(lx.z, hx.z, ly.z, hy.z, lz.z, hz.z, nl.z);
-                            float k3 = entry(lx.w, hx.w, ly.w, hy.w, lz.w, hz.w, nl.w);
-                            int l0 = nl.x, l1 = nl.y, l2 = nl.z, l3 = nl.w;
-                            const auto order = [](float& ka, int& la, float& kb, int& lb) {
-                                if (kb < ka)
-                                {
-                                    const float k = ka;
-                                    ka = kb;
-                                    kb = k;
-                                    const int l = la;
-                                    la = lb;
-                                    lb = l;
-                                }
-                            };
-                            order(k0, l0, k1, l1);
-                            order(k2, l2, k3, l3);
-                            order(k0, l0, k2, l2);
-                            order(k1, l1, k3, l3);
-                            order(k1, l1, k2, l2);
-                            if (k0 == infinity_f)
-                            {
-                                link = pop();
-                            }
-                            else
-                            {
-                                if (k3 != infinity_f)
-                                {
-                                    stack[sp++] = make_int2(l3, __float_as_int(k3));
-                                }
-                                if (k2 != infinity_f)
-                                {
-                                    stack[sp++] = make_int2(l2, __float_as_int(k2));
-                                }
-                                if (k1 != infinity_f)
-                                {
-                                    stack[sp++] = make_int2(l1, __float_as_int(k1));
-                                }
-                                link = l0;
-                            }
+                            link = wide_step(tree, link, ray, hit.t, stack, sp, pop);
                             if (link < 0 && link != traversal_done && leaf == 0)
                             {
                                 leaf = link;

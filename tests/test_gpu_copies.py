@@ -62,3 +62,16 @@ def test_calls_from_several_threads(rt):
     for t in threads:
         t.join()
     assert not wrong
+
+
+@pytest.mark.parametrize("name,kw", [("weekend", {}), ("cover-2000", {}), ("final", {}), ("mesh-ggx", dict(mesh_level=4)),
+                                     ("glass", {})])
+def test_a_ray_alone_and_among_others(rt, name, kw):
+    # the four-wide walk's hits are checked against the oracle's in tests/test_gpu_render.py; a ray asked for alone
+    # gives what it gives among its neighbours, whose walks share its warp
+    scene = rt.Scene(rt.builtin_scene(name, width=64, height=36, **kw))
+    o, d = scene.camera_rays(7, 0)
+    ids, ts = scene.closest_hits(o, d)
+    for k in range(0, len(o), 97):
+        i, t = scene.closest_hits(o[k:k + 1], d[k:k + 1])
+        assert i[0] == ids[k] and t[0] == ts[k]
