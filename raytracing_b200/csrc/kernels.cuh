@@ -276,6 +276,7 @@ inline bool pool_suits(const scene_view& v, bool quality)
     return searched && v.prim_count == v.triangle_base && (wavefront_suits(v) || !quality);
 }
 using pool_function = void (*)(launch_params, pool_run, wave_batch);
+pool_function quality_pool_kernel(bool features, bool flat); // under NEE/MIS (pool_quality.cu)
 pool_function bare_pool_kernel(); // a scene that does not suit the wavefront (pool_bare.cu)
 // Claims, renders and writes out every sample of the launch (`grid` blocks fill the GPU; a small launch takes fewer)
 cudaError_t launch_pool(const launch_params& p, bool quality, float4* samples, int64_t sample_count, int grid,

@@ -2,7 +2,10 @@
 // walk, the materials, lights and camera, one vertex of a path under either integrator, and where a sample lies in a
 // launch. Included by each source that has kernels of its own, inside namespace rtb's anonymous namespace.
 //
-// The including source defines `struct rounds` first: how each dot product below is rounded (see `rounding`).
+// The including source names its table `rounds` first: how each dot product below is rounded (rounding.cuh). With
+// RTB_COMPACT_CODE defined, the random numbers and the large spheres' quadratic are called rather than inlined at each
+// use: the NEE/MIS kernels' code outgrows the instruction cache, and a warp shading its paths waits for its
+// instructions (measured in pool_quality.cu).
 #pragma once
 
 // ---- float3 arithmetic --------------------------------------------------------------------------------------
@@ -84,6 +87,13 @@ __device__ __forceinline__ void stratum_of(const camera_params& cam, int round_p
 // 24 random bits as a float in [0, 1 - 2^-24]: every value k / 2^24 exactly, as random_real<float> (random.cuh:79-93)
 __device__ __forceinline__ float to_unit(uint32_t x) { return static_cast<float>(x >> 8) * 0x1p-24f; }
 
+#ifdef RTB_COMPACT_CODE
+#define RTB_CALLED __device__ __noinline__
+#else
+#define RTB_CALLED __device__ __forceinline__
+#endif
+RTB_CALLED uint4 random_bits(uint4 counter, uint2 key) { return philox4x32_10(counter, key); }
+
 struct sampler
 {
     uint2 key;
@@ -94,7 +104,7 @@ struct sampler
     // Four 32-bit numbers for dimension block `block` of the vertex at depth `depth` (0: the camera ray)
     __device__ __forceinline__ uint4 draw_bits(int depth, int block) const
     {
-        return philox4x32_10(make_uint4(pixel, pass, (static_cast<uint32_t>(depth) << 4) | block, job), key);
+        return random_bits(make_uint4(pixel, pass, (static_cast<uint32_t>(depth) << 4) | block, job), key);
     }
 
     // The same as uniform floats
@@ -168,6 +178,28 @@ __device__ __forceinline__ float safe_inverse(float x)
     return 1.0f / (fabsf(x) > tiny ? x : copysignf(tiny, x));
 }
 
+// A large sphere's (negative radius): the same quadratic in FP64, where FP32's 24 bits cancel on its scale
+RTB_CALLED bool sphere_roots_double(float4 s, float3 o, float3 d, float& near, float& far)
+{
+    const double r = -static_cast<double>(s.w);
+    const double ox = static_cast<double>(s.x) - o.x;
+    const double oy = static_cast<double>(s.y) - o.y;
+    const double oz = static_cast<double>(s.z) - o.z;
+    const double dx = d.x, dy = d.y, dz = d.z;
+    const double ia = 1.0 / (dx * dx + dy * dy + dz * dz);
+    const double hoa = (dx * ox + dy * oy + dz * oz) * ia;
+    const double lx = ox - hoa * dx, ly = oy - hoa * dy, lz = oz - hoa * dz;
+    const double disc = fma(-lx, lx, fma(-ly, ly, fma(-lz, lz, r * r)));
+    if (disc < 0.0)
+    {
+        return false;
+    }
+    const double half_chord = sqrt(disc * ia);
+    near = static_cast<float>(hoa - half_chord);
+    far = static_cast<float>(hoa + half_chord);
+    return true;
+}
+
 // The two roots of the line with a sphere, as (h/a) -+ sqrt(r^2 - |l|^2)/sqrt(a) with l the vector from the line's
 // closest point to the center (sphere.cuh:70-97, after Haines et al., Ray Tracing Gems ch. 7): nothing larger than
 // r^2 is subtracted, and the three squares go into r^2 through fused multiply-adds.
@@ -188,24 +220,7 @@ __device__ __forceinline__ bool sphere_roots(float4 s, float3 o, float3 d, float
         far = h_over_a + half_chord;
         return true;
     }
-    // A large sphere (negative radius): the same quadratic in FP64, where FP32's 24 bits cancel on its scale
-    const double r = -static_cast<double>(s.w);
-    const double ox = static_cast<double>(s.x) - o.x;
-    const double oy = static_cast<double>(s.y) - o.y;
-    const double oz = static_cast<double>(s.z) - o.z;
-    const double dx = d.x, dy = d.y, dz = d.z;
-    const double ia = 1.0 / (dx * dx + dy * dy + dz * dz);
-    const double hoa = (dx * ox + dy * oy + dz * oz) * ia;
-    const double lx = ox - hoa * dx, ly = oy - hoa * dy, lz = oz - hoa * dz;
-    const double disc = fma(-lx, lx, fma(-ly, ly, fma(-lz, lz, r * r)));
-    if (disc < 0.0)
-    {
-        return false;
-    }
-    const double half_chord = sqrt(disc * ia);
-    near = static_cast<float>(hoa - half_chord);
-    far = static_cast<float>(hoa + half_chord);
-    return true;
+    return sphere_roots_double(s, o, d, near, far);
 }
 
 // hit_sphere (sphere.cuh:99-117): the nearest root in (t_min, t_max); far_only for the sphere the ray leaves inward

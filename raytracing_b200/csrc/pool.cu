@@ -20,10 +20,10 @@ using rounds = rounds_session;
 
 __global__ void pool_prepare_kernel(unsigned long long* work_counter) { *work_counter = 0ull; }
 
-template <bool QUALITY, bool FEATURES>
+template <bool FEATURES>
 pool_function pool_kernel_of(bool flat)
 {
-    return flat ? pool_kernel<QUALITY, FEATURES, true, false> : pool_kernel<QUALITY, FEATURES, false, false>;
+    return flat ? pool_kernel<false, FEATURES, true, false> : pool_kernel<false, FEATURES, false, false>;
 }
 
 pool_function pool_kernel_for(const scene_view& scene, bool quality)
@@ -35,9 +35,9 @@ pool_function pool_kernel_for(const scene_view& scene, bool quality)
     }
     if (quality)
     {
-        return has_features(scene) ? pool_kernel_of<true, true>(flat) : pool_kernel_of<true, false>(flat);
+        return quality_pool_kernel(has_features(scene), flat);
     }
-    return has_features(scene) ? pool_kernel_of<false, true>(flat) : pool_kernel_of<false, false>(flat);
+    return has_features(scene) ? pool_kernel_of<true>(flat) : pool_kernel_of<false>(flat);
 }
 } // namespace
 
