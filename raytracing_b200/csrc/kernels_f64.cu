@@ -476,7 +476,7 @@ __device__ bool medium_stretch(const scene_view_f64& S, const medium_d& m, v3 o,
 __device__ void media_event(const scene_view_f64& S, v3 o, v3 d, double time, const sampler& rng, int depth,
                             hit_info& hit)
 {
-    const double inverse_a = 1.0 / length_squared(d);
+    const double inverse_a = 1.0 / length_squared<rounding::y>(d);
     const v3 inv = make_double3(safe_inverse(d.x), safe_inverse(d.y), safe_inverse(d.z));
     const double length = sqrt(length_squared<rounding::y>(d));
     uniforms u{};

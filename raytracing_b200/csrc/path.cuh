@@ -178,6 +178,14 @@ __device__ __forceinline__ float safe_inverse(float x)
     return 1.0f / (fabsf(x) > tiny ? x : copysignf(tiny, x));
 }
 
+// A large sphere's dot products, written out where the others are (a last bit of a double moves the float distance it is
+// rounded to in one hit of some ten million)
+__device__ __forceinline__ double dot_double(double ax, double ay, double az, double bx, double by, double bz)
+{
+    return rounds::other == rounding::compiler ? ax * bx + ay * by + az * bz
+                                               : __fma_rn(az, bz, __fma_rn(ax, bx, __dmul_rn(ay, by)));
+}
+
 // A large sphere's (negative radius): the same quadratic in FP64, where FP32's 24 bits cancel on its scale
 RTB_CALLED bool sphere_roots_double(float4 s, float3 o, float3 d, float& near, float& far)
 {
@@ -186,8 +194,8 @@ RTB_CALLED bool sphere_roots_double(float4 s, float3 o, float3 d, float& near, f
     const double oy = static_cast<double>(s.y) - o.y;
     const double oz = static_cast<double>(s.z) - o.z;
     const double dx = d.x, dy = d.y, dz = d.z;
-    const double ia = 1.0 / (dx * dx + dy * dy + dz * dz);
-    const double hoa = (dx * ox + dy * oy + dz * oz) * ia;
+    const double ia = 1.0 / dot_double(dx, dy, dz, dx, dy, dz);
+    const double hoa = dot_double(dx, dy, dz, ox, oy, oz) * ia;
     const double lx = ox - hoa * dx, ly = oy - hoa * dy, lz = oz - hoa * dz;
     const double disc = fma(-lx, lx, fma(-ly, ly, fma(-lz, lz, r * r)));
     if (disc < 0.0)
@@ -195,8 +203,16 @@ RTB_CALLED bool sphere_roots_double(float4 s, float3 o, float3 d, float& near, f
         return false;
     }
     const double half_chord = sqrt(disc * ia);
-    near = static_cast<float>(hoa - half_chord);
-    far = static_cast<float>(hoa + half_chord);
+    if constexpr (rounds::other == rounding::compiler)
+    {
+        near = static_cast<float>(hoa - half_chord);
+        far = static_cast<float>(hoa + half_chord);
+    }
+    else
+    {
+        near = static_cast<float>(__dadd_rn(hoa, -half_chord));
+        far = static_cast<float>(__dadd_rn(hoa, half_chord));
+    }
     return true;
 }
 
@@ -216,8 +232,16 @@ __device__ __forceinline__ bool sphere_roots(float4 s, float3 o, float3 d, float
             return false;
         }
         const float half_chord = sqrtf(disc * inverse_a);
-        near = h_over_a - half_chord;
-        far = h_over_a + half_chord;
+        if constexpr (rounds::other == rounding::compiler)
+        {
+            near = h_over_a - half_chord;
+            far = h_over_a + half_chord;
+        }
+        else // not fused with h_over_a's product (a volume's boundary and its glass must meet at one distance)
+        {
+            near = __fadd_rn(h_over_a, -half_chord);
+            far = __fadd_rn(h_over_a, half_chord);
+        }
         return true;
     }
     return sphere_roots_double(s, o, d, near, far);
@@ -902,7 +926,7 @@ RTB_FEATURE_FUNCTION void media_event(const scene_view& S, float3 o, float3 d, f
                                       int depth,
                             hit_info& hit)
 {
-    const float inverse_a = 1.0f / length_squared(d);
+    const float inverse_a = 1.0f / length_squared<rounds::flight>(d);
     const float3 inv = make_float3(safe_inverse(d.x), safe_inverse(d.y), safe_inverse(d.z));
     const float3 os = make_float3(o.x * inv.x, o.y * inv.y, o.z * inv.z);
     const float length = sqrtf(length_squared<rounds::flight>(d));

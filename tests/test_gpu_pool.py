@@ -51,6 +51,12 @@ def test_pool_many_samples_and_launches(rt, name):
     _equal(rt, scene, 3, 48, launch_seconds=1e-4)
 
 
+@pytest.mark.parametrize("name,width,height,seed", [("perlin", 1000, 800, 11), ("final", 500, 500, 5)])
+def test_pool_equals_the_steps_in_rare_samples(rt, name, width, height, seed):
+    # a last bit in a large sphere's or a volume's distances changes one sample in tens of millions
+    _equal(rt, rt.Scene(rt.builtin_scene(name, width=width, height=height, spp=64)), seed, 64)
+
+
 def test_a_tuned_session_takes_the_steps(rt):
     scene = rt.Scene(rt.builtin_scene("weekend", width=64, spp=16))
     s = rt.Session(scene, seed=2)
