@@ -265,6 +265,12 @@ struct alignas(16) medium16
     int32_t pad[3];
 };
 
+// What shading a hit runs, by the primitive's material: a path that ends (a lamp; a miss too), a vertex that draws a
+// direction around the normal, or one that reflects or refracts
+constexpr uint8_t shade_ends = 0;
+constexpr uint8_t shade_diffuse = 1;
+constexpr uint8_t shade_specular = 2;
+
 // The resident scene as the kernels see it
 struct scene_view
 {
@@ -278,6 +284,7 @@ struct scene_view
     int32_t node_count;
     int32_t prim_count;
     const int32_t* prim_material; // by global id
+    const uint8_t* prim_class;    // by global id: what shading a hit on it runs (shade_ends ...), to shade like with like
     const material12* materials;
     const light24* lights;
     int32_t light_count;

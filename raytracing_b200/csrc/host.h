@@ -247,6 +247,7 @@ private:
     device_array<quad12> quads_;
     device_array<triangle12> triangles_;
     device_array<int32_t> prim_material_;
+    device_array<uint8_t> prim_class_;
     device_array<int32_t> prim_source_;
     device_array<material12> materials_;
     device_array<light24> lights_;

@@ -265,19 +265,40 @@ struct pool_run
     int32_t claim; // samples a warp claims at a time, 1..32
     int32_t pad0;
 };
-// Whether a session's AUTO renders a scene by the pool kernel: one searched flat, or through a tree four wide. Not one
-// with triangles: a large mesh's walks live on the L1 cache that the paths would take (the 1.3M-triangle mesh 2.7 G
-// segments/s by the wavefront's steps, 1.75 here); nor a bare small scene under NEE/MIS, nor an empty one. The bare small
-// scenes too, which lost 40% in the steps: quads 397x401 x 100 2.02 ms in the persistent kernel, 0.96 here; materials
-// 800x450 x 64 6.77 and 2.82.
+// Whether a session's AUTO renders a scene by the pool kernel: one searched flat, or through a tree four wide; nor a bare
+// small scene under NEE/MIS, nor an empty one. (The bare small scenes lost 40% in the wavefront's steps: quads 397x401 x
+// 100 2.02 ms in the persistent kernel, 0.96 here; materials 800x450 x 64 6.77 and 2.82.) With triangles, only under
+// NEE/MIS without the second book's features, the kernel whose image is checked against the steps'.
 inline bool pool_suits(const scene_view& v, bool quality)
 {
     const bool searched = v.node_count > 0 && (v.flat != 0 || v.wide_nodes != nullptr);
-    return searched && v.prim_count == v.triangle_base && (wavefront_suits(v) || !quality);
+    const bool triangles = v.prim_count > v.triangle_base;
+    return searched && (wavefront_suits(v) || !quality) && (!triangles || (quality && !has_features(v)));
+}
+// The launches it renders: all, but with triangles those of up to 2^20 samples per unit of depth, and with volumes beside
+// a tree 2^22. A mesh's shading (rough metal, coat, environment) waits for its instructions beside the walks', which the
+// steps' shade kernel does less; the steps wait at each depth for their last walks. The mesh of 1,280 triangles at depth 6
+// with 3.7M samples 2.42 ms here and 2.44 in the steps, with 14.7M 9.1 and 8.0, at depth 50 with 14.7M 11.2 and 16.2, with
+// 66M 38.8 and 36.9; that of 1.3M at depth 6 with 7.4M 6.1 and 6.9, with 29M 20.7 and 19.3, at depth 50 with 66M 50 and
+// 60. The second book's final scene at depth 2 with 1.4M 0.67 and 0.95, with 23M 9.3 and 8.9, at depth 50 with 23M 23.4
+// and 28.6.
+inline int64_t pool_most_samples(const scene_view& v, int max_depth)
+{
+    const int64_t depth = max_depth < 64 ? max_depth : 64;
+    const bool triangles = v.prim_count > v.triangle_base;
+    const bool volumes = v.medium_count > 0 && v.flat == 0;
+    return triangles ? depth << 20 : volumes ? depth << 22 : INT64_MAX;
 }
 using pool_function = void (*)(launch_params, pool_run, wave_batch);
-pool_function quality_pool_kernel(bool features, bool flat); // under NEE/MIS (pool_quality.cu)
-pool_function bare_pool_kernel(); // a scene that does not suit the wavefront (pool_bare.cu)
+struct pool_program
+{
+    pool_function kernel;
+    int shared; // dynamic shared memory, bytes a block
+};
+// The kernel's attributes; and its shared memory allowed on the current device, before its first launch there
+cudaError_t pool_program_attributes(const pool_program& program, kernel_attributes& out);
+pool_program quality_pool_program(bool features, bool flat, bool mesh); // under NEE/MIS (pool_quality.cu)
+pool_program bare_pool_program(); // a scene that does not suit the wavefront (pool_bare.cu)
 // Claims, renders and writes out every sample of the launch (`grid` blocks fill the GPU; a small launch takes fewer)
 cudaError_t launch_pool(const launch_params& p, bool quality, float4* samples, int64_t sample_count, int grid,
                         cudaStream_t stream);

@@ -20,24 +20,23 @@ using rounds = rounds_session;
 
 __global__ void pool_prepare_kernel(unsigned long long* work_counter) { *work_counter = 0ull; }
 
-template <bool FEATURES>
-pool_function pool_kernel_of(bool flat)
-{
-    return flat ? pool_kernel<false, FEATURES, true, false> : pool_kernel<false, FEATURES, false, false>;
-}
-
-pool_function pool_kernel_for(const scene_view& scene, bool quality)
+pool_program program_for(const scene_view& scene, bool quality)
 {
     const bool flat = scene.flat != 0;
+    const bool features = has_features(scene);
     if (!wavefront_suits(scene))
     {
-        return bare_pool_kernel();
+        return bare_pool_program();
     }
     if (quality)
     {
-        return quality_pool_kernel(has_features(scene), flat);
+        return quality_pool_program(features, flat, scene.prim_count > scene.triangle_base);
     }
-    return has_features(scene) ? pool_kernel_of<true>(flat) : pool_kernel_of<false>(flat);
+    if (flat)
+    {
+        return features ? pool_program_of<false, true, true, false>() : pool_program_of<false, false, true, false>();
+    }
+    return features ? pool_program_of<false, true, false, false>() : pool_program_of<false, false, false, false>();
 }
 } // namespace
 
@@ -45,6 +44,17 @@ cudaError_t prepare_pool(unsigned long long* work_counter, cudaStream_t stream)
 {
     pool_prepare_kernel<<<1, 1, 0, stream>>>(work_counter);
     return cudaGetLastError();
+}
+
+cudaError_t pool_program_attributes(const pool_program& program, kernel_attributes& out)
+{
+    const auto* const kernel = reinterpret_cast<const void*>(program.kernel);
+    if (const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, program.shared);
+        e != cudaSuccess)
+    {
+        return e;
+    }
+    return function_attributes(kernel, out, program.shared);
 }
 
 // A launch of fewer samples than lanes spreads them over the warps, so that every multiprocessor takes part
@@ -66,12 +76,14 @@ cudaError_t launch_pool(const launch_params& p, bool quality, float4* samples, i
     {
         return e;
     }
-    pool_kernel_for(p.scene, quality)<<<l.blocks, render_block, 0, stream>>>(p, run, wave_batch{});
+    const pool_program program = program_for(p.scene, quality);
+    program.kernel<<<l.blocks, render_block, static_cast<size_t>(program.shared), stream>>>(p, run, wave_batch{});
     return cudaGetLastError();
 }
 
 cudaError_t pool_attributes(const scene_view& scene, bool quality, kernel_attributes& out)
 {
-    return function_attributes(reinterpret_cast<const void*>(pool_kernel_for(scene, quality)), out);
+    const pool_program program = program_for(scene, quality);
+    return pool_program_attributes(program, out);
 }
 } // namespace rtb

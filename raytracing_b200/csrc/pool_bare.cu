@@ -19,5 +19,5 @@ using rounds = rounds_bare;
 #include "pool_kernel.cuh"
 } // namespace
 
-pool_function bare_pool_kernel() { return pool_kernel<false, false, true, false>; }
+pool_program bare_pool_program() { return pool_program_of<false, false, true, false>(); }
 } // namespace rtb

@@ -19,13 +19,13 @@ using rounds = rounds_session;
 #include "path.cuh"
 #include "pool_kernel.cuh"
 
-pool_function batch_kernel_of(bool flat, bool features)
+pool_program batch_program(bool flat, bool features)
 {
     if (flat)
     {
-        return features ? pool_kernel<false, true, true, true> : pool_kernel<false, false, true, true>;
+        return features ? pool_program_of<false, true, true, true>() : pool_program_of<false, false, true, true>();
     }
-    return features ? pool_kernel<false, true, false, true> : pool_kernel<false, false, false, true>;
+    return features ? pool_program_of<false, true, false, true>() : pool_program_of<false, false, false, true>();
 }
 } // namespace
 
@@ -38,12 +38,14 @@ cudaError_t launch_pool_batch(const wave_batch& w, bool flat, bool features, flo
     {
         return e;
     }
-    batch_kernel_of(flat, features)<<<l.blocks, render_block, 0, stream>>>(launch_params{}, run, w);
+    const pool_program program = batch_program(flat, features);
+    program.kernel<<<l.blocks, render_block, static_cast<size_t>(program.shared), stream>>>(launch_params{}, run, w);
     return cudaGetLastError();
 }
 
 cudaError_t pool_batch_attributes(bool flat, bool features, kernel_attributes& out)
 {
-    return function_attributes(reinterpret_cast<const void*>(batch_kernel_of(flat, features)), out);
+    const pool_program program = batch_program(flat, features);
+    return pool_program_attributes(program, out);
 }
 } // namespace rtb

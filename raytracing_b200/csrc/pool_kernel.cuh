@@ -11,17 +11,6 @@
 // cornell-mis x 64 30.0 -> 17.9, weekend 400x225 x 32 4.36 -> 1.27, one pass of weekend at 256x256 1.35 -> 0.25,
 // final 400x400 x 100 19.9 -> 17.0, smoke 300x300 x 64 5.8 -> 1.9, checker 400x225 x 64 4.9 -> 0.85.
 
-// The lanes still walking under which a warp stops its walks to give the others something to do
-#ifndef RTB_POOL_REFILL_LANES
-#define RTB_POOL_REFILL_LANES 20
-#endif
-
-// A warp's paths: twice its lanes, so that while up to 32 of them walk, enough others wait for a full warp's shading
-#ifndef RTB_POOL_PATHS
-#define RTB_POOL_PATHS 64
-#endif
-constexpr int pool_paths = RTB_POOL_PATHS;
-
 // A path's record in shared memory, as words of a structure of arrays ([word][path]): a warp's reads of a word touch
 // consecutive banks but for the paths' order
 template <bool QUALITY, bool FEATURES, bool BATCH>
@@ -55,62 +44,73 @@ constexpr uint32_t pool_shadow = 8u;        // a shadow ray is to be walked (bef
 constexpr uint32_t pool_shadow_inward = 16u;
 constexpr uint32_t pool_blocked = 32u;      // the shadow ray's answer, where the shading needs it (smoke)
 
-// The resident blocks per multiprocessor, which cap the registers: swept on the B200 from 4 to 10 (books tree 7 -> 8:
-// weekend 6.32 -> 6.18 ms; features 5 -> 6: final 11.25 -> 10.4; NEE/MIS flat 5 -> 6: cornell-mis 8.29 -> 7.95, where the
-// tree lost 8% and the features 11% of their time to spills; a batch of 16 cover jobs 20.7, 19.8, 19.0 and 19.7 ms at 5, 6,
-// 7 and 8). With the paths a warp keeps (48, 64, 80, 96: 64 within 1%
-// of the best on every scene, 96 -11% under NEE/MIS) they also set the shared memory, 17 to 31 KB a block.
-#ifndef RTB_POOL_BLOCKS_TREE
-#define RTB_POOL_BLOCKS_TREE 8
-#endif
-#ifndef RTB_POOL_BLOCKS_FLAT
-#define RTB_POOL_BLOCKS_FLAT 8
-#endif
-#ifndef RTB_POOL_BLOCKS_QUALITY
-#define RTB_POOL_BLOCKS_QUALITY 5
-#endif
-#ifndef RTB_POOL_BLOCKS_QUALITY_FLAT
-#define RTB_POOL_BLOCKS_QUALITY_FLAT 6
-#endif
-#ifndef RTB_POOL_BLOCKS_BATCH
-#define RTB_POOL_BLOCKS_BATCH 7
-#endif
-#ifndef RTB_POOL_BLOCKS_BATCH_FEATURES
-#define RTB_POOL_BLOCKS_BATCH_FEATURES 5
-#endif
-#ifndef RTB_POOL_BLOCKS_FEATURES
-#define RTB_POOL_BLOCKS_FEATURES 6
-#endif
-template <bool QUALITY, bool FEATURES, bool FLAT, bool BATCH>
-constexpr int pool_min_blocks()
+// A kernel's shape, swept on the B200 for each kind of scene: the resident blocks, which cap its registers; a warp's paths
+// (twice its lanes, so that while up to 32 of them walk, enough others wait for a full warp's shading); and the lists
+// its answered paths wait in, by what their shading runs (shade_ends ...), so that a warp shades like with like: three
+// lists want more paths, whose shared memory a flat scene can spare. GPU times of each rule's line:
+// * flat scenes {8 blocks, 64 paths, 1 list} -> {7, 96, 3}: glass 600x600 x 64 7.13 -> 6.19 ms; {8, 96, 3} 6.30, {6, 128,
+//   3} 6.57, {7, 96, 2} 6.91. With the second book's features {6, 64, 1} -> {6, 96, 3}: smoke 1.67 -> 1.57.
+// * bare flat scenes {8, 64, 1} -> {8, 96, 2}: quads 0.92 -> 0.87, materials 1.41 -> 1.34.
+// * the books' trees keep one list: three cost weekend 3.03 -> 3.14 and its 256x256 first frame 0.237 -> 0.277 (fewer
+//   lanes a phase); 8 blocks against 7: 6.32 -> 6.18; with the features 6 against 5: final 11.25 -> 10.4. A batch, whose
+//   jobs' scenes and cameras take registers: 7 (16 cover jobs 20.7, 19.8, 19.0, 19.7 ms at 5, 6, 7, 8).
+// * NEE/MIS one list too (cornell-mis 6.65; three 7.4): flat 6 blocks (5: +4%), trees and features 5 (6 spills: +8%).
+// * a mesh under NEE/MIS {5, 64, 1} -> {4, 96, 3, 12}: the 1.3M triangles at 1280x720 x 16 14.9 -> 10.8; {5, 80, 3} 11.3,
+//   {6, 64, 3} 11.5, {3, 128, 3} 12.2, {2, 192, 3} 14.9; walks broken off at 20 lanes 10.9.
+struct pool_shape
 {
+    int blocks;  // resident per multiprocessor
+    int paths;   // a warp's
+    int classes; // lists of answered paths
+    int refill;  // the lanes still walking under which a warp stops its walks to give the others something to do
+};
+
+template <bool QUALITY, bool FEATURES, bool FLAT, bool BATCH, bool MESH>
+RTB_HD constexpr pool_shape pool_shape_of()
+{
+    if (MESH)
+    {
+        return {4, 96, 3, 12};
+    }
     if (QUALITY)
     {
-        return FLAT && !FEATURES ? RTB_POOL_BLOCKS_QUALITY_FLAT : RTB_POOL_BLOCKS_QUALITY;
+        return {FLAT && !FEATURES ? 6 : 5, 64, 1, 20};
+    }
+    if (FLAT && !BATCH)
+    {
+        if (rounds::bare)
+        {
+            return {8, 96, 2, 20};
+        }
+        return {FEATURES ? 6 : 7, 96, 3, 20};
     }
     if (BATCH)
     {
-        return FEATURES ? RTB_POOL_BLOCKS_BATCH_FEATURES : RTB_POOL_BLOCKS_BATCH;
+        return {FEATURES ? 5 : 7, 64, 1, 20};
     }
-    return FEATURES ? RTB_POOL_BLOCKS_FEATURES : (FLAT ? RTB_POOL_BLOCKS_FLAT : RTB_POOL_BLOCKS_TREE);
+    return {FEATURES ? 6 : 8, 64, 1, 20};
 }
 
-template <bool QUALITY, bool FEATURES, bool FLAT, bool BATCH>
-__global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURES, FLAT, BATCH>())
+template <bool QUALITY, bool FEATURES, bool FLAT, bool BATCH, bool MESH = false>
+__global__ void __launch_bounds__(render_block, pool_shape_of<QUALITY, FEATURES, FLAT, BATCH, MESH>().blocks)
     pool_kernel(const __grid_constant__ launch_params P, const __grid_constant__ pool_run R,
                 const __grid_constant__ wave_batch W)
 {
     using record = pool_record<QUALITY, FEATURES, BATCH>;
+    constexpr int pool_paths = pool_shape_of<QUALITY, FEATURES, FLAT, BATCH, MESH>().paths;
+    constexpr int shade_classes = pool_shape_of<QUALITY, FEATURES, FLAT, BATCH, MESH>().classes;
+    constexpr int refill = pool_shape_of<QUALITY, FEATURES, FLAT, BATCH, MESH>().refill;
     constexpr int warps = render_block / 32;
-    __shared__ uint32_t records[warps][record::words][pool_paths];
-    __shared__ uint8_t lists[warps][3][pool_paths];
+    extern __shared__ uint32_t pool_memory[];
+    auto& records = *reinterpret_cast<uint32_t(*)[warps][record::words][pool_paths]>(pool_memory);
+    auto& lists = *reinterpret_cast<uint8_t(*)[warps][2 + shade_classes][pool_paths]>(pool_memory + warps * record::words * pool_paths);
     const unsigned lane = threadIdx.x & 31u;
     const unsigned lanes_below = (1u << lane) - 1u;
     const int warp = static_cast<int>(threadIdx.x >> 5);
     uint32_t(*const rec)[pool_paths] = records[warp];
     uint8_t* const walk_list = lists[warp][0];  // paths with a ray to walk
-    uint8_t* const shade_list = lists[warp][1]; // paths with an answer to shade
-    uint8_t* const free_list = lists[warp][2];  // records without a sample
+    uint8_t* const free_list = lists[warp][1];  // records without a sample
+    uint8_t* const shade_list = lists[warp][2]; // paths with an answer to shade, a list for each class of vertex
     const auto put3 = [&](int word, int p, float3 v) {
         rec[word][p] = __float_as_uint(v.x);
         rec[word + 1][p] = __float_as_uint(v.y);
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURE
         free_list[p] = static_cast<uint8_t>(p);
     }
     int walk_count = 0;
-    int shade_count = 0;
+    int shade_count[shade_classes] = {};
     int free_count = pool_paths;
     const auto limit = static_cast<unsigned long long>(R.sample_count);
     bool dry = limit == 0ull; // every sample of the launch is claimed
@@ -149,6 +149,37 @@ __global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURE
     int sp = 0;
     hit_info hit{-1, 0.0f, false};
     int2 stack[FLAT ? 1 : wide_stack];
+
+    // The lanes for which `which` holds append their path to its class's list
+    const auto to_shade_lists = [&](bool which, int shade_class, int p) {
+#pragma unroll
+        for (int c = 0; c < shade_classes; ++c)
+        {
+            shade_count[c] = push(shade_list + c * pool_paths, shade_count[c], which && shade_class == c, p);
+        }
+    };
+    const auto fullest = [&]() -> int {
+        int best = 0;
+#pragma unroll
+        for (int c = 1; c < shade_classes; ++c)
+        {
+            best = shade_count[c] > shade_count[best] ? c : best;
+        }
+        return best;
+    };
+    const auto waiting = [&]() -> int {
+        int n = 0;
+#pragma unroll
+        for (int c = 0; c < shade_classes; ++c)
+        {
+            n += shade_count[c];
+        }
+        return n;
+    };
+    const auto class_of = [&](const scene_view& S, int id) -> int {
+        const int c = id < 0 ? shade_ends : __ldg(S.prim_class + id);
+        return c < shade_classes ? c : shade_classes - 1;
+    };
 
     const auto job_of = [&](int p) -> const batch_job* { return BATCH ? W.jobs + rec[record::job][p] : nullptr; };
 
@@ -173,6 +204,7 @@ __global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURE
             const bool answered = slot >= 0 && link == traversal_done && leaf == 0;
             bool fresh = false;
             bool to_shade = false, to_free = false;
+            int shade_class = 0;
             const int was = slot;
             if (answered)
             {
@@ -218,10 +250,11 @@ __global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURE
                     rec[record::hit][slot] = hit.id < 0 ? 0xffffffffu
                                                         : (static_cast<uint32_t>(hit.id) << 1) | (hit.front ? 1u : 0u);
                     to_shade = true;
+                    shade_class = class_of(BATCH ? job_of(slot)->scene : P.scene, hit.id);
                     slot = -1;
                 }
             }
-            shade_count = push(shade_list, shade_count, to_shade, was);
+            to_shade_lists(to_shade, shade_class, was);
             if (QUALITY && !FEATURES)
             {
                 free_count = push(free_list, free_count, to_free, was);
@@ -249,10 +282,10 @@ __global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURE
             const int walking = __popc(__ballot_sync(full_warp, slot >= 0));
             const int startable = dry ? 0 : free_count;
             // Few walks left and no ray to refill the lanes with: shade or start, whichever has the fuller warp
-            const bool few = walking < RTB_POOL_REFILL_LANES && walking * 8 < (walking + shade_count + startable) * 5;
+            const bool few = walking < refill && walking * 8 < (walking + waiting() + startable) * 5;
             if (walk_count == 0 && few)
             {
-                next = startable > shade_count ? phase::start : phase::shade;
+                next = startable > shade_count[fullest()] ? phase::start : phase::shade;
             }
             else
             {
@@ -262,13 +295,14 @@ __global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURE
         else
         {
             const int startable = dry ? 0 : free_count;
-            if (walk_count >= 32 || (walk_count >= startable && walk_count >= shade_count))
+            const int shadeable = shade_count[fullest()];
+            if (walk_count >= 32 || (walk_count >= startable && walk_count >= shadeable))
             {
                 next = walk_count > 0 ? phase::walk : phase::end;
             }
             else
             {
-                next = startable > shade_count ? phase::start : phase::shade;
+                next = startable > shadeable ? phase::start : phase::shade;
             }
         }
         if (next == phase::end)
@@ -284,6 +318,7 @@ __global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURE
                 const int p = mine ? walk_list[walk_count - taken + static_cast<int>(lane)] : 0;
                 walk_count -= taken;
                 bool to_shade = false, to_free = false;
+                int shade_class = 0;
                 if (mine)
                 {
                     const batch_job* J = job_of(p);
@@ -311,6 +346,7 @@ __global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURE
                             rec[record::hit_t][p] = __float_as_uint(h.t);
                             rec[record::hit][p] = h.id < 0 ? 0xffffffffu
                                                            : (static_cast<uint32_t>(h.id) << 1) | (h.front ? 1u : 0u);
+                            shade_class = class_of(S, h.id);
                         }
                         else if (FEATURES)
                         {
@@ -339,7 +375,7 @@ __global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURE
                         }
                     }
                 }
-                shade_count = push(shade_list, shade_count, to_shade, p);
+                to_shade_lists(to_shade, shade_class, p);
                 if (QUALITY && !FEATURES)
                 {
                     free_count = push(free_list, free_count, to_free, p);
@@ -376,9 +412,9 @@ __global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURE
                     }
                     return traversal_done;
                 };
-                const int total = __popc(__ballot_sync(full_warp, has_query)) + walk_count + shade_count +
+                const int total = __popc(__ballot_sync(full_warp, has_query)) + walk_count + waiting() +
                                   (dry ? 0 : free_count);
-                const int enough = min(RTB_POOL_REFILL_LANES, (total * 5 + 7) / 8);
+                const int enough = min(refill, (total * 5 + 7) / 8);
                 while (true)
                 {
                     while (true)
@@ -522,10 +558,15 @@ __global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURE
             continue;
         }
         // The shading of the answered paths, as the wavefront's shade kernel does it
-        const int taken = min(32, shade_count);
+        const int which = fullest();
+        const int taken = min(32, shade_count[which]);
         const bool mine = static_cast<int>(lane) < taken;
-        const int p = mine ? shade_list[shade_count - taken + static_cast<int>(lane)] : 0;
-        shade_count -= taken;
+        const int p = mine ? shade_list[which * pool_paths + shade_count[which] - taken + static_cast<int>(lane)] : 0;
+#pragma unroll
+        for (int c = 0; c < shade_classes; ++c)
+        {
+            shade_count[c] -= c == which ? taken : 0;
+        }
         bool goes_on = false;
         bool lit = false;
         int job = 0;
@@ -673,4 +714,19 @@ __global__ void __launch_bounds__(render_block, pool_min_blocks<QUALITY, FEATURE
             }
         }
     }
+}
+
+// The kernel's shared memory
+template <bool QUALITY, bool FEATURES, bool FLAT, bool BATCH, bool MESH = false>
+constexpr int pool_shared_bytes()
+{
+    constexpr pool_shape shape = pool_shape_of<QUALITY, FEATURES, FLAT, BATCH, MESH>();
+    return render_block / 32 * shape.paths *
+           (static_cast<int>(sizeof(uint32_t)) * pool_record<QUALITY, FEATURES, BATCH>::words + 2 + shape.classes);
+}
+
+template <bool QUALITY, bool FEATURES, bool FLAT, bool BATCH, bool MESH = false>
+pool_program pool_program_of()
+{
+    return {pool_kernel<QUALITY, FEATURES, FLAT, BATCH, MESH>, pool_shared_bytes<QUALITY, FEATURES, FLAT, BATCH, MESH>()};
 }

@@ -23,12 +23,16 @@ using rounds = rounds_session;
 #include "pool_kernel.cuh"
 } // namespace
 
-pool_function quality_pool_kernel(bool features, bool flat)
+pool_program quality_pool_program(bool features, bool flat, bool mesh)
 {
     if (features)
     {
-        return flat ? pool_kernel<true, true, true, false> : pool_kernel<true, true, false, false>;
+        return flat ? pool_program_of<true, true, true, false>() : pool_program_of<true, true, false, false>();
     }
-    return flat ? pool_kernel<true, false, true, false> : pool_kernel<true, false, false, false>;
+    if (flat)
+    {
+        return pool_program_of<true, false, true, false>();
+    }
+    return mesh ? pool_program_of<true, false, false, false, true>() : pool_program_of<true, false, false, false>();
 }
 } // namespace rtb

@@ -1020,6 +1020,19 @@ resident_scene::resident_scene(const rt_scene_desc& d)
     tables.add(boundary_quads_, boundary_quads);
     tables.add(quads_, quads);
     tables.add(triangles_, triangles);
+    // (a glossy coat beside the rough conductors, which share a sampler: apart from them, like the mirrors and glass)
+    std::vector<uint8_t> material_class(materials.size());
+    for (size_t i = 0; i < materials.size(); ++i)
+    {
+        const material12& m = materials[i];
+        const bool around_normal = m.lobe == RT_MICROFACET_CONDUCTOR ||
+                                   (m.lobe != RT_MICROFACET_GLOSS && (m.kind == RT_LAMBERTIAN || m.kind == RT_ISOTROPIC));
+        material_class[i] = m.kind == RT_DIFFUSE_LIGHT ? shade_ends : (around_normal ? shade_diffuse : shade_specular);
+    }
+    std::vector<uint8_t> prim_class(prim_material.size());
+    std::transform(prim_material.begin(), prim_material.end(), prim_class.begin(),
+                   [&](int32_t m) { return material_class[static_cast<size_t>(m)]; });
+    tables.add(prim_class_, prim_class);
     tables.add(prim_material_, prim_material);
     tables.add(prim_source_, prim_source);
     tables.add(materials_, materials);
@@ -1038,6 +1051,7 @@ resident_scene::resident_scene(const rt_scene_desc& d)
     view_.node_count = static_cast<int32_t>(tree.nodes.size());
     view_.prim_count = S + Q + T;
     view_.prim_material = prim_material_.data();
+    view_.prim_class = prim_class_.data();
     view_.materials = materials_.data();
     view_.lights = lights_.data();
     view_.light_count = static_cast<int32_t>(lights.size());
@@ -1279,7 +1293,7 @@ resident_scene::resident_scene(const rt_scene_desc& d)
     stats_.lamps = static_cast<int64_t>(lamps.size());
     stats_.lights = static_cast<int64_t>(lights.size());
     stats_.device_bytes = static_cast<int64_t>(nodes_.bytes() + spheres_.bytes() + quads_.bytes() + triangles_.bytes() +
-                                               prim_material_.bytes() + prim_source_.bytes() + materials_.bytes() +
+                                               prim_material_.bytes() + prim_class_.bytes() + prim_source_.bytes() + materials_.bytes() +
                                                lights_.bytes() + lamps_.bytes() + lamp_of_.bytes() +
                                                env_texels_.bytes() + env_bins_.bytes() + env_row_cos_.bytes() +
                                                sphere_motion_.bytes() + sphere_frames_.bytes() + textures_.bytes() +

@@ -15,6 +15,7 @@ enum class rounding
 // The kernels of kernels.cu: left to the compiler
 struct rounds_compiler
 {
+    static constexpr bool bare = false;
     static constexpr rounding other = rounding::compiler;
     static constexpr rounding sky = rounding::compiler;
     static constexpr rounding flight = rounding::compiler;
@@ -40,6 +41,7 @@ struct rounds_compiler
 // bit. The kernels that render a session's samples in another form take this table, so the form changes no image.
 struct rounds_session
 {
+    static constexpr bool bare = false; // whether these kernels render the bare small scenes only
     static constexpr rounding other = rounding::x;
     static constexpr rounding sky = rounding::y;
     static constexpr rounding flight = rounding::y;
@@ -63,6 +65,7 @@ struct rounds_session
 // The persistent kernel's flat search, which renders the bare small scenes: the same but for the ray's squared length
 struct rounds_bare : rounds_session
 {
+    static constexpr bool bare = true;
     static constexpr rounding walk_flat = rounding::y;
 };
 } // namespace rtb

@@ -380,7 +380,7 @@ double session::launch(int64_t end)
 
     check(cudaMemsetAsync(counters_.data(), 0, sizeof(unsigned long long), stream_), "resetting the work counter");
     wave_buffers b{};
-    const bool pool = wave && pool_;
+    const bool pool = wave && pool_ && samples <= pool_most_samples(scene_->view(), camera_.max_depth);
     if (pool)
     {
         if (pool_samples_.size() < static_cast<size_t>(samples))

@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
 
 SCENES = [("weekend", {}), ("weekend", dict(combination="mis")), ("glass", {}), ("glass", dict(sampling="lights")),
           ("cornell-mis", {}), ("final", {}), ("bouncing", {}), ("smoke", {}), ("smoke", dict(combination="mis")),
-          ("perlin", {}), ("light", dict(combination="mis")), ("ggx-furnace", {})]
+          ("perlin", {}), ("light", dict(combination="mis")), ("ggx-furnace", {}),
+          ("mesh-ggx", dict(mesh_level=3, env_width=64)), ("mesh-ggx", dict(mesh_level=6, env_width=64))]
 SIZES = [(1, 1, 1, 0), (3, 5, 2, 0), (37, 21, 19, 0), (130, 67, 33, 0), (64, 64, 16, 1), (64, 64, 16, 2)]
 
 
@@ -30,7 +31,7 @@ def _equal(rt, scene, seed, passes, form="wavefront", **kw):
     assert (ca["rays"], ca["shadow_rays"]) == (cb["rays"], cb["shadow_rays"])
 
 
-@pytest.mark.parametrize("name,kw", SCENES, ids=[f"{n}-{'-'.join(k.values())}" for n, k in SCENES])
+@pytest.mark.parametrize("name,kw", SCENES, ids=[f"{n}-{'-'.join(str(v) for v in k.values())}" for n, k in SCENES])
 def test_pool_equals_the_wavefronts_steps(rt, name, kw):
     for width, height, passes, depth in SIZES:
         scene = rt.Scene(rt.builtin_scene(name, width=width, height=height, spp=passes, depth=depth, **kw))
@@ -51,10 +52,22 @@ def test_pool_many_samples_and_launches(rt, name):
     _equal(rt, scene, 3, 48, launch_seconds=1e-4)
 
 
-@pytest.mark.parametrize("name,width,height,seed", [("perlin", 1000, 800, 11), ("final", 500, 500, 5)])
+@pytest.mark.parametrize("name,width,height,seed", [("perlin", 1000, 800, 5), ("final", 500, 500, 5)])
 def test_pool_equals_the_steps_in_rare_samples(rt, name, width, height, seed):
     # a last bit in a large sphere's or a volume's distances changes one sample in tens of millions
     _equal(rt, rt.Scene(rt.builtin_scene(name, width=width, height=height, spp=64)), seed, 64)
+
+
+@pytest.mark.parametrize("name,kw", [("mesh-ggx", dict(depth=8, mesh_level=4, env_width=64)), ("final", dict(depth=2))])
+def test_forms_by_a_launchs_size(rt, name, kw):
+    # a first launch of 7.7M samples by the pool kernel, the rest of 23M by the steps: one image
+    scene = rt.Scene(rt.builtin_scene(name, width=800, height=600, spp=64, **kw))
+    a = rt.Session(scene, seed=8, launch_seconds=0.5)
+    assert a.render_to(16)["kernel_launches"] == 3
+    assert a.render_to(64)["kernel_launches"] > 3
+    b = rt.Session(scene, seed=8, form="wavefront")
+    b.render_to(64)
+    assert np.array_equal(a.pixels(), b.pixels())
 
 
 def test_a_tuned_session_takes_the_steps(rt):
