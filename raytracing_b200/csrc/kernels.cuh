@@ -221,6 +221,10 @@ struct wave_buffers
 size_t wave_slot_bytes();
 // Every slot without a sample (its flags row zeroed), before a launch's first step
 cudaError_t clear_wave_slots(const wave_buffers& b, cudaStream_t stream);
+using wave_shade_function = void (*)(launch_params, wave_buffers, wave_batch);
+// A session's shade kernel under NEE/MIS without the second book's features (wave_quality.cu)
+wave_shade_function quality_shade_kernel();
+
 // How a session's wavefront step is launched (the autotuner's choice): the trace kernel's grid and register cap (its
 // minimum resident blocks per multiprocessor: RTB_TRACE_MIN_BLOCKS or wave_trace_roomy_blocks), the shade kernel's
 // block size (64 or 128 threads)
