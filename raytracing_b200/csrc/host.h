@@ -443,7 +443,7 @@ private:
     rt_camera_desc camera_{};
     camera_params cam_{};
     camera_d cam_d_{};  // the same view in double, for an FP64 session
-    bool f64_ = false;  // RT_FLOAT64: the books' integrator in double, persistent form
+    bool f64_ = false;  // RT_FLOAT64: the books' integrator in double, by its pool kernel
     cudaStream_t stream_ = nullptr;
     cudaEvent_t start_ = nullptr;
     cudaEvent_t stop_ = nullptr;
@@ -460,10 +460,10 @@ private:
     int padded_pixels_ = 0;
     int64_t max_partial_entries_ = 0;
 
-    // The wavefront form (RT_FORM_WAVEFRONT, or AUTO on a tree-searched scene)
+    // The wavefront form (RT_FORM_WAVEFRONT, or AUTO where wavefront_suits): its steps, or AUTO's pool kernel
     bool wavefront_ = false;
     std::unique_ptr<wave_runner> wave_;
-    bool pool_ = false;                 // AUTO's wavefront: the pool kernel
+    bool pool_ = false;                 // AUTO: the pool kernel, for launches of up to pool_most_samples
     int pool_grid_ = 0;
     device_array<float4> pool_samples_; // a pool launch's samples, kept for the next
     device_array<double> samples_f64_;  // the same of an FP64 session

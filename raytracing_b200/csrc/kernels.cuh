@@ -82,12 +82,12 @@ struct alignas(16) batch_job
 // its kernels are compiled with their code, the others without
 inline bool has_features(const scene_view& s) { return s.has_motion != 0 || s.has_textures != 0 || s.medium_count > 0; }
 
-// Whether a scene renders in the wavefront form unless a form is asked for: every tree-searched scene (its walks
-// diverge: the mesh 3.2 times and the sphere scenes 1.2-2 times as fast as in the persistent kernel) and a
-// flat-searched scene whose shading is heavy (lights or lamps, the second book's features, an environment: the glass
-// Cornell box 10-16% faster, the marble spheres 55%); the bare small flat scenes (five spheres or five quads under
-// the sky), whose paths are one or two cheap segments that cannot pay for the slots' traffic, stay in the persistent
-// kernel (40% slower in the wavefront).
+// Whether the wavefront's steps render a scene faster than the persistent kernel (a session's AUTO takes the pool kernel
+// before either, pool_suits): every tree-searched scene (its walks diverge: the mesh 3.2 times and the sphere scenes
+// 1.2-2 times as fast) and a flat-searched scene whose shading is heavy (lights or lamps, the second book's features, an
+// environment: the glass Cornell box 10-16% faster, the marble spheres 55%); not the bare small flat scenes (five spheres
+// or five quads under the sky), whose paths are one or two cheap segments that cannot pay for the slots' traffic (40%
+// slower).
 inline bool wavefront_suits(const scene_view& v)
 {
     const bool heavy = v.light_count > 0 || v.lamp_count > 0 || has_features(v) || v.has_environment;
@@ -95,9 +95,10 @@ inline bool wavefront_suits(const scene_view& v)
 }
 
 // The jobs come in twelve groups: the scenes of each search (flat, tree) without and with the second book's features,
-// in each form: the persistent kernel, the wavefront's steps, and the pool kernel (pool_batch_group: books' jobs). The first four are rendered each by its own launch of the persistent kernel compiled for it
-// (batch_group), the other four each by its own run of the wavefront's steps (wave_batch_group); a scene takes the
-// form wavefront_suits gives it, as a session's render of it does.
+// in each form. Four are rendered each by its own launch of the persistent kernel compiled for it (batch_group), four
+// each by its own run of the wavefront's steps (wave_batch_group), as wavefront_suits says; and four by the pool kernel
+// (pool_batch_group: the books' jobs of tree-searched scenes, and in the continuous server's refinement, whose images
+// follow a session's roundings, of flat ones).
 constexpr int persistent_groups = 4;
 constexpr int batch_groups = 12;
 RTB_HD constexpr int batch_group(bool flat, bool features) { return (flat ? 0 : 2) + (features ? 1 : 0); }

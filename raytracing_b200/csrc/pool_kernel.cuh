@@ -1,14 +1,14 @@
 // The pool kernel: the wavefront within a warp. Included after path.cuh by each source that compiles it.
 //
-// A persistent warp keeps 64 paths in shared memory and, in turn, walks rays (32 lanes, each with a path of its own),
+// A persistent warp keeps 64 or 96 paths in shared memory and, in turn, walks rays (32 lanes, each with a path of its own),
 // shades answered paths and starts new samples, each phase with as full a warp as the lists hold; a path is never bound
 // to a lane between phases. What it replaces: the wavefront's steps keep up to 3 x 2^20 paths in HBM and run two kernels
 // a step over all of them, so every segment paid 160 to 224 bytes of HBM traffic and a round through a queue, and every
 // launch ended with a drain of a path's length of nearly empty steps (a 400x225, 32-pass cover render spent 4.4 ms in
 // 128 steps for 1.3 ms of work). Against the one-lane-one-path persistent kernel, shading and searches run with full
 // warps. Bound by instruction issue, with the lanes that materials and walks of uneven depth leave idle.
-// Measured on the B200, GPU time, against the steps (images equal bit for bit): glass 600x600 x 256 47.0 -> 28.1 ms,
-// cornell-mis x 64 30.0 -> 17.9, weekend 400x225 x 32 4.36 -> 1.27, one pass of weekend at 256x256 1.35 -> 0.25,
+// Measured on the B200, GPU time, against the steps (images equal bit for bit): glass 600x600 x 1024 173 -> 96 ms,
+// cornell-mis x 256 109 -> 58, weekend 400x225 x 32 4.36 -> 1.27, one pass of weekend at 256x256 1.35 -> 0.25,
 // final 400x400 x 100 19.9 -> 17.0, smoke 300x300 x 64 5.8 -> 1.9, checker 400x225 x 64 4.9 -> 0.85.
 
 // A path's record in shared memory, as words of a structure of arrays ([word][path]): a warp's reads of a word touch
