@@ -294,6 +294,11 @@ inline int64_t pool_most_samples(const scene_view& v, int max_depth)
     const bool volumes = v.medium_count > 0 && v.flat == 0;
     return triangles ? depth << 20 : volumes ? depth << 22 : INT64_MAX;
 }
+// A bare small scene's single pass of up to this many samples is the persistent kernel's: each of its lanes takes one
+// sample, and there is no samples buffer to reduce (quads 64x64 35 us there and 39 here, 236x650 50 and 56, materials
+// 64x64 80 and 87; above, and with more passes, which a lane takes in turn, the pool kernel: quads 1280x720 96 and 95,
+// two passes of materials 811x274 208 and 167)
+constexpr int64_t pool_least_bare_samples = int64_t{1} << 18;
 using pool_function = void (*)(launch_params, pool_run, wave_batch);
 struct pool_program
 {

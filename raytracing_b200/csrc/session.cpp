@@ -337,8 +337,10 @@ double session::launch(int64_t end)
 {
     const int64_t first_chunk = passes_ / pass_chunk;
     const int64_t chunks = (end + pass_chunk - 1) / pass_chunk - first_chunk;
-    const bool wave = (wavefront_ || pool_) && !counting_;
     const int64_t samples = static_cast<int64_t>(padded_pixels_) * (end - passes_);
+    const bool pool = pool_ && !counting_ && samples <= pool_most_samples(scene_->view(), camera_.max_depth) &&
+                      (wavefront_ || end - passes_ > 1 || samples > pool_least_bare_samples);
+    const bool wave = pool || (wavefront_ && !counting_);
     const size_t needed = static_cast<size_t>(chunks) * static_cast<size_t>(padded_pixels_) * 3;
     if (f64_)
     {
@@ -380,7 +382,6 @@ double session::launch(int64_t end)
 
     check(cudaMemsetAsync(counters_.data(), 0, sizeof(unsigned long long), stream_), "resetting the work counter");
     wave_buffers b{};
-    const bool pool = wave && pool_ && samples <= pool_most_samples(scene_->view(), camera_.max_depth);
     if (pool)
     {
         if (pool_samples_.size() < static_cast<size_t>(samples))

@@ -70,6 +70,20 @@ def test_forms_by_a_launchs_size(rt, name, kw):
     assert np.array_equal(a.pixels(), b.pixels())
 
 
+@pytest.mark.parametrize("name", ["quads", "materials"])
+@pytest.mark.parametrize("width,height", [(1, 1), (37, 21), (512, 512), (520, 512)])
+def test_a_bare_scenes_single_passes(rt, name, width, height):
+    # one pass (by the persistent kernel up to 2^18 samples), then the rest of a chunk and more: one image
+    scene = rt.Scene(rt.builtin_scene(name, width=width, height=height, spp=36))
+    a = rt.Session(scene, seed=4)
+    b = rt.Session(scene, seed=4, form="persistent")
+    for passes in (1, 2, 20, 36):
+        a.render_to(passes)
+        b.render_to(passes)
+        assert np.array_equal(a.pixels(), b.pixels())
+    assert a.counters()["rays"] == b.counters()["rays"]
+
+
 def test_a_tuned_session_takes_the_steps(rt):
     scene = rt.Scene(rt.builtin_scene("weekend", width=64, spp=16))
     s = rt.Session(scene, seed=2)
