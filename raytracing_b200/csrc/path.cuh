@@ -821,13 +821,29 @@ __device__ __forceinline__ int wide_step(const bvh4_node* tree, int link, const 
     return l0;
 }
 
+// The closest hit as the walk of the binary tree meets it, called: a query's rare second walk
+__device__ __noinline__ void closest_hit_binary(const scene_view& S, float3 o, float3 d, hit_info& hit)
+{
+    traverse<false, false, search_tree>(S, o, d, 0.0f, infinity_f, -1, false, -1, hit);
+}
+
 // The closest hit of one ray per lane (a query of rays that do not follow from one another): the walk's inner nodes and
-// leaves by turns, each lane through the whole of its walk
+// leaves by turns, each lane through the whole of its walk. Which of several primitives at one distance (two quads in a
+// plane, a mesh's shared edge, a sphere twice in the scene) is the hit follows from the order of the walk, and the order
+// of a query's is the binary tree's: a ray that meets a second primitive as near as the nearest to within the boxes' and
+// the distances' rounding walks that tree. (The nodes' entries are off by some 2^-24 of the origin times the direction's
+// reciprocal; an axis the ray hardly moves along decides no entry near a hit.)
 __device__ __forceinline__ void closest_hit_wide(const scene_view& S, float3 o, float3 d, hit_info& hit)
 {
     hit = {-1, infinity_f, false};
     const float inverse_a = 1.0f / length_squared(d);
     const wide_ray ray = wide_ray_of(o, d);
+    const float steepest = fminf(fminf(fabsf(ray.inv.x), fabsf(ray.inv.y)), fabsf(ray.inv.z));
+    const auto reach = [&](float inv, float os) { return fabsf(inv) <= 1024.0f * steepest ? fabsf(os) : 0.0f; };
+    const float origin = fmaxf(fmaxf(reach(ray.inv.x, ray.os.x), reach(ray.inv.y, ray.os.y)), reach(ray.inv.z, ray.os.z));
+    float as_near = 0.0f; // what lies within this of the closest hit may be as near
+    float bound = infinity_f;
+    bool tied = false;
     int2 stack[wide_stack];
     int sp = 0;
     int link = 0;
@@ -835,7 +851,7 @@ __device__ __forceinline__ void closest_hit_wide(const scene_view& S, float3 o, 
         while (sp > 0)
         {
             const int2 e = stack[--sp];
-            if (__int_as_float(e.y) < hit.t)
+            if (__int_as_float(e.y) < bound)
             {
                 return e.x;
             }
@@ -846,13 +862,29 @@ __device__ __forceinline__ void closest_hit_wide(const scene_view& S, float3 o, 
     {
         while (link >= 0)
         {
-            link = wide_step(S.wide_nodes, link, ray, hit.t, stack, sp, pop);
+            link = wide_step(S.wide_nodes, link, ray, bound, stack, sp, pop);
         }
         if (link != traversal_done)
         {
-            test_leaf<false, false, true>(S, link, o, d, 0.0f, inverse_a, -1, false, -1, hit, nullptr);
+            // the leaf's own closest hit (its primitives are tested in one order by either walk)
+            hit_info found{-1, bound, false};
+            test_leaf<false, false, true>(S, link, o, d, 0.0f, inverse_a, -1, false, -1, found, nullptr);
+            if (found.id >= 0)
+            {
+                tied = hit.id >= 0 && found.t >= hit.t - as_near;
+                if (hit.id < 0 || found.t < hit.t)
+                {
+                    hit = found;
+                    as_near = 0x1p-18f * (hit.t + origin);
+                    bound = hit.t + as_near;
+                }
+            }
             link = pop();
         }
+    }
+    if (tied)
+    {
+        closest_hit_binary(S, o, d, hit);
     }
 }
 
