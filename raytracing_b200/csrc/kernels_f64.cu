@@ -227,7 +227,7 @@ __device__ __forceinline__ bool hit_quad(const quad_v& s, v3 o, v3 d, double lo,
         return false;
     }
     const v3 origin_to_q = s.q - o;
-    t = dot(s.n, origin_to_q) / denominator;
+    t = dot<rounding::y>(s.n, origin_to_q) / denominator;
     if (!(lo <= t && t <= hi))
     {
         return false;

@@ -14,6 +14,8 @@ The reference renders its books' scenes in double as a mode to compare with (all
 
 Independent seeds; a failure is re-run once with fresh seeds (the reference's re-run rule).
 """
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -135,3 +137,43 @@ def test_what_computes_in_float_only_is_refused_in_double(rt):
     books = rt.Scene(rt.builtin_scene("weekend", width=32, spp=4))
     with pytest.raises(ValueError, match="wavefront"):
         rt.Session(books, arithmetic="float64", form="wavefront")
+
+
+def _mixed(rt, spheres, quads, seed):
+    """Spheres and quads at any angle, matte, mirrors and glass: a quad's distance decides where the spheres' light
+    comes from, to the last bit."""
+    import ctypes as C
+
+    from raytracing_b200 import _abi
+
+    def v(p):
+        return _abi.Vec3(*(float(x) for x in p))
+
+    r = np.random.default_rng(seed)
+    s = (_abi.SphereDesc * spheres)(*[_abi.SphereDesc(center=v(r.uniform(-4, 4, 3)), radius=r.uniform(0.1, 0.7),
+                                                      material=i % 3, uv_cos=1.0) for i in range(spheres)])
+    q = (_abi.QuadDesc * quads)(*[_abi.QuadDesc(q=v(r.uniform(-4, 4, 3)), u=v(r.uniform(-2, 2, 3)),
+                                                v=v(r.uniform(-2, 2, 3)), material=i % 3) for i in range(quads)])
+    textures, materials = (_abi.TextureDesc * 1)(), (_abi.MaterialDesc * 3)()
+    textures[0] = _abi.TextureDesc(kind=_abi.RT_TEXTURE_SOLID)
+    textures[0].rgb = v((0.7, 0.6, 0.5))
+    materials[0] = _abi.MaterialDesc(kind=_abi.RT_LAMBERTIAN, texture=0)
+    materials[1] = _abi.MaterialDesc(kind=_abi.RT_METAL, albedo=v((0.8, 0.9, 0.7)))
+    materials[2] = _abi.MaterialDesc(kind=_abi.RT_DIELECTRIC, refraction_index=1.5)
+    cam = _abi.CameraDesc(image_width=64, image_height=48, sqrt_spp=4, max_depth=12, center=v((0, 0, 10)),
+                          sampling=_abi.RT_SAMPLING_MATERIAL)
+    cam.sky_bottom, cam.sky_top = v((1, 1, 1)), v((0.5, 0.7, 1))
+    cam.pixel_delta_u, cam.pixel_delta_v = v((1 / 64, 0, 0)), v((0, -1 / 64, 0))
+    cam.pixel00_loc = v((-0.5, 0.375, 9))
+    desc = _abi.SceneDesc(spheres=s, sphere_count=spheres, quads=q, quad_count=quads, materials=materials,
+                          material_count=3, textures=textures, texture_count=1, camera=cam)
+    session = rt.Session(rt.Scene(C.pointer(desc)), seed=4, arithmetic="float64")
+    session.render_to(16)
+    return session.pixels()
+
+
+@pytest.mark.parametrize("name,spheres,quads,seed", [("tree", 100, 100, 0), ("flat", 12, 11, 2)])
+def test_quads_distances_to_the_last_bit(rt, name, spheres, quads, seed):
+    # as the kernel that held a path in each lane rendered them
+    want = np.load(Path(__file__).resolve().parent / "golden" / "fp64_mixed.npz")[name]
+    assert np.array_equal(_mixed(rt, spheres, quads, seed), want)
