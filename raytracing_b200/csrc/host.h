@@ -449,7 +449,8 @@ private:
     cudaEvent_t stop_ = nullptr;
     device_array<double> sums_;
     device_array<double> partials_;
-    device_array<unsigned long long> counters_; // [0] work, [1] rays, [2] shadow rays, [3..6] the counting build's
+    device_array<unsigned long long> counters_; // [0] work, [1] rays, [2] shadow rays, [3..6] the counting build's,
+                                                // [7] an FP64 launch's ties (launch_params_f64)
     device_array<uint8_t> rgba_;                 // the display's bytes, grown on demand
     bool counting_ = false;
     int64_t passes_ = 0;

@@ -348,8 +348,10 @@ struct launch_params_f64
     unsigned long long* work_counter;
     double* samples;              // 3 a sample
     unsigned long long* counters; // [0] path segments
+    unsigned long long* tied;     // not 0: a path of the view so far met several primitives at one distance
 };
-cudaError_t launch_render_f64(const launch_params_f64& p, int grid, cudaStream_t stream);
+// (`kernels` grows by those launched)
+cudaError_t launch_render_f64(const launch_params_f64& p, int grid, cudaStream_t stream, int32_t& kernels);
 cudaError_t launch_reduce_f64(const launch_params_f64& p, double* sums, cudaStream_t stream);
 cudaError_t render_f64_attributes(const scene_view_f64& scene, kernel_attributes& out);
 

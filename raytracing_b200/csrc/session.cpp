@@ -99,7 +99,7 @@ session::session(std::shared_ptr<resident_scene> scene, const rt_session_options
         }
         apply(c);
     }
-    counters_.allocate(7);
+    counters_.allocate(8);
     set_camera(scene_->camera());
 }
 
@@ -435,6 +435,7 @@ double session::launch(int64_t end)
     {
         cudaEvent_t* m = timing_ ? marks(3) : nullptr;
         launch_params_f64 p64{};
+        last_kernel_launches_ = f64_ ? 1 : 2;
         if (f64_)
         {
             p64.scene = *scene_->view_f64();
@@ -450,7 +451,8 @@ double session::launch(int64_t end)
             p64.work_counter = p.work_counter;
             p64.samples = samples_f64_.data();
             p64.counters = p.counters;
-            check(launch_render_f64(p64, grid_, stream_), "launching the FP64 render kernel");
+            p64.tied = counters_.data() + 7;
+            check(launch_render_f64(p64, grid_, stream_, last_kernel_launches_), "launching the FP64 render kernel");
         }
         else
         {
@@ -463,7 +465,6 @@ double session::launch(int64_t end)
         }
         check(f64_ ? launch_reduce_f64(p64, sums_.data(), stream_) : launch_reduce(r, stream_),
               "launching the reduction");
-        last_kernel_launches_ = f64_ ? 3 : 2;
     }
     if (timing_)
     {

@@ -6,6 +6,7 @@ and for the FP64 integrator the two-wide tree's. The persistent kernel walks tha
 color each, one pass of one segment, says which primitive each of its camera rays meets.
 """
 import ctypes as C
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -13,6 +14,8 @@ import pytest
 from raytracing_b200 import _abi
 
 pytestmark = pytest.mark.gpu
+
+GOLDEN = Path(__file__).resolve().parent / "golden"
 
 
 def _v(x, y, z):
@@ -100,3 +103,31 @@ def test_a_querys_hit_among_the_nearest(rt, name):
     assert met.mean() > 0.05
     assert np.array_equal(ids[met], want[met])
     assert (ids >= 0).sum() >= met.sum() and np.isfinite(ts[met]).all()
+
+
+def _fp64_ids(rt, name):
+    session = rt.Session(_scene(rt, name, _abi.RT_DIFFUSE_LIGHT, 1), seed=7, arithmetic="float64")
+    session.render_to(1)
+    return session.pixels()[..., 0].astype(np.int64) - 1
+
+
+@pytest.mark.parametrize("name", [n for n in SCENES if n != "triangles"])
+def test_fp64_paths_hits_among_the_nearest(rt, name):
+    # as rendered by a lane's walk of the two-wide tree in double, path by path, which a path that meets a tie still takes
+    want = np.load(GOLDEN / "fp64_ties.npz")[name]
+    assert (want >= 0).mean() > 0.05
+    assert np.array_equal(_fp64_ids(rt, name), want)
+
+
+def test_fp64_ties_in_many_launches(rt):
+    # paths dropped at a tie and rendered again, in one launch and in several: one image, and each segment counted once
+    scene = _scene(rt, "tilings", _abi.RT_LAMBERTIAN, 6)
+    a = rt.Session(scene, seed=5, arithmetic="float64")
+    b = rt.Session(scene, seed=5, arithmetic="float64", launch_seconds=1e-4)
+    a.render_to(48)
+    for passes in (16, 32, 48):
+        b.render_to(passes)
+    assert np.array_equal(a.pixels(), b.pixels())
+    assert a.counters()["rays"] == b.counters()["rays"]
+    # a plane of white under a white sky: a path's second segment leaves for good
+    assert 160 * 120 * 48 < a.counters()["rays"] <= 2 * 160 * 120 * 48
