@@ -335,13 +335,16 @@ double batch_engine::step(std::vector<assignment> work, bool flat_pool)
     // largest (allocated before the timing starts)
     int64_t group_samples[batch_groups] = {};
     int group_depth[batch_groups] = {};
+    int64_t pool_job_samples = 0; // the largest of the jobs whose samples the pool kernel numbers, each job's from 0
     for (int g = persistent_groups; g < batch_groups; ++g)
     {
         for (int32_t i = header.group_jobs[g]; i < header.group_jobs[g + 1]; ++i)
         {
             batch_job& b = table_host_[i];
             b.sample_begin = group_samples[g];
-            group_samples[g] += (b.pass_end - b.pass_begin) * int64_t{b.padded_pixels};
+            const int64_t job_samples = (b.pass_end - b.pass_begin) * int64_t{b.padded_pixels};
+            group_samples[g] += job_samples;
+            pool_job_samples = std::max(pool_job_samples, g >= 2 * persistent_groups ? job_samples : 0);
             group_depth[g] = std::max(group_depth[g], b.cam.max_depth);
         }
     }
@@ -350,7 +353,8 @@ double batch_engine::step(std::vector<assignment> work, bool flat_pool)
     {
         wave_->setup(wave_most, stream_);
     }
-    float4* const samples = wave_->samples(*std::max_element(group_samples, group_samples + batch_groups), stream_);
+    float4* const samples =
+        wave_->samples(*std::max_element(group_samples, group_samples + batch_groups), pool_job_samples, stream_);
     check(cudaEventRecord(start_, stream_), "recording a CUDA event");
     if (use_graph_)
     {

@@ -14,6 +14,7 @@
 
 #include "device_types.h"
 #include "kernels.cuh"
+#include "launch_plan.h"
 #include "rt_b200.h"
 
 namespace rtb
@@ -302,8 +303,9 @@ public:
     // Buffers from the device's memory pool, stream-ordered on `stream` (which must outlive the runner): a one-shot
     // render that needs them takes them from what earlier renders left in the pool
     wave_buffers setup(int64_t samples, cudaStream_t stream);
-    // The samples' values alone, for a launch of the pool kernel
-    float4* samples(int64_t count, cudaStream_t stream);
+    // The samples' values alone, for a launch of the pool kernel; `numbered` of them are numbered in a row (the largest
+    // job's, where the launch has jobs): fewer than 2^32
+    float4* samples(int64_t count, int64_t numbered, cudaStream_t stream);
     // step() enqueues one step on `stream`; returns the steps run
     // The steps of one launch until a step queues nothing. step(draining) launches one; draining is true once the
     // host has seen every sample of the launch claimed (work_counter, when given, at sample_count or beyond): the
@@ -466,8 +468,8 @@ private:
     std::unique_ptr<wave_runner> wave_;
     bool pool_ = false;                 // AUTO: the pool kernel, for launches of up to pool_most_samples
     int pool_grid_ = 0;
-    device_array<float4> pool_samples_; // a pool launch's samples, kept for the next
-    device_array<double> samples_f64_;  // the same of an FP64 session
+    device_array<double> samples_f64_;  // an FP64 launch's samples, kept for the next
+    bool pool_takes(int64_t passes) const;
     int32_t last_kernel_launches_ = 0; // the last launch's kernels
     wave_shape shape_{};                // how a step is launched (the autotuner's choice or the defaults)
     tune_candidate tuned_{};

@@ -338,10 +338,11 @@ struct launch_params_f64
     uint64_t seed;
     int64_t pass_begin;
     int64_t pass_end;
-    int64_t sample_count;   // (pass_end - pass_begin) * padded_pixels
+    int64_t sample_count;   // (pass_end - pass_begin) * band_pixels
     int32_t chunk;
     int32_t tiles_x;
-    int32_t padded_pixels;
+    int32_t first_pixel;    // the band of the padded image's pixels this launch renders, whole tiles
+    int32_t band_pixels;
     int32_t round_passes;
     int32_t claim;          // set by the launch
     int32_t pad0;

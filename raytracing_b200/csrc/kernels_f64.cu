@@ -14,6 +14,7 @@
 // widened by the scene's box_margin before the slab test, which keeps the walk conservative.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "kernels.cuh"
@@ -1242,9 +1243,9 @@ __global__ void __launch_bounds__(render_block, 4) pool_f64_kernel(const __grid_
             if (started)
             {
                 // sample s: pass-major, then the pixels in 8 x 4 tiles; off the image for a tile over its edge
-                const auto padded = static_cast<unsigned long long>(P.padded_pixels);
-                const int q = static_cast<int>(s % padded);
-                pass = P.pass_begin + static_cast<int64_t>(s / padded);
+                const auto band = static_cast<unsigned long long>(P.band_pixels);
+                const int q = P.first_pixel + static_cast<int>(s % band);
+                pass = P.pass_begin + static_cast<int64_t>(s / band);
                 const int tile = q >> 5;
                 px = (tile % P.tiles_x) * 8 + (q & 7);
                 py = (tile / P.tiles_x) * 4 + ((q & 31) >> 3);
@@ -1340,15 +1341,20 @@ __global__ void __launch_bounds__(render_block, 4) pool_f64_kernel(const __grid_
 }
 
 // The launch's samples into the image's sums: each chunk's in pass order into its partial, the partials in chunk order
-__global__ void reduce_f64_kernel(const __grid_constant__ launch_params_f64 P, double* sums)
+// (the rows from first_y down that the band has pixels in)
+__global__ void reduce_f64_kernel(const __grid_constant__ launch_params_f64 P, int first_y, double* sums)
 {
     const int x = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
-    const int y = static_cast<int>(blockIdx.y);
+    const int y = first_y + static_cast<int>(blockIdx.y);
     if (x >= P.cam.width || y >= P.cam.height)
     {
         return;
     }
-    const int q = ((y >> 2) * P.tiles_x + (x >> 3)) * 32 + ((y & 3) << 3) + (x & 7);
+    const int q = ((y >> 2) * P.tiles_x + (x >> 3)) * 32 + ((y & 3) << 3) + (x & 7) - P.first_pixel;
+    if (q < 0 || q >= P.band_pixels)
+    {
+        return;
+    }
     double* const sum = sums + 3 * (static_cast<int64_t>(y) * P.cam.width + x);
     double r = sum[0], g = sum[1], b = sum[2];
     for (int64_t pass = P.pass_begin; pass < P.pass_end;)
@@ -1358,7 +1364,7 @@ __global__ void reduce_f64_kernel(const __grid_constant__ launch_params_f64 P, d
         double pr = 0.0, pg = 0.0, pb = 0.0;
         for (; pass < end; ++pass)
         {
-            const double* const s = P.samples + 3 * ((pass - P.pass_begin) * P.padded_pixels + q);
+            const double* const s = P.samples + 3 * ((pass - P.pass_begin) * P.band_pixels + q);
             pr += s[0];
             pg += s[1];
             pb += s[2];
@@ -1410,8 +1416,12 @@ cudaError_t launch_render_f64(const launch_params_f64& p, int grid, cudaStream_t
 cudaError_t launch_reduce_f64(const launch_params_f64& p, double* sums, cudaStream_t stream)
 {
     const dim3 block(128, 1);
-    const dim3 grid(static_cast<unsigned>((p.cam.width + 127) / 128), static_cast<unsigned>(p.cam.height));
-    reduce_f64_kernel<<<grid, block, 0, stream>>>(p, sums);
+    const int64_t row = int64_t{p.tiles_x} * 32; // the padded pixels of a row of tiles, four rows of pixels
+    const int first_y = static_cast<int>(p.first_pixel / row * 4);
+    const int end_y =
+        static_cast<int>(std::min<int64_t>(p.cam.height, (int64_t{p.first_pixel} + p.band_pixels + row - 1) / row * 4));
+    const dim3 grid(static_cast<unsigned>((p.cam.width + 127) / 128), static_cast<unsigned>(end_y - first_y));
+    reduce_f64_kernel<<<grid, block, 0, stream>>>(p, first_y, sums);
     return cudaGetLastError();
 }
 

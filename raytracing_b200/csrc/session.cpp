@@ -19,7 +19,6 @@ namespace
 {
 constexpr double max_launch_seconds = 0.5;              // renderer.h:413
 constexpr size_t partial_budget_bytes = size_t{1} << 30; // a launch's chunk partials: at most 1 GiB
-constexpr size_t wave_sample_budget_bytes = size_t{2} << 30; // a wavefront launch's samples (16 bytes each): 2 GiB
 constexpr double trial_samples = 32e6; // the autotuner's measured launch, by default
 // What a pool launch of an unknown view is taken to render a second, well under any scene's speed (0.5 to 7 G samples/s
 // measured): a first launch of that many samples fits launch_seconds, and a short render is one launch, not a chunk to
@@ -84,6 +83,7 @@ session::session(std::shared_ptr<resident_scene> scene, const rt_session_options
         kernel_attributes pool{};
         check(pool_attributes(view, scene_->quality(), pool), "querying the pool kernel");
         pool_grid_ = pool.multiprocessors * std::max(1, pool.blocks_per_sm);
+        wave_ = std::make_unique<wave_runner>(render_block, wave_group); // for its samples, where no step runs
     }
     if (wavefront_)
     {
@@ -191,7 +191,7 @@ rt_tuning session::autotune(int64_t trial_passes)
     }
     measured = std::max<int64_t>(pass_chunk, (measured + pass_chunk - 1) / pass_chunk * pass_chunk);
     const int64_t max_passes =
-        std::max<int64_t>(pass_chunk, static_cast<int64_t>(wave_sample_budget_bytes / sizeof(float4)) /
+        std::max<int64_t>(pass_chunk, sample_budget_bytes / static_cast<int64_t>(sizeof(float4)) /
                                           (static_cast<int64_t>(padded_pixels_) * pass_chunk) * pass_chunk - pass_chunk);
     measured = std::min(measured, max_passes);
     const double samples = pixels * static_cast<double>(measured);
@@ -250,7 +250,6 @@ session::~session()
     wave_.reset(); // its arrays are freed on the stream, before it goes
     rgba_.release();
     partials_.release();
-    pool_samples_.release();
     samples_f64_.release();
     sums_.release();
     counters_.release();
@@ -302,13 +301,20 @@ void session::set_camera(const rt_camera_desc& camera)
     times_ = rt_kernel_times{};
 }
 
+// Whether the pool kernel takes a launch of so many passes
+bool session::pool_takes(int64_t passes) const
+{
+    const int64_t samples = static_cast<int64_t>(padded_pixels_) * passes;
+    return pool_ && !counting_ && samples <= pool_most_samples(scene_->view(), camera_.max_depth) &&
+           (wavefront_ || (bare_samples_fit(samples) && (passes > 1 || samples > pool_least_bare_samples)));
+}
+
 int64_t session::plan(int64_t target, double budget_seconds) const
 {
     const int64_t next_chunk = (passes_ / pass_chunk + 1) * pass_chunk;
     int64_t end;
-    const double speed = samples_per_second_ > 0         ? samples_per_second_
-                         : (pool_ || f64_) && !counting_ ? least_samples_per_second
-                                                         : 0.0;
+    const bool pool = pool_ && !counting_ && (wavefront_ || pool_takes(pass_chunk));
+    const double speed = samples_per_second_ > 0 ? samples_per_second_ : (pool || f64_) ? least_samples_per_second : 0.0;
     if (speed <= 0)
     {
         end = next_chunk; // the probe: one chunk
@@ -322,12 +328,11 @@ int64_t session::plan(int64_t target, double budget_seconds) const
         end = passes_ + static_cast<int64_t>(std::min(passes, 1e12));
         end = std::max(next_chunk, end / pass_chunk * pass_chunk);
     }
-    // At most what the partials buffer holds (the wavefront: its samples buffer)
-    const size_t sample_bytes = f64_ ? 3 * sizeof(double) : sizeof(float4);
+    // At most what the partials buffer holds (the wavefront, the pool kernels: the samples buffer)
+    const int64_t sample_bytes = f64_ ? 3 * sizeof(double) : sizeof(float4);
     const int64_t max_chunks =
-        (wavefront_ || pool_ || f64_) && !counting_
-            ? std::max<int64_t>(1, static_cast<int64_t>(wave_sample_budget_bytes / sample_bytes) /
-                                       (static_cast<int64_t>(padded_pixels_) * pass_chunk))
+        (wavefront_ && !counting_) || pool || f64_
+            ? std::max<int64_t>(1, sample_budget_bytes / sample_bytes / (static_cast<int64_t>(padded_pixels_) * pass_chunk))
             : std::max<int64_t>(1, max_partial_entries_ / padded_pixels_);
     end = std::min(end, (passes_ / pass_chunk + max_chunks) * pass_chunk);
     return std::min(end, target);
@@ -338,15 +343,16 @@ double session::launch(int64_t end)
     const int64_t first_chunk = passes_ / pass_chunk;
     const int64_t chunks = (end + pass_chunk - 1) / pass_chunk - first_chunk;
     const int64_t samples = static_cast<int64_t>(padded_pixels_) * (end - passes_);
-    const bool pool = pool_ && !counting_ && samples <= pool_most_samples(scene_->view(), camera_.max_depth) &&
-                      (wavefront_ || end - passes_ > 1 || samples > pool_least_bare_samples);
+    const bool pool = pool_takes(end - passes_);
     const bool wave = pool || (wavefront_ && !counting_);
+    const int64_t band = f64_ ? band_pixels(padded_pixels_, end - passes_) : padded_pixels_;
     const size_t needed = static_cast<size_t>(chunks) * static_cast<size_t>(padded_pixels_) * 3;
     if (f64_)
     {
-        if (samples_f64_.size() < 3 * static_cast<size_t>(samples))
+        const size_t stored = 3 * static_cast<size_t>(band * (end - passes_));
+        if (samples_f64_.size() < stored)
         {
-            samples_f64_.allocate_async(3 * static_cast<size_t>(samples), stream_);
+            samples_f64_.allocate_async(stored, stream_);
         }
     }
     else if (!wave && partials_.size() < needed)
@@ -384,10 +390,7 @@ double session::launch(int64_t end)
     wave_buffers b{};
     if (pool)
     {
-        if (pool_samples_.size() < static_cast<size_t>(samples))
-        {
-            pool_samples_.allocate_async(std::max(static_cast<size_t>(samples), 2 * pool_samples_.size()), stream_);
-        }
+        b.samples = wave_->samples(samples, samples, stream_);
     }
     else if (wave)
     {
@@ -399,7 +402,6 @@ double session::launch(int64_t end)
     cudaEvent_t* reduce_marks = timing_ ? marks(2) : nullptr;
     if (pool)
     {
-        b.samples = pool_samples_.data();
         check(launch_pool(p, scene_->quality(), b.samples, samples, pool_grid_, stream_), "launching the pool kernel");
         last_kernel_launches_ = 3;
         if (timing_)
@@ -434,37 +436,46 @@ double session::launch(int64_t end)
     else
     {
         cudaEvent_t* m = timing_ ? marks(3) : nullptr;
-        launch_params_f64 p64{};
-        last_kernel_launches_ = f64_ ? 1 : 2;
+        last_kernel_launches_ = 2;
         if (f64_)
         {
+            launch_params_f64 p64{};
             p64.scene = *scene_->view_f64();
             p64.cam = cam_d_;
             p64.seed = p.seed;
             p64.pass_begin = p.pass_begin;
             p64.pass_end = p.pass_end;
-            p64.sample_count = samples;
             p64.chunk = p.chunk;
             p64.tiles_x = p.tiles_x;
-            p64.padded_pixels = p.padded_pixels;
             p64.round_passes = p.round_passes;
             p64.work_counter = p.work_counter;
             p64.samples = samples_f64_.data();
             p64.counters = p.counters;
             p64.tied = counters_.data() + 7;
-            check(launch_render_f64(p64, grid_, stream_, last_kernel_launches_), "launching the FP64 render kernel");
+            last_kernel_launches_ = 0;
+            for (int64_t first = 0; first < padded_pixels_; first += band)
+            {
+                p64.first_pixel = static_cast<int32_t>(first);
+                p64.band_pixels = static_cast<int32_t>(std::min<int64_t>(band, padded_pixels_ - first));
+                p64.sample_count = p64.band_pixels * (end - passes_);
+                check(launch_render_f64(p64, grid_, stream_, last_kernel_launches_), "launching the FP64 render kernel");
+                if (m && first + band >= padded_pixels_)
+                {
+                    check(cudaEventRecord(m[2], stream_), "recording a CUDA event");
+                }
+                check(launch_reduce_f64(p64, sums_.data(), stream_), "launching the reduction");
+                ++last_kernel_launches_;
+            }
         }
         else
         {
             check(launch_render(p, scene_->quality(), counting_, grid_, stream_), "launching the render kernel");
+            if (m)
+            {
+                check(cudaEventRecord(m[2], stream_), "recording a CUDA event");
+            }
+            check(launch_reduce(r, stream_), "launching the reduction");
         }
-        if (m)
-        {
-            check(cudaEventRecord(m[2], stream_), "recording a CUDA event");
-            reduce_marks = m + 2;
-        }
-        check(f64_ ? launch_reduce_f64(p64, sums_.data(), stream_) : launch_reduce(r, stream_),
-              "launching the reduction");
     }
     if (timing_)
     {

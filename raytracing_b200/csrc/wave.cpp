@@ -104,10 +104,7 @@ wave_buffers wave_runner::setup(int64_t samples, cudaStream_t stream)
         }
         control_.allocate_async(4, stream);
     }
-    if (samples >= (int64_t{1} << 32))
-    {
-        fail(RT_ERR_CAPACITY, "a wavefront run holds fewer than 2^32 samples (a slot keeps its sample's number in 32 bits)");
-    }
+    float4* const values = this->samples(samples, samples, stream);
     const int64_t wanted = (samples + render_block - 1) / render_block * render_block;
     const auto n = static_cast<size_t>(std::min<int64_t>(max_slots, std::max<int64_t>(wanted, render_block)));
     // grown by doubling, never shrunk: a stream of launches of growing size reallocates a few times, not every time
@@ -124,7 +121,7 @@ wave_buffers wave_runner::setup(int64_t samples, cudaStream_t stream)
     wave_buffers b{};
     b.slots = slots_.data();
     b.slot_count = static_cast<int32_t>(n);
-    b.samples = this->samples(samples, stream);
+    b.samples = values;
     b.sample_count = samples;
     b.query_o = query_o_.data();
     b.query_d = query_d_.data();
@@ -135,8 +132,12 @@ wave_buffers wave_runner::setup(int64_t samples, cudaStream_t stream)
     return b;
 }
 
-float4* wave_runner::samples(int64_t count, cudaStream_t stream)
+float4* wave_runner::samples(int64_t count, int64_t numbered, cudaStream_t stream)
 {
+    if (!samples_numbered(numbered))
+    {
+        fail(RT_ERR_CAPACITY, "a wavefront run holds fewer than 2^32 samples (a slot keeps its sample's number in 32 bits)");
+    }
     if (samples_.size() < static_cast<size_t>(count))
     {
         samples_.allocate_async(std::max(static_cast<size_t>(count), 2 * samples_.size()), stream);

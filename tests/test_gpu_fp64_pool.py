@@ -95,3 +95,21 @@ def test_the_float_boxes_miss_no_hit(rt, center, scale, seed):
     assert images[0][1] == images[1][1]
     assert np.array_equal(images[0][0], images[1][0])
     assert images[0][1] > 1.3 * 201 * 151 * 16  # paths that bounce
+
+
+@pytest.mark.parametrize("name", ["quads", "weekend"])
+def test_samples_beyond_the_budget_in_bands(rt, name):
+    # 16 passes of 2,801 x 2,011 pixels are more samples than 2 GiB hold: two bands, whose last tiles hang over both
+    # edges; of 8 passes one. The chunk's sums are added in two parts then: equal but for the rounding of 16 additions.
+    scene = rt.Scene(rt.builtin_scene(name, width=64, spp=16, depth=2))
+    camera = rt.builtin_camera(name, width=2801, height=2011, spp=16, depth=2)
+    per_band = 4 if name == "weekend" else 3
+    images, rays = [], []
+    for targets, kernels in (([16], [2 * per_band]), ([8, 16], [per_band, per_band])):
+        session = rt.Session(scene, seed=1, arithmetic="float64", launch_seconds=0.5)
+        session.set_camera(camera)
+        assert [session.render_to(t)["kernel_launches"] for t in targets] == kernels
+        images.append(session.pixels())
+        rays.append(session.counters()["rays"])
+    assert rays[0] == rays[1]
+    assert np.allclose(images[0], images[1], rtol=32 * 2.0 ** -53, atol=0)

@@ -134,3 +134,27 @@ def test_continuous_servers_books_requests_equal_their_sessions(rt, scenes):
         assert np.array_equal(server.fetch(i), session.pixels()), scenes[k]
     assert server.stats()["used_bytes"] == 0
     server.close()
+
+
+def test_an_image_whose_samples_are_too_many_to_number_is_refused(rt):
+    # a chunk of 16 passes of 16,400 x 16,400 pixels has 2^32 samples and more; one pass has not
+    scene = rt.Scene(rt.builtin_scene("cornell", width=64, spp=16, depth=1))
+    session = rt.Session(scene, seed=1)
+    session.set_camera(rt.builtin_camera("cornell", width=16400, height=16400, spp=16, depth=1))
+    with pytest.raises(rt.CapacityError):
+        session.render_to(16)
+    assert session.state() == 0
+
+
+def test_a_bare_scenes_samples_beyond_the_budget(rt):
+    # 16 passes of 3,901 x 2,201 pixels are more samples than 2 GiB hold: the persistent kernel's launch, of two kernels;
+    # of 8 passes the pool kernel's, of three
+    scene = rt.Scene(rt.builtin_scene("quads", width=64, spp=16, depth=2))
+    camera = rt.builtin_camera("quads", width=3901, height=2201, spp=16, depth=2)
+    images = []
+    for form, targets, kernels in (("auto", [16], [2]), ("auto", [8, 16], [3, 3]), ("persistent", [16], [2])):
+        session = rt.Session(scene, seed=1, form=form, launch_seconds=0.5)
+        session.set_camera(camera)
+        assert [session.render_to(t)["kernel_launches"] for t in targets] == kernels
+        images.append(session.pixels() if len(targets) == 1 else None)
+    assert np.array_equal(images[0], images[2])
