@@ -17,6 +17,13 @@ constexpr bool samples_numbered(int64_t samples) { return samples < (int64_t{1} 
 // is 24 bytes a pixel and chunk): its samples fit the budget, so they are numbered too
 constexpr bool bare_samples_fit(int64_t samples) { return samples <= sample_budget_bytes / 16; }
 
+// What a samples buffer of `held` samples grows to for a launch of `count`: twice its size, so that launches of growing
+// size reallocate a few times, but not beyond the budget for that
+constexpr int64_t grown_samples(int64_t count, int64_t held)
+{
+    return std::max(count, std::min(2 * held, sample_budget_bytes / 16));
+}
+
 // A double launch's samples in bands of whole tiles (32 pixels of the padded image) one after another, each band with all
 // of the launch's passes: a pixel's samples are added in one order whatever the bands. The pixels of a band, every band
 // but the last: all of them where they fit the budget, else an even share that does (a tile at least).

@@ -140,7 +140,7 @@ float4* wave_runner::samples(int64_t count, int64_t numbered, cudaStream_t strea
     }
     if (samples_.size() < static_cast<size_t>(count))
     {
-        samples_.allocate_async(std::max(static_cast<size_t>(count), 2 * samples_.size()), stream);
+        samples_.allocate_async(static_cast<size_t>(grown_samples(count, static_cast<int64_t>(samples_.size()))), stream);
     }
     return samples_.data();
 }

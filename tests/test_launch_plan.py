@@ -4,7 +4,7 @@ that no test can render.
 * A path keeps its sample's number in 32 bits: a bare scene's launch that the pool kernel takes, and every band of a
   double launch, has fewer than 2^32 samples, whatever the image (up to 2^31 pixels) and the passes; a wavefront's launch
   of 2^32 samples or more is refused.
-* The stored samples of either stay within 2 GiB.
+* The stored samples of either stay within 2 GiB, a buffer grown by doubling too.
 * A double launch's bands are whole tiles, cover the image, and are one where the samples fit.
 """
 import shutil
@@ -44,6 +44,19 @@ int main()
         wrong += samples * 24 > (int64_t{2} << 30) && band == padded;
         (band < padded ? banded : whole) += 1;
     };
+    for (int i = 0; i < 20000; ++i)
+    {
+        // a buffer grown from launch to launch: it holds the launch, and more than 2 GiB only where the launch does
+        int64_t held = 0;
+        for (int k = 0; k < 8; ++k)
+        {
+            const int64_t count = 1 + static_cast<int64_t>(gen() >> (24 + gen() % 30));
+            held = count > held ? grown_samples(count, held) : held;
+            wrong += held < count;
+            if (count * 16 > (int64_t{2} << 30)) { break; }
+            wrong += held * 16 > (int64_t{2} << 30);
+        }
+    }
     for (int64_t p : {1, 2, 15, 16, 32, 4096})
     {
         for (int64_t w : {1, 8, 9, 256, 1920, 3840, 7680, 16383, 16384, 16400, 30000, 46300})
