@@ -20,10 +20,6 @@ namespace
 constexpr double max_launch_seconds = 0.5;              // renderer.h:413
 constexpr size_t partial_budget_bytes = size_t{1} << 30; // a launch's chunk partials: at most 1 GiB
 constexpr double trial_samples = 32e6; // the autotuner's measured launch, by default
-// What a pool launch of an unknown view is taken to render a second, well under any scene's speed (0.5 to 7 G samples/s
-// measured): a first launch of that many samples fits launch_seconds, and a short render is one launch, not a chunk to
-// measure the speed and the rest (each launch ends with its last paths: 400x225 x 32 in 1.27 ms as two launches)
-constexpr double least_samples_per_second = 1e8;
 } // namespace
 
 session::session(std::shared_ptr<resident_scene> scene, const rt_session_options& options)
@@ -314,7 +310,7 @@ int64_t session::plan(int64_t target, double budget_seconds) const
     const int64_t next_chunk = (passes_ / pass_chunk + 1) * pass_chunk;
     int64_t end;
     const bool pool = pool_ && !counting_ && (wavefront_ || pool_takes(pass_chunk));
-    const double speed = samples_per_second_ > 0 ? samples_per_second_ : (pool || f64_) ? least_samples_per_second : 0.0;
+    const double speed = samples_per_second_ > 0 ? samples_per_second_ : (pool || f64_) ? first_launch_speed(camera_.max_depth, f64_) : 0.0;
     if (speed <= 0)
     {
         end = next_chunk; // the probe: one chunk

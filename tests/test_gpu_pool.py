@@ -158,3 +158,34 @@ def test_a_bare_scenes_samples_beyond_the_budget(rt):
         assert [session.render_to(t)["kernel_launches"] for t in targets] == kernels
         images.append(session.pixels() if len(targets) == 1 else None)
     assert np.array_equal(images[0], images[2])
+
+
+@pytest.mark.parametrize("arithmetic", ["float32", "float64"])
+def test_a_first_launch_of_long_paths_is_short(rt, arithmetic):
+    # a white room without a way out: paths run to their 4,000th segment, and a launch is asked to take 50 ms
+    import ctypes as C
+
+    from raytracing_b200 import _abi
+
+    def v(x, y, z):
+        return _abi.Vec3(float(x), float(y), float(z))
+
+    walls = []
+    for a in range(3):
+        for side in (-3, 3):
+            q, u, w = [-3, -3, -3], [0, 0, 0], [0, 0, 0]
+            q[a], u[(a + 1) % 3], w[(a + 2) % 3] = side, 6, 6
+            walls.append(_abi.QuadDesc(q=v(*q), u=v(*u), v=v(*w)))
+    quads, textures, materials = (_abi.QuadDesc * 6)(*walls), (_abi.TextureDesc * 1)(), (_abi.MaterialDesc * 1)()
+    textures[0] = _abi.TextureDesc(kind=_abi.RT_TEXTURE_SOLID)
+    textures[0].rgb = v(1, 1, 1)
+    materials[0] = _abi.MaterialDesc(kind=_abi.RT_LAMBERTIAN, texture=0)
+    cam = _abi.CameraDesc(image_width=64, image_height=64, sqrt_spp=1, max_depth=4000, center=v(0, 0, 2),
+                          sampling=_abi.RT_SAMPLING_MATERIAL)
+    cam.pixel_delta_u, cam.pixel_delta_v, cam.pixel00_loc = v(1 / 64, 0, 0), v(0, -1 / 64, 0), v(-0.5, 0.5, 1)
+    desc = _abi.SceneDesc(quads=quads, quad_count=6, materials=materials, material_count=1, textures=textures,
+                          texture_count=1, camera=cam)
+    session = rt.Session(rt.Scene(C.pointer(desc)), seed=1, arithmetic=arithmetic, launch_seconds=0.05)
+    report = session.render_to(512)
+    assert session.counters()["rays"] > 1000 * 64 * 64 * 512  # (a ray leaves through an edge now and then)
+    assert report["launches"] > 1 and report["longest_launch_seconds"] < 0.1

@@ -5,6 +5,7 @@ that no test can render.
   double launch, has fewer than 2^32 samples, whatever the image (up to 2^31 pixels) and the passes; a wavefront's launch
   of 2^32 samples or more is refused.
 * The stored samples of either stay within 2 GiB, a buffer grown by doubling too.
+* A first launch of an unknown view is planned by its paths' longest, so its length in time does not grow with the depth.
 * A double launch's bands are whole tiles, cover the image, and are one where the samples fit.
 """
 import shutil
@@ -68,6 +69,15 @@ int main()
     {
         const int64_t w = 1 + static_cast<int64_t>(gen() % 46300), h = 1 + static_cast<int64_t>(gen() % 46300);
         check(w, h, 1 + static_cast<int64_t>(gen() % 64));
+    }
+    for (const bool f64 : {false, true})
+    {
+        // a first launch's segments a second never above what the slowest measured scenes make, times 2.5
+        for (int depth : {0, 1, 50, 51, 1000, 10000, 2147483647})
+        {
+            wrong += first_launch_speed(depth, f64) * std::max(depth, 1) > (f64 ? 2.2e9 : 2.0e9) * 2.5;
+        }
+        wrong += first_launch_speed(50, f64) != first_launch_speed(1, f64) || first_launch_speed(5000, f64) * 100 != first_launch_speed(50, f64);
     }
     std::printf("%lld %lld %lld %lld %lld\n", checked, wrong, refused, banded, whole);
     return wrong == 0 ? 0 : 1;
