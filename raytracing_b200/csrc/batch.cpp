@@ -242,7 +242,8 @@ double batch_engine::step(std::vector<assignment> work, bool flat_pool)
         return 0;
     }
     ensure_capacity(work.size(), static_cast<size_t>(entries) * 3);
-    // The books' jobs on trees four wide go to the pool kernel, in any step: its launches end without a drain.
+    // The books' jobs on trees four wide go to the pool kernel, in any step: its launches end without a drain. (They count
+    // toward the step's length as they did in the steps: the flat-searched jobs' form, and so their rounding, follows it.)
     // A short step (a server's) keeps its wavefront runs to one: every run ends with a drain (its last paths finishing
     // while most slots idle, a path's length of steps), so the tree-searched jobs share one group (the kernels with
     // the second book's features render the scenes without them) and the flat-searched ones take the persistent

@@ -80,7 +80,7 @@ struct alignas(16) batch_job
 
 // Whether a scene has any of the second book's features (moving spheres, textures other than solid colors, smoke):
 // its kernels are compiled with their code, the others without
-inline bool has_features(const scene_view& s) { return s.has_motion != 0 || s.has_textures != 0 || s.medium_count > 0; }
+RTB_HD inline bool has_features(const scene_view& s) { return s.has_motion != 0 || s.has_textures != 0 || s.medium_count > 0; }
 
 // Whether the wavefront's steps render a scene faster than the persistent kernel (a session's AUTO takes the pool kernel
 // before either, pool_suits): every tree-searched scene (its walks diverge: the mesh 3.2 times and the sphere scenes

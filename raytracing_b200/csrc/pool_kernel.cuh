@@ -397,7 +397,9 @@ __global__ void __launch_bounds__(render_block, pool_shape_of<QUALITY, FEATURES,
                     from = static_cast<int>(rec[record::from][slot]);
                     skip = QUALITY && shadow ? static_cast<int>(rec[record::skip][slot]) : -1;
                     inward = (meta & (QUALITY && shadow ? pool_shadow_inward : pool_inward)) != 0u;
-                    inverse_a = 1.0f / (FEATURES ? length_squared<rounds::walk_features>(d) : length_squared(d));
+                    // (a batch's kernel with the features may render a scene without them too: rounded as its own does)
+                    const bool features = FEATURES && (!BATCH || has_features(S));
+                    inverse_a = 1.0f / (features ? length_squared<rounds::walk_features>(d) : length_squared(d));
                     ray = wide_ray_of(o, d);
                 }
                 const bool has_query = slot >= 0;

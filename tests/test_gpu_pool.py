@@ -189,3 +189,15 @@ def test_a_first_launch_of_long_paths_is_short(rt, arithmetic):
     report = session.render_to(512)
     assert session.counters()["rays"] > 1000 * 64 * 64 * 512  # (a ray leaves through an edge now and then)
     assert report["launches"] > 1 and report["longest_launch_seconds"] < 0.1
+
+
+@pytest.mark.parametrize("passes", [1, 17])
+def test_a_batched_tree_job_beside_others_with_features(rt, passes):
+    # a step of few samples, plain scenes and scenes with motion, textures or smoke in one batch
+    named = ["weekend", "final", "cover-700", "bouncing", "cover-2000"]
+    jobs = [(rt.builtin_scene(n, width=160 + 8 * k, height=120, spp=passes), 70 + k, passes) for k, n in enumerate(named)]
+    batch = rt.batch_render(jobs)
+    for (desc, seed, _), image, name in zip(jobs, batch.images, named):
+        session = rt.Session(rt.Scene(desc), seed=seed)
+        session.render_to(passes)
+        assert np.array_equal(image, session.pixels()), name
