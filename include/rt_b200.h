@@ -426,7 +426,9 @@ rt_status rt_session_kernel_times(const rt_session* session, rt_kernel_times* ti
  * its launch bounds give: 8, or 6 with more registers a thread) and its grid (blocks per multiprocessor); the slot
  * pool, which is the query queue's capacity (two queries a slot); the shade kernel's block size. The best shape stays
  * with the session and is remembered, per device and scene class (flat or tree, integrator, features, triangles,
- * size), for the sessions made after it. The image does not depend on the shape. The view must have no passes yet
+ * size), for the sessions made after it. An AUTO session whose launches of the trials' length the pool kernel renders
+ * measures that too: it keeps the pool kernel for all its launches if no shape is faster, else for the shorter ones
+ * (speeds reported are the shapes'). The image does not depend on the shape. The view must have no passes yet
  * (RT_ERR_LOGIC otherwise) and starts over afterwards; a persistent-form session has nothing to tune (slots 0). */
 typedef struct rt_tuning
 {

@@ -372,6 +372,7 @@ struct tune_candidate
     int trace_blocks_per_sm;
     int shade_block;
     int trace_min_blocks;
+    int64_t pool_most = INT64_MAX; // AUTO: a launch of more samples than this takes the steps, measured faster there
 };
 struct tune_space
 {
@@ -468,6 +469,7 @@ private:
     std::unique_ptr<wave_runner> wave_;
     bool pool_ = false;                 // AUTO: the pool kernel, for launches of up to pool_most_samples
     int pool_grid_ = 0;
+    int64_t pool_most_ = INT64_MAX;     // and up to this many (tune_candidate)
     device_array<double> samples_f64_;  // an FP64 launch's samples, kept for the next
     bool pool_takes(int64_t passes) const;
     int32_t last_kernel_launches_ = 0; // the last launch's kernels

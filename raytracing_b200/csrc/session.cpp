@@ -92,6 +92,7 @@ session::session(std::shared_ptr<resident_scene> scene, const rt_session_options
         {
             c = cached;
             tuning_.from_cache = 1;
+            pool_most_ = cached.pool_most;
         }
         apply(c);
     }
@@ -210,17 +211,39 @@ rt_tuning session::autotune(int64_t trial_passes)
         apply(c);
         return speed();
     };
-    // An AUTO session that renders by the pool kernel stays with it unless the steps' best shape is faster
-    const double pool_speed = pool_ ? speed() : 0.0;
-    pool_ = false;
-    const tune_outcome o = coordinate_descent(tuned_, space, measure);
+    // Where the pool kernel takes a launch as long as the trials', it is measured too: a launch of the trials' length or
+    // longer takes the steps if their best shape is faster. Shorter launches, and all where the trials are beyond the
+    // pool kernel anyway, go as before.
+    const bool pool = pool_;
+    tune_outcome o{};
+    int64_t pool_most = pool_most_;
+    try
+    {
+        pool_most_ = INT64_MAX;
+        const bool compared = pool_takes(measured);
+        const double pool_speed = compared ? speed() : 0.0;
+        pool_ = false;
+        o = coordinate_descent(tuned_, space, measure);
+        if (compared)
+        {
+            pool_most = pool_speed > o.best_speed ? INT64_MAX : static_cast<int64_t>(padded_pixels_) * measured - 1;
+        }
+    }
+    catch (...)
+    {
+        pool_ = pool;
+        pool_most_ = pool_most;
+        counting_ = counting;
+        throw;
+    }
+    pool_ = pool;
+    pool_most_ = o.best.pool_most = pool_most;
     counting_ = counting;
     tuning_.from_cache = 0;
     tuning_.trials = o.trials;
     tuning_.samples_per_second = o.best_speed;
     tuning_.default_samples_per_second = o.default_speed;
     apply(o.best);
-    pool_ = pool_speed > o.best_speed;
     remember_tuning(tune_key(scene_->device(), view, scene_->quality()), o.best);
     set_camera(camera_);
     return tuning_;
@@ -301,7 +324,8 @@ void session::set_camera(const rt_camera_desc& camera)
 bool session::pool_takes(int64_t passes) const
 {
     const int64_t samples = static_cast<int64_t>(padded_pixels_) * passes;
-    return pool_ && !counting_ && samples <= pool_most_samples(scene_->view(), camera_.max_depth) &&
+    return pool_ && !counting_ && samples <= pool_most_ &&
+           samples <= pool_most_samples(scene_->view(), camera_.max_depth) &&
            (wavefront_ || (bare_samples_fit(samples) && (passes > 1 || samples > pool_least_bare_samples)));
 }
 

@@ -106,3 +106,20 @@ def test_kernel_times_add_up(rt):
         else:
             assert kt["render"][1] == rep["launches"] and kt["shade"][1] == 0
         assert kt["reduce"][1] == rep["launches"]
+
+
+@pytest.mark.parametrize("name,kw,trial", [("mesh-ggx", dict(width=160, spp=16, mesh_level=3, env_width=64, depth=6), 0),
+                                           ("weekend", dict(width=160, spp=16), 32)])
+def test_an_auto_session_keeps_its_kernel_where_it_was_not_beaten(rt, name, kw, trial):
+    # the mesh's trials (some 32M samples at depth 6) are beyond the pool kernel, which renders its short launches; the
+    # cover scene's are its own, and it is the faster. Either way, and in a later session of the class, a short launch
+    # is one pool kernel (with its counter's clearing and the reduction: three), and the image the untuned session's.
+    scene = rt.Scene(rt.builtin_scene(name, **kw))
+    plain = rt.Session(scene, seed=4)
+    plain.render_to(16)
+    tuned = rt.Session(scene, seed=4)
+    assert tuned.autotune(trial)["trials"] >= 8
+    for session in (tuned, rt.Session(scene, seed=4)):
+        assert session.tuning()["from_cache"] == (session is not tuned)
+        assert session.render_to(16)["kernel_launches"] == 3
+        assert np.array_equal(session.pixels(), plain.pixels())
