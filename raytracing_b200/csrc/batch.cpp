@@ -210,10 +210,28 @@ double batch_engine::step(std::vector<assignment> work, bool flat_pool)
     work.erase(std::remove_if(work.begin(), work.end(),
                               [&](const assignment& a) { return a.pass_end <= jobs_.at(a.handle)->passes; }),
                work.end());
+    const auto pooled = [&](const job& j) {
+        const scene_view& v = j.scene->view();
+        return !j.scene->quality() && (v.flat == 0 || flat_pool) && wavefront_suits(v) && pool_suits(v, false);
+    };
     int64_t entries = 0;
-    for (const assignment& a : work)
+    for (assignment& a : work)
     {
-        const job& j = *jobs_.at(a.handle);
+        job& j = *jobs_.at(a.handle);
+        if (a.band > 0)
+        {
+            if (!pooled(j))
+            {
+                fail(RT_ERR_LOGIC, "only the pool kernel renders an image in bands");
+            }
+            a.pass_end = std::min(a.pass_end, (j.passes / pass_chunk + 1) * pass_chunk);
+            a.band = std::min<int64_t>((a.band + 31) / 32 * 32, j.padded - j.banded);
+            if (j.bands.size() == 0)
+            {
+                j.bands.allocate_async(3 * static_cast<size_t>(j.padded), stream_);
+            }
+            continue;
+        }
         entries += chunks_of(j.passes, a.pass_end) * j.padded;
     }
     while (entries > max_partial_entries_)
@@ -222,7 +240,7 @@ double batch_engine::step(std::vector<assignment> work, bool flat_pool)
         for (assignment& a : work)
         {
             const job& j = *jobs_.at(a.handle);
-            const int64_t chunks = chunks_of(j.passes, a.pass_end);
+            const int64_t chunks = a.band > 0 ? 1 : chunks_of(j.passes, a.pass_end);
             if (chunks > 1 && entries > max_partial_entries_)
             {
                 const int64_t keep = std::max<int64_t>(1, chunks / 2);
@@ -249,10 +267,6 @@ double batch_engine::step(std::vector<assignment> work, bool flat_pool)
     // the second book's features render the scenes without them) and the flat-searched ones take the persistent
     // kernel, whose tail overlaps nothing either but is shorter. Measured on the 10 ms steps of the served stream: 2%
     // above the flat scenes in a wavefront group of their own, whose second drain costs more than its walks save.
-    const auto pooled = [&](const job& j) {
-        const scene_view& v = j.scene->view();
-        return !j.scene->quality() && (v.flat == 0 || flat_pool) && wavefront_suits(v) && pool_suits(v, false);
-    };
     int64_t wave_samples = 0;
     bool tree_features = false;
     bool pool_features = false;
@@ -319,10 +333,23 @@ double batch_engine::step(std::vector<assignment> work, bool flat_pool)
         b.partials = arena_.data() + 3 * partial_offset;
         b.sums = j.sums.data();
         b.counters = j.counters.data();
+        const int64_t image = int64_t{j.camera.image_width} * j.camera.image_height;
+        if (work[i].band > 0)
+        {
+            b.first_pixel = static_cast<int32_t>(j.banded);
+            b.padded_pixels = static_cast<int32_t>(work[i].band);
+            b.cam.div_padded = make_fast_divisor(static_cast<uint32_t>(work[i].band));
+            b.partials = j.bands.data() + 3 * j.banded;
+            pixels += j.banded + work[i].band == j.padded ? image : 0;
+            last_samples_ += work[i].band * (b.pass_end - b.pass_begin);
+        }
+        else
+        {
+            pixels += image;
+            last_samples_ += image * (b.pass_end - b.pass_begin);
+            partial_offset += int64_t{b.chunks} * b.padded_pixels;
+        }
         items += int64_t{b.chunks} * b.padded_pixels;
-        pixels += int64_t{j.camera.image_width} * j.camera.image_height;
-        last_samples_ += int64_t{j.camera.image_width} * j.camera.image_height * (b.pass_end - b.pass_begin);
-        partial_offset += int64_t{b.chunks} * b.padded_pixels;
     }
     // Each group's item range: from its first job's start to the next group's
     for (int g = 0; g <= batch_groups; ++g)
@@ -428,7 +455,14 @@ double batch_engine::step(std::vector<assignment> work, bool flat_pool)
     check(cudaEventElapsedTime(&ms, start_, stop_), "timing the GPU");
     for (const assignment& a : work)
     {
-        jobs_.at(a.handle)->passes = a.pass_end;
+        job& j = *jobs_.at(a.handle);
+        j.banded += a.band;
+        if (a.band == 0 || j.banded == j.padded)
+        {
+            j.passes = a.pass_end;
+            j.banded = 0;
+            j.bands.release();
+        }
     }
     return ms / 1000.0;
 }
@@ -544,7 +578,7 @@ render_server::render_server(const rt_server_options& options) : options_(option
         // First frames are rendered in batched steps of their own (a first frame's last paths then advance through
         // steps of a few slots, not of the whole pool), on a stream whose kernels go first, and handed over
         engine_ = std::make_unique<batch_engine>(size_t{256} << 20, options.use_graph != 0, true);
-        engine_->reserve_wavefront(int64_t{1} << 24);
+        engine_->reserve_wavefront(batched_samples);
         // The requests' memory (48 bytes a pixel) mapped now: a pool grown while requests wait stalls the step that
         // admits them (tens of GB at once when large requests arrive together)
         stream_->reserve_pool(std::min<size_t>(static_cast<size_t>(options_.hbm_budget_bytes), size_t{64} << 30));
@@ -600,10 +634,13 @@ void render_server::release(request& r)
 }
 
 // The continuous server's batched requests refined for about `seconds`, least remaining work first, each to the end of
-// a chunk or to its target (as the continuous run adds them), at most a values ring's worth of samples; the GPU seconds
+// a chunk or to its target (as the continuous run adds them), at most batched_samples of them; the GPU seconds. A request
+// whose next chunk alone is longer than what is left of that renders a band of its pixels, and the next band in the next
+// step: a 4K chunk is 133M samples, 40 ms of a step of 2.
 double render_server::refine_batched(double seconds)
 {
-    constexpr double most_samples = double(int64_t{1} << 26);
+    constexpr double most_samples = double(batched_samples);
+    constexpr double least_band = 1 << 18; // a band's samples, but where the image has fewer: a launch's worth of paths
     std::vector<std::pair<double, request*>> refine;
     for (auto& [id, r] : requests_)
     {
@@ -629,7 +666,25 @@ double render_server::refine_batched(double seconds)
         const double pixels = double(r.camera.image_width) * r.camera.image_height;
         const double per_pass = pixels * cost_of(r.scene.get());
         const double want = std::min((seconds - planned) / per_pass, (most_samples - samples) / pixels);
-        const int64_t boundary = (done / pass_chunk + 1) * pass_chunk;
+        const int64_t boundary = std::min(r.target, (done / pass_chunk + 1) * pass_chunk);
+        const double chunk = double(boundary - done);
+        // (a chunk that ends a quarter of the step late is not worth a band)
+        if (engine_->banded(r.handle) > 0 || want + 0.25 * seconds / per_pass < chunk || pixels * chunk > most_samples)
+        {
+            if (!work.empty() && want * pixels < least_band)
+            {
+                break;
+            }
+            const int64_t padded = batch_engine::padded_of(r.camera);
+            const int64_t left = padded - engine_->banded(r.handle);
+            int64_t band = static_cast<int64_t>(std::max(want * pixels, least_band) / chunk) / 32 * 32;
+            band = std::min(std::max<int64_t>(band, 32), left);
+            work.push_back({r.handle, boundary, band});
+            step_samples.emplace_back(r.scene.get(), double(band) * chunk);
+            planned += cost_of(r.scene.get()) * double(band) * chunk;
+            samples += double(band) * chunk;
+            continue;
+        }
         const int64_t end = std::min(
             r.target, std::max(boundary, (done + static_cast<int64_t>(std::max(want, 0.0))) / pass_chunk * pass_chunk));
         work.push_back({r.handle, end});

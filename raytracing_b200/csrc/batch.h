@@ -31,10 +31,14 @@ public:
     int add(std::shared_ptr<resident_scene> scene, const rt_camera_desc& camera, uint64_t seed, uint32_t job_id);
     void remove(int handle);
 
+    // `band`: not all of the image's pixels but the next so many of its padded ones, whole tiles, with the passes to the end
+    // of the chunk the job is in (or to pass_end, if that is sooner); the chunk's sums go into the job's with its last
+    // band, which a band may reach beyond. For the pool kernel's jobs; 0: the whole image.
     struct assignment
     {
         int handle;
         int64_t pass_end;
+        int64_t band = 0;
     };
     // One step; returns its GPU seconds. Jobs whose partials do not fit the arena this step are cut back to fewer
     // chunks (at least one each), so every assignment makes progress.
@@ -48,6 +52,8 @@ public:
     // maps no new memory
     void reserve_pool(size_t bytes);
     int64_t passes(int handle) const;
+    // The padded pixels that the job has rendered of its next chunk, in bands
+    int64_t banded(int handle) const { return jobs_.at(handle)->banded; }
     void pixels(int handle, double* out, int64_t count);
     // The job's sums (width * height * 3 doubles) into device memory, complete on return
     void copy_sums(int handle, double* device_out);
@@ -78,6 +84,8 @@ private:
         int64_t passes = 0;
         int tiles_x = 0;
         int padded = 0;
+        int64_t banded = 0;             // the padded pixels whose chunk partials `bands` holds
+        device_array<double> bands;     // 3 a padded pixel, while a chunk is rendered in bands
     };
     std::map<int, std::unique_ptr<job>> jobs_;
     int next_handle_ = 0;
@@ -296,6 +304,8 @@ private:
     uint64_t first_shadow_rays_ = 0;
     // the estimated GPU time of a step of first frames (at least one frame a step)
     static constexpr double first_frame_seconds = 0.004;
+    // the samples of a step of the continuous server's batched refinement at most (1 GB, reserved when it is made)
+    static constexpr int64_t batched_samples = int64_t{1} << 26;
     int64_t next_id_ = 1;
     size_t used_bytes_ = 0;
     std::map<const resident_scene*, double> cost_; // seconds per pixel pass, learned per scene

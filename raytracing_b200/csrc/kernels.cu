@@ -367,7 +367,7 @@ __global__ void reduce_batch_kernel(const batch_params P)
         const int64_t local = i - J.pixel_begin;
         const int y = static_cast<int>(local / J.cam.width);
         const int x = static_cast<int>(local - static_cast<int64_t>(y) * J.cam.width);
-        const int q = ((y >> 2) * J.tiles_x + (x >> 3)) * 32 + ((y & 3) << 3) + (x & 7);
+        const int q = ((y >> 2) * J.tiles_x + (x >> 3)) * 32 + ((y & 3) << 3) + (x & 7) - J.first_pixel;
         double* sum = J.sums + 3 * local;
         double r = sum[0], g = sum[1], b = sum[2];
         for (int k = 0; k < J.chunks; ++k)
@@ -929,7 +929,7 @@ __global__ void wave_batch_partials_kernel(const wave_batch W, const float4* sam
         const int64_t local = i - J.item_begin;
         const int64_t k = local / J.padded_pixels;
         const int q = static_cast<int>(local - k * J.padded_pixels);
-        const int tile = q >> 5;
+        const int tile = (J.first_pixel + q) >> 5;
         const int l = q & 31;
         if ((tile % J.tiles_x) * 8 + (l & 7) >= J.cam.width || (tile / J.tiles_x) * 4 + (l >> 3) >= J.cam.height)
         {

@@ -47,7 +47,9 @@ struct reduce_params
 // One job of a batched launch: a resident scene's view, its camera, and the passes this step renders of it. Its work
 // items are numbered from item_begin in the batch's item space, its pixels from pixel_begin in the batch's pixel
 // space (for the reduction); partials is its own slice of the batch's partials arena. A job of a group the wavefront
-// renders numbers its samples from sample_begin in its group's sample space.
+// renders numbers its samples from sample_begin in its group's sample space. A job rendered in bands (the pool kernel's
+// alone) has in this step padded_pixels of the padded image from first_pixel on, with its camera's divisor and its items
+// to match, one chunk of passes, and its partials from that pixel on; the pixels come into the reduction with its last.
 struct alignas(16) batch_job
 {
     scene_view scene;
@@ -69,7 +71,7 @@ struct alignas(16) batch_job
     int32_t round_passes;
     int32_t quality;
     uint32_t job;                 // the RNG counter's job field
-    int32_t pad0;
+    int32_t first_pixel;
     // A stream run's segment (the server's continuous wavefront): its samples are [sample_begin, sample_begin +
     // pass-major count) of the run's sample space, numbered within the request from local_begin; their values go to
     // values[local - local_begin] and each finished one is counted in *done

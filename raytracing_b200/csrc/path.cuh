@@ -2072,8 +2072,9 @@ struct sample_place
 };
 
 // (uses the camera's divisors: cam.div_padded and cam.div_tiles_x; a number of 2^32 or more, which only a served
-// request's numbering reaches, takes the 64-bit division)
-__device__ __forceinline__ sample_place place_of(int64_t local, const camera_params& cam, int64_t pass_begin)
+// request's numbering reaches, takes the 64-bit division; `first_pixel`: of a job rendered in bands)
+__device__ __forceinline__ sample_place place_of(int64_t local, const camera_params& cam, int64_t pass_begin,
+                                                 int first_pixel = 0)
 {
     const uint32_t padded = cam.div_padded.d;
     int64_t j;
@@ -2090,7 +2091,7 @@ __device__ __forceinline__ sample_place place_of(int64_t local, const camera_par
         j = local / padded;
         q = static_cast<int>(local - j * padded);
     }
-    const int tile = q >> 5;
+    const int tile = (first_pixel + q) >> 5;
     const int l = q & 31;
     const auto ty = static_cast<int>(quotient(static_cast<uint32_t>(tile), cam.div_tiles_x));
     const int tx = tile - ty * static_cast<int>(cam.div_tiles_x.d);

@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(render_block, pool_shape_of<QUALITY, FEATURES,
             sample_place at{0, 0, 0};
             if (started)
             {
-                at = place_of(index, cam, BATCH ? J->pass_begin : P.pass_begin);
+                at = place_of(index, cam, BATCH ? J->pass_begin : P.pass_begin, BATCH ? J->first_pixel : 0);
                 started = at.x < cam.width && at.y < cam.height; // a lane of a tile over the image's edge: no sample
             }
             const unsigned lanes = __ballot_sync(full_warp, started);

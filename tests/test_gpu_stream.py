@@ -173,3 +173,73 @@ def test_continuous_budget_counts_the_accumulator(rt):
         server.step()
     _same_render(server.fetch(ids[1]), _session_split(rt, g, glass.camera, 1, 16))
     server.close()
+
+
+def _steps(server):
+    out = []
+    while True:
+        r = server.step()
+        if r["active"] == 0 and r["queued"] == 0:
+            return out
+        out.append(r["gpu_seconds"])
+
+
+def test_continuous_large_books_requests_keep_the_step(rt):
+    """A 4K request's chunk of 16 passes is some 30 ms; the steps stay near the 2 ms asked for: its chunks are rendered in
+    bands, over several steps. The first steps learn what a pass costs, and a first frame is a pass of its own."""
+    scene = rt.Scene(rt.builtin_scene("weekend"))
+    cam = rt.builtin_camera("weekend", width=3840, height=2160, spp=16, depth=50)
+    server = rt.Server(hbm_budget_bytes=8 << 30, step_seconds=0.002, continuous=1)
+    ids = [server.submit(scene, cam, 5, 20), server.submit(scene, cam, 6, 3)]
+    seconds = _steps(server)
+    assert len(seconds) > 12
+    assert np.median(seconds) < 0.003 and max(seconds[6:]) < 0.006, seconds
+    for i, (seed, target) in zip(ids, ((5, 20), (6, 3))):
+        assert np.array_equal(server.fetch(i), _session_split(rt, scene, cam, seed, target))
+    assert server.stats()["used_bytes"] == 0
+    server.close()
+
+
+@pytest.mark.parametrize("name", ["weekend", "final", "glass", "smoke"])
+def test_continuous_images_in_bands_equal_sessions(rt, name):
+    """Steps so short that every chunk is in bands: images of ragged sizes, read while a chunk is in progress too, between
+    requests cancelled in the middle of theirs."""
+    scene = rt.Scene(rt.builtin_scene(name))
+    views = [(rt.builtin_camera(name, width=w, height=h, spp=16, depth=50), k, t)
+             for k, (w, h, t) in enumerate([(701, 403, 35), (1021, 515, 17), (333, 1001, 2), (900, 700, 33)])]
+    server = rt.Server(hbm_budget_bytes=1 << 30, step_seconds=1e-4, continuous=1)
+    ids = [server.submit(scene, cam, seed, target) for cam, seed, target in views]
+    # least work left first: the third request, the second, the first (cancelled a few steps into its chunk), the fourth
+    read, waited = 0, 0
+    for _ in range(4000):
+        report = server.step()
+        states = [server.poll(i)["state"] for i in ids]
+        if states[1] == "done" and states[0] == "active":
+            waited += 1
+            if waited == 4:
+                server.cancel(ids[0])
+        if states[0] == "cancelled" and states[3] == "active" and report["refined"] == 0 and read < 3:
+            read += 1
+            passes = server.poll(ids[3])["passes"]  # those before the chunk in progress
+            session = rt.Session(scene, seed=3)
+            session.set_camera(views[3][0])
+            session.render_to(1)
+            if passes > 1:
+                session.render_to(passes)
+            if name in ("weekend", "final"):
+                assert np.array_equal(server.fetch(ids[3]), session.pixels())
+                assert np.array_equal(server.display(ids[3]), session.display())
+            else:
+                _same_render(server.fetch(ids[3]), session.pixels())
+        if report["active"] == 0 and report["queued"] == 0:
+            break
+    assert states == ["cancelled", "done", "done", "done"] and read == 3
+    for k in (1, 2, 3):
+        cam, seed, target = views[k]
+        image, want = server.fetch(ids[k]), _session_split(rt, scene, cam, seed, target)
+        if name in ("weekend", "final"):
+            assert np.array_equal(image, want), k
+        else:
+            _same_render(image, want)  # a flat scene's first pass is the persistent kernel's, of its own rounding
+    assert server.stats()["used_bytes"] == 0
+    server.close()
