@@ -5,6 +5,7 @@
 // the blocks to and from the caller's memory, each with two blocks in flight.
 #include <algorithm>
 #include <condition_variable>
+#include <cstdint>
 #include <cstring>
 #include <exception>
 #include <functional>
@@ -245,6 +246,22 @@ void trace_rays(const scene_view& scene, const int32_t* prim_source, const float
     constexpr int64_t per_block = 16384;
     static_assert(per_block * 8 * sizeof(float) <= block_bytes);
     const auto rays_of = [&](int64_t block) { return std::min(per_block, count - block * per_block); };
+    // Answers over the rays' own memory: a block's would overwrite the rays of one not yet read
+    std::vector<float> rays;
+    const auto over = [&](const void* out, const float* in) {
+        const auto o = reinterpret_cast<uintptr_t>(out), i = reinterpret_cast<uintptr_t>(in);
+        const auto n = static_cast<uintptr_t>(count);
+        return o < i + n * 3 * sizeof(float) && i < o + n * sizeof(float);
+    };
+    if (over(ids, origins) || over(ids, directions) || over(ts, origins) || over(ts, directions))
+    {
+        const size_t n = static_cast<size_t>(count) * 3;
+        rays.resize(2 * n);
+        std::copy_n(origins, n, rays.data());
+        std::copy_n(directions, n, rays.data() + n);
+        origins = rays.data();
+        directions = rays.data() + n;
+    }
     pipeline(
         (count + per_block - 1) / per_block, nullptr, true,
         [&](int64_t block, void* memory, cudaStream_t s) {

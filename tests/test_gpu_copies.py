@@ -75,3 +75,19 @@ def test_a_ray_alone_and_among_others(rt, name, kw):
     for k in range(0, len(o), 97):
         i, t = scene.closest_hits(o[k:k + 1], d[k:k + 1])
         assert i[0] == ids[k] and t[0] == ts[k]
+
+
+@pytest.mark.parametrize("n", [100, 2000003])
+def test_hits_over_the_rays_memory(rt, n):
+    # a caller that needs its rays no more: the answers over the end of the origins and of the directions
+    import ctypes as C
+
+    scene = rt.Scene(rt.builtin_scene("weekend"))
+    o, d = _rays(n, 8)
+    ids, ts = scene.closest_hits(o, d)
+    ts_over, ids_over = o.ravel()[2 * n:], d.ravel()[2 * n:].view(np.int32)
+    p = lambda a, t: a.ctypes.data_as(C.POINTER(t))  # noqa: E731
+    rt._check(rt._lib().rt_scene_closest_hits(scene._handle, p(o, C.c_float), p(d, C.c_float), n, p(ids_over, C.c_int32),
+                                              p(ts_over, C.c_float)))
+    assert np.array_equal(ts_over, ts)
+    assert np.array_equal(ids_over, ids)
