@@ -1235,7 +1235,7 @@ __device__ bool sample_lamp(const emitter20& e, float3 x, float a, float b, lamp
         const float inverse_distance = rsqrtf(distance_squared);
         out.wi = inverse_distance * to;
         out.distance = distance_squared * inverse_distance;
-        const float cos_light = -dot(out.wi, make_float3(e.nx, e.ny, e.nz));
+        const float cos_light = -dot<rounds::lamp_cosine>(out.wi, make_float3(e.nx, e.ny, e.nz));
         if (!(cos_light > 0.0f))
         {
             return false;
@@ -1577,12 +1577,12 @@ __device__ __forceinline__ float3 schlick(float3 f0, float cosine)
 }
 
 // f * cos(theta_l) = F D cl / (2 (cl A_v + cv A_l)) and the visible-normal density D / (2 (cv + A_v))
-template <rounding LENGTH>
+template <rounding LENGTH, rounding LIGHT = rounds::other>
 __device__ float3 ggx_eval(float3 n, float3 v, float3 l, float alpha, float3 f0, float& pdf)
 {
     pdf = 0.0f;
     const float cv = dot<rounds::ggx_eval_view>(n, v);
-    const float cl = dot(n, l);
+    const float cl = dot<LIGHT>(n, l);
     const float3 sum = v + l;
     const float len2 = length_squared<LENGTH>(sum);
     if (!(cv > 0.0f) || !(cl > 0.0f) || !(len2 > 0.0f))
@@ -1669,18 +1669,18 @@ __device__ __forceinline__ float gloss_crossing(float c)
 
 // The coat over a matte base of color rho: GGX with F0 0.04 plus the coupled diffuse term; pdf the half-and-half
 // mixture of the two lobes' densities
-template <rounding LENGTH>
+template <rounding LENGTH, rounding LIGHT = rounds::other>
 __device__ float3 gloss_eval(float3 n, float3 v, float3 l, float alpha, float3 rho, float& pdf)
 {
     pdf = 0.0f;
-    const float cv = dot(n, v);
-    const float cl = dot(n, l);
+    const float cv = dot<rounds::ggx_eval_view>(n, v);
+    const float cl = dot<LIGHT>(n, l);
     if (!(cv > 0.0f) || !(cl > 0.0f))
     {
         return make_float3(0.0f, 0.0f, 0.0f);
     }
     float coat_pdf;
-    const float3 coat = ggx_eval<LENGTH>(n, v, l, alpha, make_float3(gloss_coat_f0, gloss_coat_f0, gloss_coat_f0), coat_pdf);
+    const float3 coat = ggx_eval<LENGTH, LIGHT>(n, v, l, alpha, make_float3(gloss_coat_f0, gloss_coat_f0, gloss_coat_f0), coat_pdf);
     pdf = 0.5f * (coat_pdf + cl * inverse_pi_f);
     const float base = gloss_diffuse_scale * (gloss_crossing(cl) * gloss_crossing(cv)) * cl;
     return coat + base * rho;
@@ -1986,7 +1986,7 @@ __device__ __forceinline__ step_result shade_quality(const scene_view& S, const 
         }
         if (scattered)
         {
-            const float3 f = gloss_eval<rounds::ggx_gloss_length>(s.normal, wo, wi, m.alpha, albedo, pdf);
+            const float3 f = gloss_eval<rounds::ggx_gloss_length, rounds::ggx_gloss_light>(s.normal, wo, wi, m.alpha, albedo, pdf);
             scattered = pdf > 0.0f;
             weight = (1.0f / pdf) * f;
         }
@@ -1994,9 +1994,9 @@ __device__ __forceinline__ step_result shade_quality(const scene_view& S, const 
     else if (lobe == lobe_smooth_conductor)
     {
         // The mirror with Schlick's F: no random number (bsdf.cuh:153-166)
-        scattered = dot(s.normal, wo) > 0.0f;
-        wi = unit_vector(reflect(-wo, s.normal));
-        weight = schlick(albedo, dot(s.normal, wo));
+        scattered = dot<rounds::mirror_cosine>(s.normal, wo) > 0.0f;
+        wi = unit_vector(reflect<rounds::mirror_reflect>(-wo, s.normal));
+        weight = schlick(albedo, dot<rounds::mirror_cosine>(s.normal, wo));
     }
     else if (m.kind == RT_METAL)
     {

@@ -26,19 +26,24 @@ struct rounds_compiler
     static constexpr rounding dielectric_reflect = rounding::compiler;
     static constexpr rounding view = rounding::compiler;
     static constexpr rounding lamp_distance = rounding::compiler;
+    static constexpr rounding lamp_cosine = rounding::compiler;
     static constexpr rounding lamp_hit = rounding::compiler;
     static constexpr rounding ggx_eval_view = rounding::compiler;
     static constexpr rounding ggx_eval_half = rounding::compiler;
     static constexpr rounding ggx_light_length = rounding::compiler;
     static constexpr rounding ggx_gloss_length = rounding::compiler;
+    static constexpr rounding ggx_gloss_light = rounding::compiler;
     static constexpr rounding ggx_sample_view = rounding::compiler;
     static constexpr rounding ggx_sample_half = rounding::compiler;
     static constexpr rounding energy = rounding::compiler;
+    static constexpr rounding mirror_cosine = rounding::compiler;
+    static constexpr rounding mirror_reflect = rounding::compiler;
 };
 
 // A session's wavefront, as its shade and trace kernels come out of the compiler: found by writing out one product at
-// a time in those kernels and keeping the form that leaves every image (19 scenes, both integrators) the same bit for
-// bit. The kernels that render a session's samples in another form take this table, so the form changes no image.
+// a time in those kernels and keeping the form that leaves every image (the built-in scenes under both integrators, scenes
+// of each material alone, scenes drawn at random) the same bit for bit. The kernels that render a session's samples in
+// another form take this table, so the form changes no image.
 struct rounds_session
 {
     static constexpr bool bare = false; // whether these kernels render the bare small scenes only
@@ -52,14 +57,18 @@ struct rounds_session
     static constexpr rounding dielectric_reflect = rounding::yz;
     static constexpr rounding view = rounding::y;
     static constexpr rounding lamp_distance = rounding::y;
+    static constexpr rounding lamp_cosine = rounding::y;
     static constexpr rounding lamp_hit = rounding::y;
     static constexpr rounding ggx_eval_view = rounding::y;
     static constexpr rounding ggx_eval_half = rounding::y;
     static constexpr rounding ggx_light_length = rounding::x;
     static constexpr rounding ggx_gloss_length = rounding::y;
+    static constexpr rounding ggx_gloss_light = rounding::y;
     static constexpr rounding ggx_sample_view = rounding::y;
     static constexpr rounding ggx_sample_half = rounding::y;
     static constexpr rounding energy = rounding::y;
+    static constexpr rounding mirror_cosine = rounding::yz;
+    static constexpr rounding mirror_reflect = rounding::yz;
 };
 
 // The persistent kernel's flat search, which renders the bare small scenes: the same but for the ray's squared length

@@ -6,6 +6,8 @@ warp; images whose tiles hang over both edges (claimed numbers without a pixel);
 several launches; paths of one segment. Scenes: both searches, both integrators, with and without the second book's
 features.
 """
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -201,3 +203,55 @@ def test_a_batched_tree_job_beside_others_with_features(rt, passes):
         session = rt.Session(rt.Scene(desc), seed=seed)
         session.render_to(passes)
         assert np.array_equal(image, session.pixels()), name
+
+
+def _every_material(rt, shapes, moving):
+    """Shapes at any angle under NEE with MIS, of every material, with lamps among them: matte, mirrors, glass, metal
+    rough, smooth and below the roughness of a perfect mirror, a coat, lamps that are spheres and quads at any angle."""
+    import ctypes as C
+
+    from raytracing_b200 import _abi
+
+    def v(p):
+        return _abi.Vec3(*(float(x) for x in p))
+
+    r = np.random.default_rng(shapes)
+    kinds = [(_abi.RT_LAMBERTIAN, 0, 0), (_abi.RT_METAL, 0, 0), (_abi.RT_DIELECTRIC, 0, 0), (_abi.RT_DIFFUSE_LIGHT, 0, 0),
+             (_abi.RT_METAL, _abi.RT_MICROFACET_CONDUCTOR, 0.4), (_abi.RT_METAL, _abi.RT_MICROFACET_CONDUCTOR, 0.02),
+             (_abi.RT_LAMBERTIAN, _abi.RT_MICROFACET_GLOSS, 0.4)]
+    n = len(kinds)
+    textures, materials, facets = (_abi.TextureDesc * 2)(), (_abi.MaterialDesc * n)(), (_abi.MicrofacetDesc * n)()
+    textures[0], textures[1] = _abi.TextureDesc(), _abi.TextureDesc()
+    textures[0].rgb, textures[1].rgb = v((0.7, 0.6, 0.5)), v((5, 6, 4))
+    for k, (kind, facet, roughness) in enumerate(kinds):
+        materials[k] = _abi.MaterialDesc(kind=kind, texture=int(kind == _abi.RT_DIFFUSE_LIGHT), albedo=v((0.9, 0.7, 0.5)),
+                                         refraction_index=1.5)
+        facets[k] = _abi.MicrofacetDesc(kind=facet, roughness=roughness)
+    s = (_abi.SphereDesc * shapes)(*[_abi.SphereDesc(center=v(r.uniform(-4, 4, 3)), radius=r.uniform(0.2, 1.0),
+                                                     material=i % n, uv_cos=1.0) for i in range(shapes)])
+    q = (_abi.QuadDesc * shapes)(*[_abi.QuadDesc(q=v(r.uniform(-5, 4, 3)), u=v(r.uniform(-2, 2, 3)),
+                                                 v=v(r.uniform(-2, 2, 3)), material=i % n) for i in range(shapes)])
+    if moving:
+        s[0].displacement = v((0.3, 0.2, -0.1))
+    cam = _abi.CameraDesc(image_width=64, image_height=48, sqrt_spp=4, max_depth=10, center=v((0, 0, 11)),
+                          sampling=_abi.RT_SAMPLING_MATERIAL)
+    cam.sky_bottom, cam.sky_top = v((0.3, 0.3, 0.3)), v((0.1, 0.2, 0.3))
+    cam.pixel_delta_u, cam.pixel_delta_v = v((1 / 64, 0, 0)), v((0, -1 / 64, 0))
+    cam.pixel00_loc = v((-0.5, 0.375, 10))
+    desc = _abi.SceneDesc(spheres=s, sphere_count=shapes, quads=q, quad_count=shapes, materials=materials, material_count=n,
+                          textures=textures, texture_count=2, microfacets=facets, microfacet_count=n, camera=cam,
+                          combination=_abi.RT_COMBINE_POWER_HEURISTIC, quality=1)
+    return rt.Scene(C.pointer(desc))
+
+
+@pytest.mark.parametrize("moving", [False, True])
+@pytest.mark.parametrize("shapes", [10, 60], ids=["flat", "tree"])
+def test_every_material_under_nee(rt, shapes, moving):
+    # the pool kernel, the steps, and the steps as they were before the pool kernel: one image, to the last bit
+    scene = _every_material(rt, shapes, moving)
+    assert scene.stats()["flat"] == (shapes == 10)
+    _equal(rt, scene, 9, 16)
+    session = rt.Session(scene, seed=9)
+    session.render_to(16)
+    want = np.load(Path(__file__).resolve().parent / "golden" / "nee_materials.npz")[f"{shapes}-{int(moving)}"]
+    assert np.array_equal(session.pixels(), want)
