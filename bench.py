@@ -144,8 +144,8 @@ def read_peaks() -> dict:
     return {"hbm_gbs": 6650.0, "source": "fallback"}
 
 
-# The wavefront's state per unit of work, by the layout of its slots and queues (raytracing_b200/csrc/kernels.cu): what
-# the shade kernel must move through HBM for each segment (the slot's 16-byte rows in and out: five, or for a scene
+# The wavefront's state per unit of work, by the layout of its slots and queues (raytracing_b200/csrc/wave_shade.cuh):
+# what the shade kernel must move through HBM for each segment (the slot's 16-byte rows in and out: five, or for a scene
 # without the second book's features, whose paths carry no time or job, three for the books' integrator and four for
 # NEE/MIS; the walk's answer; the next query of 48 bytes), for each shadow ray (its answer, its three rows out and back in, its query) and for each sample
 # (its value). These are the bytes that bind the shade kernel: the scene itself (a few KB) is read from L1.
@@ -158,8 +158,8 @@ SHADE_BYTES_PER_SAMPLE = 16
 
 
 def slot_rows_of(desc, kernel_name: str) -> int:
-    """The rows of a session's wavefront slot for a scene without moving spheres, textures or smoke (kernels.cu
-    compact_slots): three for the books' integrator, four for NEE/MIS; five otherwise."""
+    """The rows of a session's wavefront slot for a scene without moving spheres, textures or smoke
+    (wave_shade.cuh compact_slots): three for the books' integrator, four for NEE/MIS; five otherwise."""
     d = desc.contents
     moving = any(d.spheres[i].displacement.x or d.spheres[i].displacement.y or d.spheres[i].displacement.z
                  for i in range(d.sphere_count))
@@ -505,7 +505,7 @@ def batched_jobs(rt, count: int = 64, seed: int = 2024):
 
 
 def batched_measurement(rt, torch, rank: int = 0, world: int = 1) -> dict:
-    """64 jobs in one batched render (the jobs' wavefront runs sharing one slot pool, per step) against the plain
+    """64 jobs in one batched render (the jobs of a group sharing each step's launch) against the plain
     form (one render per job), on the same jobs and seeds; every job's image compared bit for bit. With N ranks the
     jobs are split by cost (pixels x passes, longest first to the least loaded rank) and each rank renders its share
     on its own GPU: the times are the slowest rank's, the segments everyone's (no collective on the data)."""
@@ -569,7 +569,7 @@ def batched_measurement(rt, torch, rank: int = 0, world: int = 1) -> dict:
                      "speedup_gpu_over_reference": (batch_rays / batch_gpu) / (ref_rays / ref_kernel),
                      "speedup_e2e_over_reference": ref_wall / batch_wall}
     return {**reference, "workload": "64 cover-scene variants (50-2000 spheres, W,H log-uniform 64-1024, spp log-uniform "
-                        "16-1024, seeds 0-63), mixture of sizes sharing one wavefront run per step",
+                        "16-1024, seeds 0-63), mixture of sizes sharing each step's launches",
             "ranks": world, "pixels": pixels, "samples": samples, "segments": batch_rays,
             "batched_segments_per_s": batch_rays / batch_gpu, "batched_gpu_s": batch_gpu,
             "batched_e2e_segments_per_s": batch_rays / batch_wall, "batched_e2e_s": batch_wall,

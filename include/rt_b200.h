@@ -211,7 +211,8 @@ typedef struct rt_render_options
 
 typedef struct rt_kernel_info
 {
-    char name[32];
+    char name[32];              /* the form whose image it is, "wavefront" or "persistent", and the integrator; the pool
+                                   kernel goes by the form it stands in for (RT_FORM_AUTO), with its own registers */
     int32_t registers;
     int32_t local_bytes;
     int32_t blocks_per_multiprocessor;
@@ -245,14 +246,19 @@ typedef struct rt_device_info
 /* How a session's launches run (no counterpart in the reference, whose renderer has one kernel): the persistent
    kernel, whose lanes each carry a path from its camera ray to its end, or the wavefront, whose paths wait in device
    memory between a shade kernel and a trace kernel that gives each lane a new ray as soon as its own is answered.
-   Both make the same image from the same seed. AUTO takes the wavefront for scenes searched through the tree and the
-   persistent kernel for the small ones searched flat (and for the counting build). */
+   Both make the same image from the same seed, to the rounding of separately compiled code. AUTO renders by the pool
+   kernel, a wavefront within each warp, wherever it suits: every scene with a primitive but the small ones with neither
+   lights, textures, smoke nor an environment under NEE/MIS, and those with triangles under the books' integrator or with
+   textures, motion or smoke. Its image is, bit for bit, that of the form AUTO takes elsewhere (for the launches it does
+   not take: the longest of scenes with triangles, or with volumes beside a tree; the shortest, and those beyond 2 GiB of
+   samples, of the small bare scenes; the counting build): the wavefront for scenes searched through the tree and for
+   small ones with lights, textures, smoke or an environment, the persistent kernel for the small bare ones. */
 enum { RT_FORM_AUTO = 0, RT_FORM_PERSISTENT = 1, RT_FORM_WAVEFRONT = 2 };
 
 typedef struct rt_session_options
 {
     uint64_t seed;
-    int32_t arithmetic;         /* RT_FLOAT32 or RT_FLOAT64 (a persistent-form session; RT_FORM_WAVEFRONT is refused) */
+    int32_t arithmetic;         /* RT_FLOAT32 or RT_FLOAT64 (by its own pool kernel; RT_FORM_WAVEFRONT is refused) */
     int32_t form;               /* RT_FORM_*; 0 (AUTO) where the caller zeroed the struct */
     double launch_seconds;
 } rt_session_options;
@@ -271,7 +277,8 @@ typedef struct rt_render_report
     rt_accumulation state;
     int32_t launches;
     int32_t kernel_launches;    /* GPU kernels the call launched: a persistent launch's render and reduction, a
-                                   wavefront launch's shade and trace per step and its reduction (no counterpart) */
+                                   wavefront launch's shade and trace per step and its reduction, a pool launch's
+                                   cleared counter, render and reduction (no counterpart) */
     double gpu_seconds;
     double longest_launch_seconds;
 } rt_render_report;
@@ -409,7 +416,7 @@ rt_status rt_session_device_sums(const rt_session* session, const double** sums,
 
 /* Per-kernel timing (no counterpart in the reference, whose render_result gives the launches' total only): while on,
  * every kernel a launch runs is bracketed by CUDA events on the session's stream and its time added to its kind's
- * total: [0] the persistent render kernel, [1] the wavefront's shade kernel, [2] its trace kernel, [3] the
+ * total: [0] the persistent or the pool kernel, [1] the wavefront's shade kernel, [2] its trace kernel, [3] the
  * reductions. Off by default (the events cost a few microseconds a kernel); totals since the view was set. */
 enum { RT_KERNEL_RENDER = 0, RT_KERNEL_SHADE = 1, RT_KERNEL_TRACE = 2, RT_KERNEL_REDUCE = 3 };
 typedef struct rt_kernel_times
@@ -498,7 +505,7 @@ typedef struct rt_batch_report
 } rt_batch_report;
 
 /* Renders every job to its passes in batched steps (many jobs of any size and scene per step; each group of them,
-   by search and form, one persistent launch or one wavefront run per step). */
+   by search and form, one launch of the pool or the persistent kernel or one wavefront run per step). */
 rt_status rt_batch_render(const rt_batch_job* jobs, int32_t count, const rt_batch_options* options,
                           rt_batch_report* report);
 
@@ -513,7 +520,8 @@ typedef struct rt_server_options
      * is published into it while the unclaimed backlog is short, so that no step drains the pool; its first pass is
      * rendered in a batched step of first frames (whose last paths advance through steps of a few slots, not of the
      * whole pool) and handed over. A step runs the pool for about step_seconds of GPU time and returns with work still
-     * running. Images equal a session's rendered to one pass, then to the target. 2: the same with the first passes
+     * running. The books' requests that the pool kernel renders are refined beside it, in batched steps that share the
+     * step's time; a chunk of passes that would take longer is rendered in bands over several steps. Images equal a session's rendered to one pass, then to the target. 2: the same with the first passes
      * published into the pool too. 0: batched steps (each step a batch of passes, drained before it returns). */
     int32_t continuous;
     /* The continuous wavefront (ignored otherwise): its slot pool (a multiple of 128; 0: 1.5 x 2^20), its steps

@@ -330,7 +330,7 @@ class Session:
     def __init__(self, scene: Scene, seed: int = 0, launch_seconds: float = 0.05, form: str = "auto",
                  arithmetic: str = "float32"):
         """form: "auto", "persistent" or "wavefront" (FORMS): how the launches run; the image is the same.
-        arithmetic: "float32" or "float64" (ARITHMETIC; float64 renders the books' scenes in the persistent form)."""
+        arithmetic: "float32" or "float64" (ARITHMETIC; float64 renders the books' scenes by a kernel of its own)."""
         self._scene = scene
         o = _abi.SessionOptions(seed=seed, arithmetic=ARITHMETIC[arithmetic], form=FORMS[form],
                                 launch_seconds=launch_seconds)
@@ -467,8 +467,8 @@ class BatchResult:
 
 
 def batch_render(jobs: list, partial_budget_bytes: int = 0, use_graph: bool = True) -> BatchResult:
-    """Renders many jobs together: per step, one launch (persistent kernel) or one run (wavefront) per group of jobs
-    over all their work items. jobs: a list of
+    """Renders many jobs together: per step, one launch (pool or persistent kernel) or one run (wavefront) per group of
+    jobs over all their work items. jobs: a list of
     (scene, seed, passes) with scene an OwnedScene or a SceneDesc pointer and passes 0 for the camera's sqrt_spp^2."""
     n = len(jobs)
     table = (_abi.BatchJob * max(n, 1))()
@@ -492,7 +492,8 @@ REQUEST_STATES = {0: "queued", 1: "active", 2: "done", 3: "cancelled"}
 class Server:
     """A stream of render requests served in batched steps: admission under an HBM budget, a first frame (one pass)
     for every newly admitted request before refinement, each request done at its target passes. `continuous` 1: the
-    refinement runs in one pool of path slots kept running across steps, first frames in batched steps of their own;
+    refinement runs in one pool of path slots kept running across steps (the books' requests that the pool kernel renders
+    in batched steps beside it), first frames in batched steps of their own;
     2: first frames in the pool too (rt_server_options.continuous)."""
 
     def __init__(self, hbm_budget_bytes: int = 8 << 30, step_seconds: float = 0.02, use_graph: bool = True,

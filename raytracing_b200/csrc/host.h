@@ -466,7 +466,7 @@ private:
 
     // The wavefront form (RT_FORM_WAVEFRONT, or AUTO where wavefront_suits): its steps, or AUTO's pool kernel
     bool wavefront_ = false;
-    std::unique_ptr<wave_runner> wave_;
+    std::unique_ptr<wave_runner> wave_; // (the pool kernel's samples are its too, a bare scene's as well)
     bool pool_ = false;                 // AUTO: the pool kernel, for launches of up to pool_most_samples
     int pool_grid_ = 0;
     int64_t pool_most_ = INT64_MAX;     // and up to this many (tune_candidate)

@@ -283,7 +283,9 @@ inline bool pool_suits(const scene_view& v, bool quality)
     return searched && (wavefront_suits(v) || !quality) && (!triangles || (quality && !has_features(v)));
 }
 // The launches it renders: all, but with triangles those of up to 2^20 samples per unit of depth, and with volumes beside
-// a tree 2^22. A mesh's shading (rough metal, coat, environment) waits for its instructions beside the walks', which the
+// a tree 2^22. (The line follows the smaller mesh, where the steps are ahead above it; the larger crosses later, and a
+// launch of it between the two, as at depth 50 with 66M, is 10 to 20% slower in the steps that the rule gives it to. The
+// crossing moves with the mesh's size, which the rule does not read.) A mesh's shading (rough metal, coat, environment) waits for its instructions beside the walks', which the
 // steps' shade kernel does less; the steps wait at each depth for their last walks. The mesh of 1,280 triangles at depth 6
 // with 3.7M samples 2.42 ms here and 2.44 in the steps, with 14.7M 9.1 and 8.0, at depth 50 with 14.7M 11.2 and 16.2, with
 // 66M 38.8 and 36.9; that of 1.3M at depth 6 with 7.4M 6.1 and 6.9, with 29M 20.7 and 19.3, at depth 50 with 66M 50 and

@@ -6,12 +6,13 @@
 // the NEE/MIS integrator and triangle meshes compute in float only, there as here. Every number of a path is a
 // double: rays, hits, normals, throughput, the random numbers (53-bit uniforms, as random_real<double> draws).
 //
-// The B200 form is the float kernel's: a persistent kernel whose lanes claim (pixel, chunk of 16 passes) work items by
-// a warp ballot and one atomic a warp, regenerate paths as they end, and write each item's sum to its slot of the
-// chunk partials, which the float path's reduction adds into the FP64 sums in chunk order. So the grouping of passes
-// into launches does not change the image, as in float. The tree is the float tables' (its boxes rounded outward in
-// float); a double primitive can stand out of its float box by the rounding of its float copy, so every node bound is
-// widened by the scene's box_margin before the slab test, which keeps the walk conservative.
+// The B200 form is the float pool kernel's (pool_kernel.cuh): persistent warps that keep their paths in shared memory and
+// walk, shade and start them a warp's worth at a time. A finished sample's value goes to its place in a buffer, and a
+// reduction of its own adds them in pass order, chunk by chunk, in the FP64 sums, so the grouping of passes into launches
+// does not change the image, as in float; an image whose samples would not fit the buffer is rendered in bands of tiles.
+// The tree is the float tables' (its boxes rounded outward in float); a double primitive can stand out of its float box by
+// the rounding of its float copy, so every node bound is widened by the scene's box_margin, and the walk, four wide with
+// its boxes tested in float, sets them out by its own rounding too (float_ray): it meets every primitive the ray meets.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -1,12 +1,13 @@
-// A session: one view of a resident scene, its image's sums kept on the device and grown by launches of the
-// persistent kernel (renderer.h:591-673; the launch loop of renderer.cu:1315-1334, 1924-1971).
+// A session: one view of a resident scene, its image's sums kept on the device and grown by launches of the pool kernel,
+// the wavefront's steps or the persistent kernel (renderer.h:591-673; the launch loop of renderer.cu:1315-1334, 1924-1971).
 //
 // Launch planning. The reference plans ~50 ms launches from measured row times and renders a pass in bands of rows
 // when one pass is too long for a launch (renderer.cu:179-308), because Windows stops long kernels. Here a launch is
-// a range of whole passes for every pixel, cut into (pixel, chunk) work items that the persistent threads pull, so a
-// launch's length is set by its number of passes alone: the first launch is one chunk (a probe of the speed), and
-// each later one as many chunks as fit launch_seconds at the last measured speed. A launch may span rounds of
-// strata: every sample finds its round, and so its seed, from its own absolute pass.
+// a range of whole passes for every pixel, cut into samples or (pixel, chunk) work items that the warps pull, so a
+// launch's length is set by its number of passes alone: the first launch is one chunk (a probe of the speed; the pool
+// kernels', as many chunks as surely fit, first_launch_speed), and each later one as many chunks as fit launch_seconds at
+// the last measured speed. A launch may span rounds of strata: every sample finds its round, and so its seed, from its
+// own absolute pass. Only a double launch whose samples would not fit their buffer is cut into bands of tiles.
 #include <algorithm>
 #include <cmath>
 #include <cstring>

@@ -21,8 +21,9 @@ constexpr uint32_t wave_inward = 1u << 9;
 constexpr uint32_t wave_reserved = 1u << 10; // a stream run's slot holds a claim beyond what is published (its number
                                              // in the flags row's last two words) and waits for it
 
-// ---- the persistent render kernel ------------------------------------------------------------------------------
-// The render kernel's resident blocks per multiprocessor, which caps its registers: the books' integrator at 64 (8
+// ---- resident blocks -------------------------------------------------------------------------------------------
+// The persistent render kernel's (kernels.cu) resident blocks per multiprocessor, which caps its registers, and which the
+// shade kernel takes too unless its source chooses its own: the books' integrator at 64 (8
 // blocks of 128 threads measured fastest against 5 and 6 blocks, for the latency they hide), the NEE/MIS integrator,
 // whose GGX and environment code spills heavily at 64, at 80 (6 blocks); with the flat search (no tree stack) both
 // at 72 (7 blocks), measured fastest against 5, 6 and 8 on the Cornell boxes
