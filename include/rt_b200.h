@@ -520,8 +520,8 @@ typedef struct rt_server_options
      * is published into it while the unclaimed backlog is short, so that no step drains the pool; its first pass is
      * rendered in a batched step of first frames (whose last paths advance through steps of a few slots, not of the
      * whole pool) and handed over. A step runs the pool for about step_seconds of GPU time and returns with work still
-     * running. The books' requests that the pool kernel renders are refined beside it, in batched steps that share the
-     * step's time; a chunk of passes that would take longer is rendered in bands over several steps. Images equal a session's rendered to one pass, then to the target. 2: the same with the first passes
+     * running. The books' requests that the pool kernel renders are refined in batched steps, a chunk of passes that would
+     * take longer in bands over several steps; a step goes to them or to the slots, by the least work left. Images equal a session's rendered to one pass, then to the target. 2: the same with the first passes
      * published into the pool too. 0: batched steps (each step a batch of passes, drained before it returns). */
     int32_t continuous;
     /* The continuous wavefront (ignored otherwise): its slot pool (a multiple of 128; 0: 1.5 x 2^20), its steps

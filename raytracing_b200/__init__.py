@@ -493,7 +493,7 @@ class Server:
     """A stream of render requests served in batched steps: admission under an HBM budget, a first frame (one pass)
     for every newly admitted request before refinement, each request done at its target passes. `continuous` 1: the
     refinement runs in one pool of path slots kept running across steps (the books' requests that the pool kernel renders
-    in batched steps beside it), first frames in batched steps of their own;
+    in batched steps between), first frames in batched steps of their own;
     2: first frames in the pool too (rt_server_options.continuous)."""
 
     def __init__(self, hbm_budget_bytes: int = 8 << 30, step_seconds: float = 0.02, use_graph: bool = True,

@@ -703,7 +703,8 @@ double render_server::refine_batched(double seconds)
 // A step of the continuous wavefront: admission as in a batched step; the first frames of the admitted requests in
 // a batched step of their own (arrival order, about max(first_frame_seconds, step_seconds) of them, at least one),
 // handed over to the pool; then, if no first frame is left waiting, the pool runs for about step_seconds of GPU time
-// and returns with work still running. A request's state follows the passes its sums hold.
+// and returns with work still running, or the batched requests are refined for as long. A request's state follows the
+// passes its sums hold.
 rt_server_step_report render_server::step_continuous()
 {
     rt_server_step_report report{};
@@ -809,23 +810,26 @@ rt_server_step_report render_server::step_continuous()
     // frame waits for no refinement; the pool's paths wait in their slots meanwhile, without draining)
     if (first_queue_.empty())
     {
-        // the batched requests and the pool's halve the step when both have work
-        bool batched = false, streamed = false;
+        // The step goes to the batched requests or to the pool's, whichever have the request with the least work left:
+        // by estimated time, as each side orders its own.
+        double batched = INFINITY, streamed = INFINITY;
         for (const auto& [id, r] : requests_)
         {
-            if (r.state == RT_REQUEST_ACTIVE && passes_of(r) < r.target)
+            const int64_t left = r.state == RT_REQUEST_ACTIVE ? r.target - passes_of(r) : 0;
+            if (left > 0)
             {
-                (r.batched ? batched : streamed) = true;
+                double& least = r.batched ? batched : streamed;
+                least = std::min(least, double(r.camera.image_width) * r.camera.image_height * double(left) *
+                                            cost_of(r.scene.get()));
             }
         }
-        const double seconds = batched && streamed ? 0.5 * options_.step_seconds : options_.step_seconds;
-        if (batched)
+        if (batched < INFINITY && batched <= streamed)
         {
-            report.gpu_seconds += refine_batched(seconds);
+            report.gpu_seconds += refine_batched(options_.step_seconds);
         }
-        if (streamed)
+        else if (streamed < INFINITY)
         {
-            report.gpu_seconds += stream_->advance(seconds);
+            report.gpu_seconds += stream_->advance(options_.step_seconds);
         }
     }
     stats_.gpu_seconds += report.gpu_seconds;

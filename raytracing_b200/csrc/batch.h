@@ -262,7 +262,7 @@ private:
 // step gives the newly admitted their first frame (one pass) before it refines the others, and a request is done when
 // it reaches its target passes. Driven by the caller: submit between steps, step, poll, fetch. Its steps are batches
 // of passes (batch_engine) or runs of the continuous wavefront (stream_engine); the continuous server's books'
-// requests, which the pool kernel renders, are refined in batched steps beside it.
+// requests, which the pool kernel renders, are refined in batched steps between the runs.
 class render_server
 {
 public:

@@ -243,3 +243,24 @@ def test_continuous_images_in_bands_equal_sessions(rt, name):
             _same_render(image, want)  # a flat scene's first pass is the persistent kernel's, of its own rounding
     assert server.stats()["used_bytes"] == 0
     server.close()
+
+
+def test_continuous_requests_with_the_least_work_left_come_first(rt):
+    """A books' request (batched steps) and one under NEE/MIS (the slot pool) together: the step is not divided, so the
+    smaller one, of either kind, is done in about the steps it takes alone, as when one pool served both."""
+    scenes = {n: rt.Scene(rt.builtin_scene(n)) for n in ("weekend", "cornell-mis")}
+
+    def steps_until_done(requests):
+        server = rt.Server(hbm_budget_bytes=1 << 30, step_seconds=0.002, continuous=1)
+        ids = [server.submit(scenes[n], rt.builtin_camera(n, width=w, height=w, spp=16), 3, passes) for n, w, passes in requests]
+        steps = 0
+        while server.poll(ids[0])["state"] != "done":
+            server.step()
+            steps += 1
+        server.close()
+        return steps
+
+    for small, large in ((("weekend", 600, 256), ("cornell-mis", 1200, 256)), (("cornell-mis", 400, 128), ("weekend", 1600, 512))):
+        alone = min(steps_until_done([small]) for _ in range(2))
+        assert alone >= 8
+        assert steps_until_done([small, large]) <= 1.5 * alone + 3
