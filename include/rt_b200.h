@@ -278,7 +278,8 @@ typedef struct rt_render_report
     int32_t launches;
     int32_t kernel_launches;    /* GPU kernels the call launched: a persistent launch's render and reduction, a
                                    wavefront launch's shade and trace per step and its reduction, a pool launch's
-                                   cleared counter, render and reduction (no counterpart) */
+                                   cleared counter, render (in double on a tree a second for the samples whose paths
+                                   met a tie) and reduction (no counterpart) */
     double gpu_seconds;
     double longest_launch_seconds;
 } rt_render_report;
